@@ -17,7 +17,8 @@ import time
 import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-sys.path.insert(0, os.path.dirname(HERE))
+# (the script's own folder first on the path would make oracle.py hide the package)
+sys.path[:] = [os.path.dirname(HERE)] + [p for p in sys.path if os.path.abspath(p or ".") != HERE]
 
 from oracle import oracle as O  # noqa: E402
 
