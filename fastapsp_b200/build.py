@@ -33,10 +33,10 @@ METIS_A = os.path.join(CUDA_LIB, "libmetis_static.a")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden",
           "-I" + INCLUDE, "-I" + CSRC]
-SOURCES = ["fap_device.cu", "fap_capi.cu", "fap_legacy.cu", "fap_noalloc.cu", "fap_host.cpp",
+SOURCES = ["fap_device.cu", "fap_capi.cu", "fap_elim.cu", "fap_elim.cpp", "fap_legacy.cu", "fap_noalloc.cu", "fap_host.cpp",
            "fap_serve.cpp"]
 HEADERS = ["fap_common.cuh", "minplus_tile.cuh", "floyd.cuh", "sssp.cuh", "tma.cuh", "tma_tile.cuh",
-           "fap_internal.h"]
+           "fap_internal.h", "fap_elim.h"]
 
 
 def _stale(target: str, deps: list[str]) -> bool:
@@ -62,7 +62,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     objs = []
     for src in SOURCES:
         path = os.path.join(CSRC, src)
-        obj = os.path.join(OBJDIR, os.path.splitext(src)[0] + ".o")
+        obj = os.path.join(OBJDIR, src.replace(".", "_") + ".o")
         objs.append(obj)
         if force or _stale(obj, [path] + hdrs + [__file__]):
             cmd = [NVCC] + ARCH + COMMON + ["-c", path, "-o", obj]

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -12,10 +13,13 @@
 #include <exception>
 #include <new>
 #include <string>
+#include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "fap_b200.h"
 #include "fap_common.cuh"
+#include "fap_elim.h"
 #include "fap_internal.h"
 
 using namespace fapb;
@@ -270,6 +274,46 @@ bool queue_order_ok(const std::vector<PartDesc> &parts, bool sym, const std::vec
 
 }  // namespace
 
+// Boundary sets up to this size close dB by Floyd; larger ones by the tiled
+// Bellman-Ford over the boundary graph (Floyd's cube grows too fast).
+constexpr int64_t kBgraphFloydMax = 8192;
+
+// Device copy of an elimination plan (fap_elim.h), one buffer made with the
+// partition.
+struct ElimBuf {
+  ElimPlan plan;
+  DevBuf buf;
+  ElimDev dev{};
+  void release() {
+    buf.release();
+    plan = ElimPlan{};
+  }
+  int upload() {
+    const struct { const void *p; size_t bytes; } src[] = {
+        {plan.parts.data(), plan.parts.size() * sizeof(ElimPart)},
+        {plan.loc.data(), plan.loc.size() * 4},   {plan.inv.data(), plan.inv.size() * 4},
+        {plan.eptr.data(), plan.eptr.size() * 4}, {plan.ecol.data(), plan.ecol.size() * 4},
+        {plan.eend.data(), plan.eend.size() * 4}, {plan.w0.data(), plan.w0.size() * 4},
+        {plan.lev.data(), plan.lev.size() * 4},   {nullptr, plan.ecol.size() * sizeof(int2)}};
+    size_t off[9], bytes = 0;
+    for (int i = 0; i < 9; i++) {
+      off[i] = bytes;
+      bytes += (src[i].bytes + 255) / 256 * 256;
+    }
+    FAP_TRY(buf.ensure(std::max<size_t>(bytes, 256)));
+    std::vector<char> host(off[8]);
+    for (int i = 0; i < 8; i++)
+      if (src[i].bytes > 0) std::memcpy(host.data() + off[i], src[i].p, src[i].bytes);
+    FAP_CK(cudaMemcpy(buf.p, host.data(), host.size(), cudaMemcpyHostToDevice));
+    char *d = buf.as<char>();
+    auto at = [&](int i) { return reinterpret_cast<const int32_t *>(d + off[i]); };
+    dev = ElimDev{reinterpret_cast<const ElimPart *>(d), at(1), at(2), at(3), at(4), at(5), at(6), at(7),
+                  reinterpret_cast<int2 *>(d + off[8]), (int32_t)plan.parts.size(), plan.max_s, plan.max_b,
+                  plan.max_nent, plan.max_nlev};
+    return FAP_OK;
+  }
+};
+
 struct fap_dgraph {
   fap_ctx *ctx = nullptr;
   int32_t n = 0;
@@ -378,6 +422,15 @@ struct fap_dgraph {
   // stores each one's transpose (floyd_queue_items, sym).
   bool sym_local = false;
   int64_t total_b = 0;
+  // Elimination form of the boundary graph (elim_ok): el the parts' plan, el2
+  // the boundary graph's own (one part without a boundary, up to
+  // kElimGraphMax vertices; larger ones are closed by Floyd), barcs the arcs
+  // between boundary vertices as (boundary index, boundary index, weight).
+  bool eliminate = true;   // parameter "eliminate"
+  bool last_elim = false;  // the prepared batch uses it
+  ElimBuf el, el2;
+  std::vector<int32_t> barcs;
+  DevBuf d_barcs, d_elist, d_eoff;
   std::vector<int32_t> boff;
   std::vector<int32_t> bpcol;  // boundary columns of dB padded per part to multiples of 4 (prefix sums)
   bool last_bmethod = false;   // the prepared batch uses it
@@ -625,6 +678,115 @@ void cache_drop(fap_dgraph *G) {
 }
 }  // namespace
 
+namespace {
+// Boundary graphs are closed by elimination up to this size and number of
+// entries, larger ones by Floyd on dB: one CTA runs the numeric part, with
+// the entries in its shared memory (road114k, 650 vertices and 4,100
+// entries: 0.10 ms against 0.56 ms for Floyd; a 1,726-vertex boundary graph of
+// a geometric graph, 67,000 entries in L2: 5.5 ms against 1.9).
+constexpr int64_t kElimGraphMax = 2048;
+constexpr int64_t kElimGraphEntries = 24576;
+
+// The elimination plans of the parts and of the boundary graph, for
+// undirected int32 graphs (every arc has its reverse with the same weight)
+// without duplicate arcs inside a part.  Host work of some milliseconds on
+// up to 16 threads.
+int build_elim(fap_dgraph *G) {
+  G->el.release();
+  G->el2.release();
+  G->barcs.clear();
+  if (G->dtype != FAP_DTYPE_I32 || !G->sym_local || G->total_b <= 0) return FAP_OK;
+  const int32_t K = (int32_t)G->vnum.size() - 1;
+  auto bidx = [&](int32_t v) { return G->boff[G->gid[v]] + (G->ed2st[v] - G->voff[G->gid[v]]); };
+  auto weight = [&](int32_t e) {
+    int32_t w;
+    std::memcpy(&w, &G->h_w[e], 4);
+    return w;
+  };
+  auto part_graph = [&](int i0, ElimGraph *g) {
+    const int32_t p = i0 + 1, first = G->voff[p];
+    g->s = G->vnum[p];
+    g->b = G->bnum[p];
+    g->boff = G->boff[p];
+    g->ptr.reserve(g->s + 1);
+    g->ptr.push_back(0);
+    for (int32_t i = 0; i < g->s; i++) {
+      const int32_t u = G->st2ed[first + i];
+      for (int32_t e = G->h_ro[u]; e < G->h_ro[u + 1]; e++) {
+        const int32_t v = G->h_col[e];
+        if (v == u || G->gid[v] != p) continue;
+        g->adj.push_back(G->ed2st[v] - first);
+        g->w.push_back(weight(e));
+      }
+      g->ptr.push_back((int32_t)g->adj.size());
+    }
+  };
+  std::vector<std::array<int32_t, 3>> cross;
+  for (int32_t p = 1; p <= K; p++)
+    for (int32_t i = 0; i < G->bnum[p]; i++) {
+      const int32_t u = G->st2ed[G->voff[p] + i];
+      for (int32_t e = G->h_ro[u]; e < G->h_ro[u + 1]; e++) {
+        const int32_t v = G->h_col[e];
+        if (G->gid[v] != p)
+          cross.push_back({bidx(u), bidx(v), weight(e)});
+        else if (v != u && G->ed2st[v] - G->voff[p] < G->bnum[p])
+          G->barcs.insert(G->barcs.end(), {bidx(u), bidx(v), weight(e)});
+      }
+    }
+  // the least weight of every crossing pair has to be the same both ways
+  std::sort(cross.begin(), cross.end());
+  cross.erase(std::unique(cross.begin(), cross.end(),
+                          [](const auto &a, const auto &b) { return a[0] == b[0] && a[1] == b[1]; }),
+              cross.end());
+  for (const auto &a : cross) {
+    const auto it = std::lower_bound(cross.begin(), cross.end(), std::array<int32_t, 3>{a[1], a[0], 0});
+    if (it == cross.end() || (*it)[0] != a[1] || (*it)[1] != a[0] || (*it)[2] != a[2]) return FAP_OK;
+  }
+  for (const auto &a : cross) G->barcs.insert(G->barcs.end(), a.begin(), a.end());
+  if (G->barcs.size() > (size_t)INT32_MAX) return FAP_OK;
+  elim_build(K, part_graph, std::min(16, (int)std::thread::hardware_concurrency()), &G->el.plan);
+  if (!G->el.plan.ok) return FAP_OK;
+  FAP_TRY(G->el.upload());
+  FAP_TRY(G->d_barcs.ensure(std::max<size_t>(G->barcs.size(), 4) * 4));
+  if (!G->barcs.empty())
+    FAP_CK(cudaMemcpy(G->d_barcs.p, G->barcs.data(), G->barcs.size() * 4, cudaMemcpyHostToDevice));
+  if (G->total_b > kElimGraphMax) return FAP_OK;
+  auto boundary_graph = [&](int, ElimGraph *g) {
+    g->s = (int32_t)G->total_b;
+    g->ptr.push_back(0);
+    size_t x = 0;
+    for (int32_t p = 1; p <= K; p++)
+      for (int32_t i = G->boff[p]; i < G->boff[p + 1]; i++) {
+        for (int32_t j = G->boff[p]; j < G->boff[p + 1]; j++)
+          if (j != i) g->adj.push_back(j);
+        for (; x < cross.size() && cross[x][0] == i; x++) g->adj.push_back(cross[x][1]);
+        g->ptr.push_back((int32_t)g->adj.size());
+      }
+  };
+  elim_build(1, boundary_graph, 1, &G->el2.plan);
+  if (G->el2.plan.nent > kElimGraphEntries) G->el2.plan = ElimPlan{};
+  if (!G->el2.plan.ok) return FAP_OK;
+  elim_offsets(round_up(G->total_b, kFloydTile), &G->el2.plan);
+  return G->el2.upload();
+}
+
+// Whether solves close the boundary graph and the parts by elimination:
+// where a plan exists and no parameter asks for one of the other forms.
+// A batch of some of the parts (`sources` boundary vertices; all parts: -1)
+// takes it where elimination closes the whole boundary graph too, and dB
+// needs no more memory than the SSSP scratch rows it replaces, or 4 MB (the
+// server admits such batches by that size).  One part of a 50,001-vertex road
+// graph: 0.17 ms instead of 4.6.
+constexpr int64_t kElimBatchElems = int64_t(1) << 20;
+bool elim_ok(const fap_dgraph *G, int64_t sources) {
+  if (!G->eliminate || !G->el.plan.ok || G->dtype != FAP_DTYPE_I32 || G->stage1 == 1 || G->bgraph_form != 0 ||
+      !G->floyd_queue || !G->floyd_sym || G->floyd_per_cta || G->total_b > kBgraphFloydMax)
+    return false;
+  const int64_t ldB = round_up(G->total_b, kFloydTile);
+  return sources < 0 || (G->el2.plan.ok && ldB * ldB <= std::max<int64_t>(sources * G->n, kElimBatchElems));
+}
+}  // namespace
+
 extern "C" int fap_graph_destroy(fap_dgraph *G) try {
   if (!G) return FAP_OK;
   fap_ctx *c = G->ctx;
@@ -632,7 +794,9 @@ extern "C" int fap_graph_destroy(fap_dgraph *G) try {
     DeviceGuard g(c->device);
     cudaStreamSynchronize(c->stream);
     if (G->gexec) cudaGraphExecDestroy(G->gexec);
-    for (DevBuf *b : {&G->ro, &G->col, &G->w, &G->ro_s, &G->col_s, &G->w_s, &G->sssp_scratch, &G->d_thin,
+    G->el.release();
+    G->el2.release();
+    for (DevBuf *b : {&G->d_barcs, &G->d_elist, &G->d_eoff, &G->ro, &G->col, &G->w, &G->ro_s, &G->col_s, &G->w_s, &G->sssp_scratch, &G->d_thin,
                       &G->d_gid, &G->d_st2ed, &G->d_ed2st, &G->D, &G->F, &G->d_parts, &G->d_work,
                       &G->d_src, &G->d_srcrows, &G->d_status, &G->d_checks, &G->staging, &G->P,
                       &G->d_tro, &G->d_tcol, &G->d_tw, &G->d_dB, &G->d_bpart, &G->d_brows, &G->d_FB,
@@ -768,6 +932,7 @@ extern "C" int fap_graph_set_parts(fap_dgraph *G, int32_t K, const int32_t *grap
       G->sym_local = sym;
     }
   }
+  FAP_TRY(build_elim(G));
   {
     // edges of the boundary graph
     int64_t cross = 0;
@@ -846,9 +1011,6 @@ extern "C" int fap_graph_reserve(fap_dgraph *G, int64_t max_rows) try {
 
 namespace {
 
-// Boundary sets up to this size close dB by Floyd; larger ones by the tiled
-// Bellman-Ford over the boundary graph (Floyd's cube grows too fast).
-constexpr int64_t kBgraphFloydMax = 8192;
 // The staged expansion keeps kExpandRows rows of dB in shared memory.
 constexpr int64_t kBgraphStagedMax = 4096;
 // Largest column table of the staged expansion (max_b x ldD values).
@@ -1102,9 +1264,70 @@ int expand_bgraph(fap_dgraph *G, const PartDesc *dp, int np, int max_s, const T 
   return FAP_OK;
 }
 
+// Device state of the elimination form for the listed parts (row_base and
+// f_off final): the plans, dB, the parts to close and, for a batch of some of
+// the parts, the boundary rows to write.
+int prepare_elim(fap_dgraph *G, const std::vector<PartDesc> &parts) {
+  G->ldB = round_up(std::max<int64_t>(G->total_b, 1), kFloydTile);
+  FAP_TRY(G->d_dB.ensure((size_t)G->ldB * G->ldB * 4));
+  std::vector<int32_t> list;
+  std::vector<int64_t> off{0}, rows;  // (the first offset is the boundary graph's own)
+  for (const PartDesc &d : parts) {
+    list.push_back(d.part - 1);
+    off.push_back(d.f_off);
+    for (int32_t k = 0; k < d.b; k++) {
+      rows.push_back(G->boff[d.part] + k);
+      rows.push_back(d.row_base + k);
+    }
+  }
+  FAP_TRY(G->d_elist.ensure(list.size() * 4));
+  FAP_TRY(G->d_eoff.ensure(off.size() * 8));
+  FAP_TRY(G->d_brows.ensure(std::max<size_t>(rows.size(), 2) * 8));
+  FAP_CK(cudaMemcpy(G->d_elist.p, list.data(), list.size() * 4, cudaMemcpyHostToDevice));
+  FAP_CK(cudaMemcpy(G->d_eoff.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice));
+  if (!rows.empty()) FAP_CK(cudaMemcpy(G->d_brows.p, rows.data(), rows.size() * 8, cudaMemcpyHostToDevice));
+  return FAP_OK;
+}
+
+// Stages 1-2 by elimination: F = the listed parts' exact closures, Dout = the
+// rows of their boundary vertices.  ev[0..3] mark the phases (numeric
+// elimination, boundary graph, closures, boundary rows).
+int run_elim(fap_dgraph *G, const PartDesc *dp, int count, int max_s, int32_t *F, int64_t ldf, int32_t *Dout, cudaEvent_t ev1,
+             cudaEvent_t ev2, cudaEvent_t ev3, int *status, int64_t *L) {
+  cudaStream_t st = G->ctx->stream;
+  int32_t *dB = G->d_dB.as<int32_t>();
+  const int64_t *off = G->d_eoff.as<const int64_t>();
+  const bool all = count == G->K;
+  const int nb = (int)G->total_b;
+  int nrows = 0;
+  if (!all)
+    for (const PartDesc &d : G->parts) nrows += d.b;
+  FAP_CK(launch_elim_seed(dB, G->ldB, nb, G->el2.plan.ok ? nb : (int)G->ldB, G->d_barcs.as<const int32_t>(),
+                          (int)(G->barcs.size() / 3), st, L));
+  FAP_CK(launch_elim_up(G->el.dev, nullptr, dB, G->ldB, st, L));
+  FAP_CK(record_event(ev1, st));
+  if (G->el2.plan.ok) {
+    FAP_CK(launch_elim_up(G->el2.dev, dB, nullptr, 0, st, L));
+    FAP_CK(launch_elim_close(G->el2.dev, nullptr, off, 1, nb, nullptr, 0, dB, G->ldB, st, L));
+  } else {
+    FAP_CK(launch_floyd_matrix<int32_t>(dB, G->ldB, (int)ceil_div(nb, kFloydTile), status, st, L, nb));
+  }
+  FAP_CK(record_event(ev2, st));
+  FAP_CK(launch_elim_close(G->el.dev, G->d_elist.as<const int32_t>(), off + 1, count, max_s, dB, G->ldB, F, ldf, st, L));
+  FAP_CK(record_event(ev3, st));
+  if (all) {
+    FAP_TRY(expand_bgraph<int32_t>(G, dp, count, max_s, F, Dout, ldf, status, L));
+  } else {
+    FAP_CK(launch_elim_expand(G->el.dev, G->d_brows.as<const int64_t>(), nrows, dB, G->ldB,
+                              G->d_st2ed.as<const int32_t>(), G->n, Dout, G->ldD, st, L));
+  }
+  return FAP_OK;
+}
+
 // Builds (or reuses) the batch descriptors for the requested parts.
-int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, bool bmethod) {
-  const bool same = (ids == G->last_ids) && (cached == G->last_cached) && (bmethod == G->last_bmethod);
+int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, bool bmethod, bool elim) {
+  const bool same = (ids == G->last_ids) && (cached == G->last_cached) && (bmethod == G->last_bmethod) &&
+                    (elim == G->last_elim);
   if (same) return FAP_OK;
   // The descriptors change from here on: until they are complete no batch
   // counts as prepared, so a failure below forces a full rebuild next time.
@@ -1243,7 +1466,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
     }
   }
   std::vector<QItem> qitems;
-  if (!cached) {
+  if (!cached && !elim) {
     int32_t mnb = 0;
     // (the local closures of the boundary-graph form are symmetric when the
     // parts are; the SSSP form's matrices hold boundary rows and are not)
@@ -1258,7 +1481,8 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
   FAP_CK(cudaStreamSynchronize(st));
   if (!qitems.empty())
     FAP_CK(cudaMemcpy(G->q.items.p, qitems.data(), qitems.size() * sizeof(QItem), cudaMemcpyHostToDevice));
-  if (bmethod) FAP_TRY(prepare_bgraph(G, G->parts, true));
+  if (elim) FAP_TRY(prepare_elim(G, G->parts));
+  if (bmethod && (int32_t)ids.size() == G->K) FAP_TRY(prepare_bgraph(G, G->parts, true));
   FAP_CK(cudaMemcpy(G->d_parts.p, G->parts.data(), G->parts.size() * sizeof(PartDesc), cudaMemcpyHostToDevice));
   if (!G->work.empty())
     FAP_CK(cudaMemcpy(G->d_work.p, G->work.data(), G->work.size() * sizeof(MPWork), cudaMemcpyHostToDevice));
@@ -1275,6 +1499,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
   G->last_ids = ids;
   G->last_cached = cached;
   G->last_bmethod = bmethod;
+  G->last_elim = elim;
   G->epoch++;
   return FAP_OK;
 }
@@ -1328,6 +1553,8 @@ bool use_msbf(const fap_dgraph *G) {
   if (G->sssp_form == 2) return true;
   return G->n > 0 && G->m >= 6 * (int64_t)G->n;
 }
+
+constexpr const char *kElimName = "boundary graph, Floyd class closed by elimination";
 
 const char *stage1_form_name(const fap_dgraph *G, bool bmethod) {
   if (bmethod) return bgraph_bf(G) ? "boundary graph, Bellman-Ford closure" : "boundary graph, Floyd closure";
@@ -1410,7 +1637,22 @@ int run_solve(fap_dgraph *G, int mode) {
   int64_t L = 0;
   FAP_CK(cudaMemsetAsync(status, 0, sizeof(int), st));
   for (int i = 0; i < 5; i++) G->timing[i] = -1.0f;
-  if (mode == FAP_MODE_BATCHED && G->last_bmethod) {
+  if (mode == FAP_MODE_BATCHED && G->last_elim) {
+    // Elimination form: numeric elimination and the boundary graph, the
+    // parts' closures, the boundary rows, then the min-plus merge (event
+    // slots as below).
+    if constexpr (std::is_same<T, int32_t>::value) {
+      FAP_CK(record_event(c->ev[0], st));
+      FAP_TRY(run_elim(G, dp, np, G->max_s, F, G->max_ldf, D, c->ev[5], c->ev[1], c->ev[2], status, &L));
+      FAP_CK(record_event(c->ev[3], st));
+      FAP_CK(launch_minplus_thin<T>(dp, G->d_thin.as<int32_t>(), (int)G->thin.size(), G->max_s, G->n, F, D,
+                                    G->ldD, gid, ed2st, st, &L));
+      FAP_CK(launch_minplus_parts<T>(dp, np, dw, (int)G->work.size(), G->n, F, G->max_ldf, D, G->ldD,
+                                     G->max_rows, gid, ed2st, status, st, &L, pack16_of(G)));
+      if (G->paths) FAP_TRY(launch_paths<T>(G, dp, np, G->max_s, F, &L));
+      FAP_CK(record_event(c->ev[4], st));
+    }
+  } else if (mode == FAP_MODE_BATCHED && G->last_bmethod) {
     // Boundary-graph form: local closures of all parts, boundary-graph APSP,
     // boundary rows by expansion, then the min-plus merge.  The events keep
     // the stage slots in order of time: [gather, floyd, boundary graph +
@@ -1553,13 +1795,19 @@ extern "C" int fap_solve(fap_dgraph *G, const int32_t *parts, int32_t count, int
     for (const int32_t p : ids)
       if (!G->cache_valid[p])
         return fail(FAP_ERR_STATE, "part %d is another rank's: the sharded cache holds this rank's parts only", p);
-  const bool bmethod = !cached && mode == FAP_MODE_BATCHED && (int32_t)ids.size() == G->K && bmethod_ok(G);
-  FAP_TRY(prepare_batch(G, ids, cached, bmethod));
+  const bool all_parts = (int32_t)ids.size() == G->K;
+  int64_t sources = all_parts ? -1 : 0;
+  if (!all_parts)
+    for (const int32_t p : ids) sources += G->bnum[p];
+  const bool elim = !cached && mode == FAP_MODE_BATCHED && elim_ok(G, sources);
+  const bool bmethod = elim || (!cached && mode == FAP_MODE_BATCHED && all_parts && bmethod_ok(G));
+  FAP_TRY(prepare_batch(G, ids, cached, bmethod, elim));
   int rc = FAP_OK;
   cudaStream_t st = G->ctx->stream;
   // (the tiled SSSP form tests convergence on the host: not capturable)
   const bool host_loop = !cached && (bmethod ? bgraph_bf(G) : use_msbf(G));
-  G->stage1_name = cached ? "resident cache (" + G->cache_stage1_name + ")" : stage1_form_name(G, bmethod);
+  G->stage1_name = cached ? "resident cache (" + G->cache_stage1_name + ")"
+                          : elim ? kElimName : stage1_form_name(G, bmethod);
   // A batch is captured the second time it is solved unchanged: a batch
   // solved once (a server's batches of changing composition) runs its
   // launches directly instead of paying for a capture and an instantiation.
@@ -2199,6 +2447,11 @@ extern "C" int fap_graph_set_param(fap_dgraph *G, const char *key, double value)
     G->last_ids.clear();
     return FAP_OK;
   }
+  if (std::strcmp(key, "eliminate") == 0) {
+    G->eliminate = value != 0.0;
+    G->last_ids.clear();
+    return FAP_OK;
+  }
   if (std::strcmp(key, "floyd_symmetric") == 0) {
     G->floyd_sym = value != 0.0;
     G->last_ids.clear();
@@ -2394,8 +2647,9 @@ extern "C" int fap_graph_device_bytes(const fap_dgraph *G, int64_t *bytes) try {
                           &G->d_bDt, &G->d_bact, &G->d_bpact, &G->d_bgpart, &G->d_bpcolmap, &G->d_grow,
                           &G->d_bTc, &G->d_pk_off, &G->d_pk_range, &G->d_pk_maxa, &G->d_pk_tiles, &G->d_pk_s16,
                           &G->d_pk_at, &G->d_pk_krow, &G->d_xk_off, &G->d_xk_range, &G->d_xk_maxb, &G->d_xk_tiles,
-                          &G->d_xk_ap, &G->d_xk_bd})
+                          &G->d_xk_ap, &G->d_xk_bd, &G->d_barcs, &G->d_elist, &G->d_eoff})
     t += (int64_t)b->bytes;
+  t += (int64_t)(G->el.buf.bytes + G->el2.buf.bytes);
   *bytes = t;
   return FAP_OK;
 } catch (...) {
@@ -2452,7 +2706,8 @@ int cache_build_impl(fap_dgraph *G) {
   G->cparts.clear();
   std::vector<int32_t> src;
   std::vector<int64_t> srows;
-  const bool bm = bmethod_ok(G);
+  const bool elim = elim_ok(G, -1);
+  const bool bm = elim || bmethod_ok(G);
   for (int32_t p = 1; p <= K; p++) {
     PartDesc d{};
     d.part = p;
@@ -2477,7 +2732,7 @@ int cache_build_impl(fap_dgraph *G) {
   if (!bm && !use_msbf(G))  // (the tiled form sizes its own tiles)
     FAP_TRY(G->sssp_scratch.ensure(
         (size_t)std::max(sssp_scratch_rows(G->n, (int)src.size()), 1) * (size_t)G->n * 4));
-  {
+  if (!elim) {
     int32_t mnb = 0;
     G->cq.sym = bm && G->sym_local && G->floyd_sym;
     const std::vector<QItem> qitems = floyd_queue_items(G->cparts, G->cq.sym, &G->cq.nfloyd, &mnb);
@@ -2508,7 +2763,19 @@ int cache_build_impl(fap_dgraph *G) {
   for (cudaEvent_t &ev : G->cev)
     if (!ev) FAP_CK(cudaEventCreate(&ev));
   FAP_CK(cudaMemsetAsync(status, 0, sizeof(int), st));
-  if (bm) {
+  if (elim) {
+    // Elimination: phases [numeric elimination, boundary graph, closures,
+    // boundary rows].
+    if constexpr (std::is_same<T, int32_t>::value) {
+      FAP_TRY(prepare_elim(G, G->cparts));
+      FAP_TRY(prepare_bgraph(G, G->cparts));
+      FAP_CK(cudaEventRecord(G->cev[0], st));
+      FAP_TRY(run_elim(G, dp, K, cs.max_s, F, cs.ldf, Bd, G->cev[1], G->cev[2], G->cev[3], status, &L));
+      FAP_CK(cudaEventRecord(G->cev[4], st));
+    }
+    G->cache_bmethod = true;
+    G->cache_stage1_name = kElimName;
+  } else if (bm) {
     // Boundary-graph form: local closures, boundary-graph APSP, expansion.
     FAP_TRY(prepare_bgraph(G, G->cparts));
     FAP_CK(cudaEventRecord(G->cev[0], st));

@@ -1,0 +1,104 @@
+// Vertex elimination inside the parts of an undirected int32 graph: the host
+// plan (fap_elim.cpp) and the launchers of its kernels (fap_elim.cu).
+// Internal, not installed.
+//
+// Every part's inner vertices are eliminated one after the other (least
+// remaining degree first, boundary vertices never).  Eliminating v joins the
+// vertices N+(v) it is still adjacent to, so that every path from v to a
+// vertex not eliminated before v leaves through N+(v): with W(v, u) the
+// shortest path from v to u through vertices eliminated earlier,
+//   D[v][x] = min over u in N+(v) of W(v, u) + D[u][x]
+// for every x that is not eliminated before v.  Sums and minima of int32 are
+// exact, so the values are those of Floyd-Warshall.  On road-shaped parts
+// N+(v) holds 1.4 vertices on average (a part of 830 vertices: 1,300
+// relaxations per column instead of 830^2), on grid parts about 20.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <functional>
+#include <vector>
+
+namespace fapb {
+
+// One part of the plan.  Its vertices are renumbered: 0..b-1 the boundary
+// vertices in their local order, b..s-1 the inner ones by level, last
+// eliminated first, so that N+(v) holds smaller numbers only.  All offsets
+// are into the plan's arrays.
+struct ElimPart {
+  int32_t s, b;
+  int32_t voff;        // loc / inv: s entries; eptr: s + 1 entries at voff + index of the part
+  int32_t eptr_off;
+  int32_t ent_off;     // ecol / eend / w0: nent entries, vertex after vertex
+  int32_t nent;
+  int32_t lev_off;     // nlev + 1 level starts, first level = highest (next to the boundary)
+  int32_t nlev;
+  int32_t boff;        // first boundary index of the part
+};
+
+struct ElimPlan {
+  bool ok = false;
+  std::vector<ElimPart> parts;
+  std::vector<int32_t> loc, inv;   // plan number <-> local index
+  std::vector<int32_t> eptr;       // entries of a vertex, relative to ent_off
+  std::vector<int32_t> ecol;       // N+(v), plan numbers, descending
+  std::vector<int32_t> eend;       // end of the entry's vertex, relative to ent_off
+  std::vector<int32_t> w0;         // weight of the edge (v, u), or the sentinel
+  std::vector<int32_t> lev;
+  int32_t max_s = 0, max_b = 0, max_nent = 0, max_nlev = 0;
+  int64_t nent = 0;
+};
+
+// Adjacency of part p (0-based) for the plan: local indices and weights of
+// the undirected edges, both directions listed, no self loops.
+struct ElimGraph {
+  int32_t s = 0, b = 0, boff = 0;
+  std::vector<int32_t> ptr, adj, w;  // w empty: weights come from a dense matrix
+};
+
+// Symbolic elimination of the parts on up to `threads` host threads; graph(p)
+// fills in part p's adjacency and is called on any of them.  ok
+// stays false when a part has more than kElimMaxS vertices (a strip of eight
+// columns fills the shared memory) or more than s^2 / kElimDense entries.
+constexpr int32_t kElimMaxS = 6144;
+constexpr int64_t kElimDense = 16;
+void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, int threads, ElimPlan *out);
+// w0 of a one-part plan := offsets of the entries in a matrix whose rows and
+// columns are the part's local indices.
+void elim_offsets(int64_t ld, ElimPlan *plan);
+
+// Device arrays of a plan.
+struct ElimDev {
+  const ElimPart *parts;
+  const int32_t *loc, *inv, *eptr, *ecol, *eend, *w0, *lev;
+  int2 *ent;  // {plan number of u, W(v, u)}, written by launch_elim_up
+  int32_t nparts, max_s, max_b, max_nent, max_nlev;
+};
+
+// M (ld): the sentinel on nfill x nfill, 0 on the first nb diagonal entries,
+// and the least weight of each listed arc (i, j, weight).
+cudaError_t launch_elim_seed(int32_t *M, int64_t ld, int nb, int nfill, const int32_t *arcs, int narcs, cudaStream_t stream,
+                             int64_t *launches);
+
+// W of every part of the plan, and into M (boundary indices) the shortest
+// paths between a part's boundary vertices through its inner ones.  from:
+// the edges' weights are the elements of this matrix that w0 names (offsets,
+// elim_offsets) instead of w0 itself.
+cudaError_t launch_elim_up(const ElimDev &e, const int32_t *from, int32_t *M, int64_t ldM,
+                           cudaStream_t stream, int64_t *launches);
+
+// Exact closures of the listed parts (0-based plan parts; list null: all of
+// them in order) from the closed boundary matrix dB (null: the parts have no
+// boundary): out_off[i] + local row * ld + local column.
+cudaError_t launch_elim_close(const ElimDev &e, const int32_t *list, const int64_t *out_off, int count, int max_s,
+                              const int32_t *dB, int64_t ldB, int32_t *out, int64_t ld, cudaStream_t stream,
+                              int64_t *launches);
+
+// Rows of D for the listed boundary vertices (pairs boundary index, row of
+// D), every column, from the closed dB; vid: sorted position -> column.
+cudaError_t launch_elim_expand(const ElimDev &e, const int64_t *rows, int nrows, const int32_t *dB, int64_t ldB,
+                               const int32_t *vid, int n, int32_t *D, int64_t ldD, cudaStream_t stream,
+                               int64_t *launches);
+
+}  // namespace fapb

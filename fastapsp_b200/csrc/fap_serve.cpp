@@ -72,6 +72,7 @@ struct GSlot {
   int64_t base_bytes = 0;  // CSR + partition, always resident
   std::vector<int32_t> vnum, voff, bnum;
   int64_t max_part = 0;        // largest part (rows)
+  int64_t bgraph_bytes = 0;    // the boundary graph's matrix
   int64_t reserved_rows = 0;   // output rows the graph's D holds (0: released)
   // the batch in flight: distance rows, checksums on the device and their
   // pinned host copy, status word (buffers grow with the largest batch)
@@ -427,7 +428,8 @@ bool fap_server::launch(int gi) {
       if (!cached) need += r * (int64_t)g.n * 4;
     } else {
       need += std::max<int64_t>(0, target - g.reserved_rows) * g.ldD * 4;
-      if (!cached) need += np * lf * lf * 4 + sc * (int64_t)g.n * 4;
+      // (or the boundary graph's matrix, up to 4 MB more)
+      if (!cached) need += np * lf * lf * 4 + std::max(sc * (int64_t)g.n * 4, std::min(g.bgraph_bytes, int64_t(4) << 20));
     }
     return need;
   };
@@ -714,6 +716,9 @@ int fap_server_add_graph(fap_server *s, int32_t n, int64_t m, const int32_t *row
   g->vnum.assign(ver_num, ver_num + K + 1);
   g->voff.assign(ver_offset, ver_offset + K + 1);
   g->bnum.assign(bdy_num, bdy_num + K + 1);
+  int64_t bsum = 0;
+  for (int32_t p = 1; p <= K; p++) bsum += bdy_num[p];
+  g->bgraph_bytes = ((bsum + 127) / 128 * 128) * ((bsum + 127) / 128 * 128) * 4;
   for (int32_t p = 1; p <= K; p++) g->max_part = std::max<int64_t>(g->max_part, ver_num[p]);
   // Batches change from one launch to the next: launch the stages directly
   // instead of capturing a CUDA graph per batch.

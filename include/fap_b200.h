@@ -203,7 +203,13 @@ FAP_API int fap_graph_sssp_rows(fap_dgraph *g, const int32_t *sources, int32_t c
  * queue; 0: three launches per pivot block); "floyd_symmetric" (default 1:
  * on parts whose arcs all have reverses of equal weight, the queue computes
  * the local closures' tiles on and above the diagonal and stores their
- * transposes); "thin_max_b" (0..16, default 16: parts with at most this many
+ * transposes); "eliminate" (default 1: on undirected int32 graphs without
+ * duplicate arcs inside a part, whose parts eliminate with short lists, the
+ * batched solves and the resident cache close the parts and small boundary
+ * graphs by vertex elimination instead of Floyd-Warshall and SSSP, also for
+ * batches of some of the parts; needs "floyd_queue" and "floyd_symmetric" on
+ * and "stage1" and "bgraph_form" not forced to another form; the same values
+ * either way); "thin_max_b" (0..16, default 16: parts with at most this many
  * boundary vertices take the store-shaped thin min-plus kernel, the others
  * the register-tiled one); "max_resident_rows" (>= 1: at most this many
  * output rows are reserved on the device, as when HBM cannot hold all n
@@ -341,7 +347,8 @@ FAP_API int fap_graph_last_stage1(const fap_dgraph *g);
 
 /* How stage 1 of the last solve ran, in words: "SSSP, frontier", "SSSP,
  * tiled Bellman-Ford", "boundary graph, Floyd closure", "boundary graph,
- * Bellman-Ford closure", or "resident cache (<how it was built>)"; "" before
+ * Bellman-Ford closure", "boundary graph, Floyd class closed by elimination"
+ * (at most 8192 boundary vertices, "eliminate"), or "resident cache (<how it was built>)"; "" before
  * the first solve.  The string lives until the next solve or cache build. */
 FAP_API const char *fap_graph_stage1_name(const fap_dgraph *g);
 
