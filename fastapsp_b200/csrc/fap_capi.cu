@@ -294,22 +294,28 @@ struct ElimBuf {
         {plan.loc.data(), plan.loc.size() * 4},   {plan.inv.data(), plan.inv.size() * 4},
         {plan.eptr.data(), plan.eptr.size() * 4}, {plan.ecol.data(), plan.ecol.size() * 4},
         {plan.eend.data(), plan.eend.size() * 4}, {plan.w0.data(), plan.w0.size() * 4},
-        {plan.lev.data(), plan.lev.size() * 4},   {nullptr, plan.ecol.size() * sizeof(int2)}};
-    size_t off[9], bytes = 0;
-    for (int i = 0; i < 9; i++) {
+        {plan.lev.data(), plan.lev.size() * 4},   {plan.units.data(), plan.units.size() * sizeof(ElimUnit)},
+        {plan.glev.data(), plan.glev.size() * 4}, {plan.rows8.data(), plan.rows8.size() * 4},
+        {plan.list.data(), plan.list.size() * 2}, {plan.sloc.data(), plan.sloc.size() * 4},
+        {plan.chunks.data(), plan.chunks.size() * sizeof(ElimChunk)}, {nullptr, plan.ecol.size() * sizeof(int2)}};
+    constexpr int N = sizeof(src) / sizeof(src[0]);
+    size_t off[N], bytes = 0;
+    for (int i = 0; i < N; i++) {
       off[i] = bytes;
       bytes += (src[i].bytes + 255) / 256 * 256;
     }
     FAP_TRY(buf.ensure(std::max<size_t>(bytes, 256)));
-    std::vector<char> host(off[8]);
-    for (int i = 0; i < 8; i++)
+    std::vector<char> host(off[N - 1]);
+    for (int i = 0; i + 1 < N; i++)
       if (src[i].bytes > 0) std::memcpy(host.data() + off[i], src[i].p, src[i].bytes);
     FAP_CK(cudaMemcpy(buf.p, host.data(), host.size(), cudaMemcpyHostToDevice));
     char *d = buf.as<char>();
     auto at = [&](int i) { return reinterpret_cast<const int32_t *>(d + off[i]); };
     dev = ElimDev{reinterpret_cast<const ElimPart *>(d), at(1), at(2), at(3), at(4), at(5), at(6), at(7),
-                  reinterpret_cast<int2 *>(d + off[8]), (int32_t)plan.parts.size(), plan.max_s, plan.max_b,
-                  plan.max_nent, plan.max_nlev};
+                  reinterpret_cast<const ElimUnit *>(d + off[8]), at(9), at(10), at(12),
+                  reinterpret_cast<const uint16_t *>(d + off[11]),
+                  reinterpret_cast<const ElimChunk *>(d + off[13]), reinterpret_cast<int2 *>(d + off[N - 1]), (int32_t)plan.parts.size(), plan.max_s, plan.max_b,
+                  plan.max_nent, plan.max_nlev, plan.max_chunk16, plan.max_chunks};
     return FAP_OK;
   }
 };
@@ -431,6 +437,12 @@ struct fap_dgraph {
   ElimBuf el, el2;
   std::vector<int32_t> barcs;
   DevBuf d_barcs, d_elist, d_eoff;
+  // Parts of the prepared batch whose inner rows the group merge makes
+  // (plan part, batch index), and its coefficients (ElimMerge).
+  std::vector<int2> merge;
+  bool last_merge = false;
+  int32_t merge_units = 0, merge_slots = 0;
+  DevBuf d_merge, d_coef32, d_coef16, d_far;
   std::vector<int32_t> boff;
   std::vector<int32_t> bpcol;  // boundary columns of dB padded per part to multiples of 4 (prefix sums)
   bool last_bmethod = false;   // the prepared batch uses it
@@ -796,7 +808,7 @@ extern "C" int fap_graph_destroy(fap_dgraph *G) try {
     if (G->gexec) cudaGraphExecDestroy(G->gexec);
     G->el.release();
     G->el2.release();
-    for (DevBuf *b : {&G->d_barcs, &G->d_elist, &G->d_eoff, &G->ro, &G->col, &G->w, &G->ro_s, &G->col_s, &G->w_s, &G->sssp_scratch, &G->d_thin,
+    for (DevBuf *b : {&G->d_barcs, &G->d_elist, &G->d_eoff, &G->d_merge, &G->d_coef32, &G->d_coef16, &G->d_far, &G->ro, &G->col, &G->w, &G->ro_s, &G->col_s, &G->w_s, &G->sssp_scratch, &G->d_thin,
                       &G->d_gid, &G->d_st2ed, &G->d_ed2st, &G->D, &G->F, &G->d_parts, &G->d_work,
                       &G->d_src, &G->d_srcrows, &G->d_status, &G->d_checks, &G->staging, &G->P,
                       &G->d_tro, &G->d_tcol, &G->d_tw, &G->d_dB, &G->d_bpart, &G->d_brows, &G->d_FB,
@@ -1324,10 +1336,33 @@ int run_elim(fap_dgraph *G, const PartDesc *dp, int count, int max_s, int32_t *F
   return FAP_OK;
 }
 
+// Whether part p's inner rows come from the group merge instead of the
+// min-plus tiles: its padded relaxations have to be at most half of the
+// tiles' inner x b.
+bool merge_ok(const fap_dgraph *G, int32_t p) {
+  return elim_merge_fits(G->el.plan, G->el.plan.parts[p - 1].nslots) && G->vnum[p] > G->bnum[p] &&
+         2 * G->el.plan.group_work[p - 1] <= (int64_t)(G->vnum[p] - G->bnum[p]) * G->bnum[p];
+}
+
+// The batch's group merge (launch_elim_coef, launch_elim_merge) from the
+// parts' closed matrices F.
+int run_merge(fap_dgraph *G, const PartDesc *dp, const int32_t *F, int64_t *L) {
+  if (G->merge.empty()) return FAP_OK;
+  cudaStream_t st = G->ctx->stream;
+  const ElimMerge m{G->d_merge.as<const int2>(), (int32_t)G->merge.size(), G->d_coef32.as<int4>(),
+                    G->d_coef16.as<int4>(), G->d_far.as<int32_t>(),
+                    G->pack16 ? G->d_pk_tiles.as<unsigned long long>() : nullptr};
+  FAP_CK(launch_elim_coef(G->el.dev, m, dp, F, G->merge_units, st, L));
+  FAP_CK(launch_elim_merge(G->el.dev, m, dp, F, G->n, G->D.as<int32_t>(), G->ldD, G->d_gid.as<const int32_t>(),
+                           G->d_ed2st.as<const int32_t>(), G->merge_slots, st, L));
+  return FAP_OK;
+}
+
 // Builds (or reuses) the batch descriptors for the requested parts.
-int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, bool bmethod, bool elim) {
+int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, bool bmethod, bool elim,
+                  bool merge) {
   const bool same = (ids == G->last_ids) && (cached == G->last_cached) && (bmethod == G->last_bmethod) &&
-                    (elim == G->last_elim);
+                    (elim == G->last_elim) && (merge == G->last_merge);
   if (same) return FAP_OK;
   // The descriptors change from here on: until they are complete no batch
   // counts as prepared, so a failure below forces a full rebuild next time.
@@ -1358,6 +1393,8 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
   G->part_work_end.clear();
   G->thin.clear();
   G->thin_pos.clear();
+  G->merge.clear();
+  G->merge_units = G->merge_slots = 0;
   // Floyd arena: equal padded squares (one tensor map describes all parts);
   // with the resident cache, the parts' closed matrices in the cache.
   int32_t ldf = kFloydTile;
@@ -1395,7 +1432,14 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
       G->thin.push_back((int32_t)i);
     } else {
       G->thin_pos.push_back(-1);
-      for (int32_t m0 = 0; m0 < d.s - d.b; m0 += kMinplusBM) G->work.push_back(MPWork{(int32_t)i, m0});
+      if (merge && merge_ok(G, p)) {
+        G->merge.push_back(make_int2(p - 1, (int)i));
+        const ElimPart &q = G->el.plan.parts[p - 1];
+        G->merge_units = std::max(G->merge_units, G->el.plan.glev[q.glev_off + q.gnlev] - G->el.plan.glev[q.glev_off]);
+        G->merge_slots = std::max(G->merge_slots, q.nslots);
+      } else {
+        for (int32_t m0 = 0; m0 < d.s - d.b; m0 += kMinplusBM) G->work.push_back(MPWork{(int32_t)i, m0});
+      }
     }
     G->part_work_end.push_back((int32_t)G->work.size());
   }
@@ -1414,6 +1458,17 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
   if (!cached && !bmethod)  // (the plain form runs the frontier SSSP per part whatever the form)
     FAP_TRY(G->sssp_scratch.ensure_async(
         (size_t)std::max(sssp_scratch_rows(G->n, (int)G->src.size()), 1) * (size_t)G->n * 4, st));
+  if (!G->merge.empty()) {
+    const ElimPlan &pl = G->el.plan;
+    FAP_TRY(G->d_merge.ensure_async(G->merge.size() * sizeof(int2), st));
+    FAP_TRY(G->d_coef32.ensure_async(std::max<size_t>((size_t)pl.stream16, 1) * 16, st));
+    FAP_TRY(G->d_coef16.ensure_async(std::max<size_t>((size_t)pl.stream16, 1) * 16, st));
+    FAP_TRY(G->d_far.ensure_async(pl.parts.size() * 4, st));
+    if (G->pack16 && !G->d_pk_tiles.p) {
+      FAP_TRY(G->d_pk_tiles.ensure_async(2 * sizeof(unsigned long long), st));
+      FAP_CK(cudaMemsetAsync(G->d_pk_tiles.p, 0, 2 * sizeof(unsigned long long), st));
+    }
+  }
   G->pk = Pack16{};
   if (G->pack16 && G->dtype == FAP_DTYPE_I32 && !G->work.empty()) {
     const size_t np = G->parts.size();
@@ -1486,6 +1541,8 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
   FAP_CK(cudaMemcpy(G->d_parts.p, G->parts.data(), G->parts.size() * sizeof(PartDesc), cudaMemcpyHostToDevice));
   if (!G->work.empty())
     FAP_CK(cudaMemcpy(G->d_work.p, G->work.data(), G->work.size() * sizeof(MPWork), cudaMemcpyHostToDevice));
+  if (!G->merge.empty())
+    FAP_CK(cudaMemcpy(G->d_merge.p, G->merge.data(), G->merge.size() * sizeof(int2), cudaMemcpyHostToDevice));
   if (!G->thin.empty())
     FAP_CK(cudaMemcpy(G->d_thin.p, G->thin.data(), G->thin.size() * 4, cudaMemcpyHostToDevice));
   if (G->pk.s16 != nullptr)
@@ -1500,6 +1557,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
   G->last_cached = cached;
   G->last_bmethod = bmethod;
   G->last_elim = elim;
+  G->last_merge = merge;
   G->epoch++;
   return FAP_OK;
 }
@@ -1647,6 +1705,7 @@ int run_solve(fap_dgraph *G, int mode) {
       FAP_CK(record_event(c->ev[3], st));
       FAP_CK(launch_minplus_thin<T>(dp, G->d_thin.as<int32_t>(), (int)G->thin.size(), G->max_s, G->n, F, D,
                                     G->ldD, gid, ed2st, st, &L));
+    if constexpr (std::is_same<T, int32_t>::value) FAP_TRY(run_merge(G, dp, F, &L));
       FAP_CK(launch_minplus_parts<T>(dp, np, dw, (int)G->work.size(), G->n, F, G->max_ldf, D, G->ldD,
                                      G->max_rows, gid, ed2st, status, st, &L, pack16_of(G)));
       if (G->paths) FAP_TRY(launch_paths<T>(G, dp, np, G->max_s, F, &L));
@@ -1672,6 +1731,7 @@ int run_solve(fap_dgraph *G, int mode) {
     FAP_CK(record_event(c->ev[3], st));
     FAP_CK(launch_minplus_thin<T>(dp, G->d_thin.as<int32_t>(), (int)G->thin.size(), G->max_s, G->n, F, D,
                                   G->ldD, gid, ed2st, st, &L));
+    if constexpr (std::is_same<T, int32_t>::value) FAP_TRY(run_merge(G, dp, F, &L));
     FAP_CK(launch_minplus_parts<T>(dp, np, dw, (int)G->work.size(), G->n, F, G->max_ldf, D, G->ldD,
                                    G->max_rows, gid, ed2st, status, st, &L, pack16_of(G)));
     if (G->paths) FAP_TRY(launch_paths<T>(G, dp, np, G->max_s, F, &L));
@@ -1687,6 +1747,7 @@ int run_solve(fap_dgraph *G, int mode) {
     FAP_CK(record_event(c->ev[3], st));
     FAP_CK(launch_minplus_thin<T>(dp, G->d_thin.as<int32_t>(), (int)G->thin.size(), G->max_s, G->n, cF, D,
                                   G->ldD, gid, ed2st, st, &L));
+    if constexpr (std::is_same<T, int32_t>::value) FAP_TRY(run_merge(G, dp, cF, &L));
     FAP_CK(launch_minplus_parts<T>(dp, (int)G->K, dw, (int)G->work.size(), G->n, cF, G->cache_ldf, D,
                                    G->ldD, G->max_rows, gid, ed2st, status, st, &L, pack16_of(G)));
     if (G->paths) FAP_TRY(launch_paths<T>(G, dp, np, G->max_s, cF, &L));
@@ -1714,6 +1775,7 @@ int run_solve(fap_dgraph *G, int mode) {
     FAP_CK(record_event(c->ev[3], st));
     FAP_CK(launch_minplus_thin<T>(dp, G->d_thin.as<int32_t>(), (int)G->thin.size(), G->max_s, G->n, F, D,
                                   G->ldD, gid, ed2st, st, &L));
+    if constexpr (std::is_same<T, int32_t>::value) FAP_TRY(run_merge(G, dp, F, &L));
     if (mp_in_queue == 0)
       FAP_CK(launch_minplus_parts<T>(dp, np, dw, (int)G->work.size(), G->n, F, G->max_ldf, D, G->ldD,
                                      G->max_rows, gid, ed2st, status, st, &L, pack16_of(G)));
@@ -1801,7 +1863,8 @@ extern "C" int fap_solve(fap_dgraph *G, const int32_t *parts, int32_t count, int
     for (const int32_t p : ids) sources += G->bnum[p];
   const bool elim = !cached && mode == FAP_MODE_BATCHED && elim_ok(G, sources);
   const bool bmethod = elim || (!cached && mode == FAP_MODE_BATCHED && all_parts && bmethod_ok(G));
-  FAP_TRY(prepare_batch(G, ids, cached, bmethod, elim));
+  const bool merge = mode == FAP_MODE_BATCHED && G->eliminate && G->el.plan.ok;
+  FAP_TRY(prepare_batch(G, ids, cached, bmethod, elim, merge));
   int rc = FAP_OK;
   cudaStream_t st = G->ctx->stream;
   // (the tiled SSSP form tests convergence on the host: not capturable)
@@ -2647,7 +2710,8 @@ extern "C" int fap_graph_device_bytes(const fap_dgraph *G, int64_t *bytes) try {
                           &G->d_bDt, &G->d_bact, &G->d_bpact, &G->d_bgpart, &G->d_bpcolmap, &G->d_grow,
                           &G->d_bTc, &G->d_pk_off, &G->d_pk_range, &G->d_pk_maxa, &G->d_pk_tiles, &G->d_pk_s16,
                           &G->d_pk_at, &G->d_pk_krow, &G->d_xk_off, &G->d_xk_range, &G->d_xk_maxb, &G->d_xk_tiles,
-                          &G->d_xk_ap, &G->d_xk_bd, &G->d_barcs, &G->d_elist, &G->d_eoff})
+                          &G->d_xk_ap, &G->d_xk_bd, &G->d_barcs, &G->d_elist, &G->d_eoff, &G->d_merge, &G->d_coef32, &G->d_coef16,
+                          &G->d_far})
     t += (int64_t)b->bytes;
   t += (int64_t)(G->el.buf.bytes + G->el2.buf.bytes);
   *bytes = t;

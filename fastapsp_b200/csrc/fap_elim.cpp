@@ -15,6 +15,13 @@ struct PartPlan {
   bool ok = false;
   int32_t b = 0, boff = 0;
   std::vector<int32_t> loc, inv, eptr, ecol, w0, lev;
+  std::vector<ElimUnit> units;
+  std::vector<int32_t> glev, rows8;
+  std::vector<uint16_t> list;
+  std::vector<int32_t> sloc;
+  std::vector<ElimChunk> chunks;
+  int32_t stream16 = 0;
+  int64_t group_work = 0;
 };
 
 // Least-degree elimination of one part on bitset rows: joining v's
@@ -119,6 +126,93 @@ void eliminate(const ElimGraph &g, PartPlan *out) {
   out->ok = true;
 }
 
+// Separator groups from the elimination order (plan numbers descending).  A
+// group's cost is its chunks of four rows times its list, plus kChunkCost
+// entries' worth for storing the rows.
+constexpr int64_t kChunkCost = 6;
+
+void group_rows(PartPlan *q) {
+  const int32_t s = (int32_t)q->loc.size(), b = q->b;
+  auto deg = [&](int32_t v) { return q->eptr[v + 1] - q->eptr[v]; };
+  auto cost = [&](int64_t g, int64_t u) { return (g + 3) / 4 * (u + kChunkCost); };
+  std::vector<int32_t> size(s, 0), into(s, -1), par(s, -1);
+  std::vector<std::vector<int32_t>> child(s);
+  for (int32_t v = s - 1; v >= b; v--) {
+    size[v] = 1;
+    for (int32_t c : child[v])
+      if (cost(size[v] + size[c], deg(v)) <= cost(size[v], deg(v)) + cost(size[c], deg(c))) {
+        size[v] += size[c];
+        into[c] = v;
+      }
+    if (deg(v) > 0 && q->ecol[q->eptr[v]] >= b) {
+      par[v] = q->ecol[q->eptr[v]];
+      child[par[v]].push_back(v);
+    }
+  }
+  std::vector<int32_t> rep(s, -1), lev(s, -1);
+  std::vector<std::vector<int32_t>> rows(s);
+  int32_t nlev = 0;
+  for (int32_t v = b; v < s; v++) {
+    rep[v] = into[v] >= 0 ? rep[into[v]] : v;
+    rows[rep[v]].push_back(v);
+    if (rep[v] == v) {
+      lev[v] = par[v] >= 0 ? lev[rep[par[v]]] + 1 : 0;
+      nlev = std::max(nlev, lev[v] + 1);
+    }
+  }
+  // slots: the boundary vertices and every row that a list names
+  std::vector<int32_t> slot(s, -1);
+  for (int32_t v = b; v < s; v++)
+    if (rep[v] == v)
+      for (int32_t i = q->eptr[v]; i < q->eptr[v + 1]; i++) slot[q->ecol[i]] = 0;
+  for (int32_t v = 0; v < s; v++)
+    if (v < b || slot[v] == 0) {
+      slot[v] = (int32_t)q->sloc.size();
+      q->sloc.push_back(q->loc[v]);
+    }
+  std::vector<std::vector<ElimUnit>> units(nlev);
+  for (int32_t v = b; v < s; v++) {
+    if (rep[v] != v) continue;
+    const int32_t list = (int32_t)q->list.size(), nu = (deg(v) + 3) / 4 * 4;
+    for (int32_t i = 0; i < nu; i++)
+      q->list.push_back((uint16_t)slot[q->ecol[q->eptr[v] + std::min(i, deg(v) - 1)]]);
+    for (size_t r = 0; r < rows[v].size(); r += kElimUnitRows) {
+      const int32_t k = (int32_t)std::min<size_t>(kElimUnitRows, rows[v].size() - r);
+      const bool wide = k > 4;
+      units[lev[v]].push_back(ElimUnit{(int32_t)q->rows8.size() / 2, list, nu | (wide ? kElimWide : 0), 0, 0, 0});
+      for (int32_t i = 0; i < kElimUnitRows; i++) {
+        q->rows8.push_back(i < k ? slot[rows[v][r + i]] : -1);
+        q->rows8.push_back(i < k ? q->loc[rows[v][r + i]] : -1);
+      }
+      q->group_work += (int64_t)nu * (wide ? 8 : 4);
+    }
+  }
+  q->glev.push_back(0);
+  for (auto &u : units) {  // longest first: the last units of a level are short
+    std::stable_sort(u.begin(), u.end(),
+                     [](const ElimUnit &x, const ElimUnit &y) { return elim_body16(x.nu) > elim_body16(y.nu); });
+    for (size_t i = 0; i < u.size();) {
+      size_t k = i;
+      int32_t bodies = 0;
+      while (k < u.size() && (k == i || bodies + elim_body16(u[k].nu) + (int32_t)(k - i + 2) / 2 <= kElimChunk16))
+        bodies += elim_body16(u[k++].nu);
+      const int32_t off = q->stream16, heads = (int32_t)(k - i + 1) / 2;
+      q->chunks.push_back(ElimChunk{off, heads + bodies, (int32_t)(k - i), 0});
+      int32_t body = off + heads;
+      for (size_t j = i; j < k; j++) {
+        u[j].head = 2 * off + (int32_t)(j - i);
+        u[j].body = body;
+        u[j].chunk = off;
+        body += elim_body16(u[j].nu);
+      }
+      q->stream16 = body;
+      i = k;
+    }
+    q->units.insert(q->units.end(), u.begin(), u.end());
+    q->glev.push_back((int32_t)q->units.size());
+  }
+}
+
 }  // namespace
 
 void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, int threads, ElimPlan *out) {
@@ -137,6 +231,7 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
         pp[p].b = g.b;
         if (g.s <= kElimMaxS) eliminate(g, &pp[p]);
         if (!pp[p].ok) dense = true;
+        else if (g.b > 0) group_rows(&pp[p]);
       }
     } catch (...) {
       failed = true;
@@ -173,6 +268,31 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
     d.nent = (int32_t)q.ecol.size();
     d.lev_off = (int32_t)out->lev.size();
     d.nlev = (int32_t)q.lev.size() - 1;
+    d.glev_off = (int32_t)out->glev.size();
+    d.gnlev = std::max(0, (int32_t)q.glev.size() - 1);
+    d.stream_off = (int32_t)out->stream16;
+    d.chunk_off = (int32_t)out->chunks.size();
+    d.nchunks = (int32_t)q.chunks.size();
+    for (const ElimChunk &c : q.chunks) out->max_chunk16 = std::max(out->max_chunk16, c.n16);
+    out->max_chunks = std::max(out->max_chunks, d.nchunks);
+    out->chunks.insert(out->chunks.end(), q.chunks.begin(), q.chunks.end());
+    d.nslots = (int32_t)q.sloc.size();
+    d.sloc_off = (int32_t)out->sloc.size();
+    out->sloc.insert(out->sloc.end(), q.sloc.begin(), q.sloc.end());
+    out->max_slots = std::max(out->max_slots, d.nslots);
+    const int32_t rows0 = (int32_t)out->rows8.size() / 2, list0 = (int32_t)out->list.size(),
+                  unit0 = (int32_t)out->units.size();
+    for (ElimUnit u : q.units) {
+      u.rows += rows0;
+      u.list += list0;
+      out->units.push_back(u);
+    }
+    for (int32_t l : q.glev) out->glev.push_back(unit0 + l);
+    out->rows8.insert(out->rows8.end(), q.rows8.begin(), q.rows8.end());
+    out->list.insert(out->list.end(), q.list.begin(), q.list.end());
+    out->stream16 += q.stream16;
+    out->group_work.push_back(q.group_work);
+    out->max_units = std::max(out->max_units, (int32_t)q.units.size());
     out->parts.push_back(d);
     out->loc.insert(out->loc.end(), q.loc.begin(), q.loc.end());
     out->inv.insert(out->inv.end(), q.inv.begin(), q.inv.end());
@@ -188,7 +308,7 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
     out->max_nlev = std::max(out->max_nlev, d.nlev);
   }
   out->nent = (int64_t)out->ecol.size();
-  out->ok = out->nent < INT32_MAX / 2;
+  out->ok = out->nent < INT32_MAX / 2 && out->stream16 < INT32_MAX / 2;
 }
 
 void elim_offsets(int64_t ld, ElimPlan *plan) {

@@ -270,6 +270,300 @@ __global__ void __launch_bounds__(kElimSweepThreads)
   }
 }
 
+// The groups' streams: a warp per unit, a lane per list entry.
+__global__ void __launch_bounds__(256)
+    elim_coef_kernel(ElimDev e, ElimMerge m, const PartDesc *__restrict__ parts, const int32_t *__restrict__ F) {
+  const int2 w = m.list[blockIdx.y];
+  const ElimPart P = e.parts[w.x];
+  const PartDesc pd = parts[w.y];
+  const int32_t *Fp = F + pd.f_off, *sloc = e.sloc + P.sloc_off;
+  const int lane = threadIdx.x % 32;
+  int4 *s32 = m.s32 + P.stream_off, *s16 = m.s16 + P.stream_off;
+  int far = 0;
+  const int u0 = e.glev[P.glev_off], u1 = e.glev[P.glev_off + P.gnlev];
+  for (int i = u0 + (blockIdx.x * blockDim.x + threadIdx.x) / 32; i < u1; i += gridDim.x * blockDim.x / 32) {
+    const ElimUnit U = e.units[i];
+    const int nu = U.nu & ~kElimWide, chunks = U.nu & kElimWide ? 2 : 1;
+    const int2 head = make_int2(U.body - U.chunk, U.nu);
+    const int2 *rows = reinterpret_cast<const int2 *>(e.rows8) + U.rows;
+    if (lane == 0) {
+      reinterpret_cast<int2 *>(s32)[U.head] = head;
+      reinterpret_cast<int2 *>(s16)[U.head] = head;
+    }
+    if (lane < kElimUnitRows) {
+      reinterpret_cast<int2 *>(s32 + U.body)[lane] = rows[lane];
+      reinterpret_cast<int2 *>(s16 + U.body)[lane] = rows[lane];
+    }
+    const int lists = U.body + kElimUnitRows / 2, coef = lists + nu / 4;
+    for (int k = lane; k < nu; k += 32) {
+      reinterpret_cast<int32_t *>(s32 + lists)[k] = e.list[U.list + k] * 128;
+      reinterpret_cast<int32_t *>(s16 + lists)[k] = e.list[U.list + k] * 128;
+    }
+    for (int t = lane; t < nu * chunks; t += 32) {
+      const int k = t / chunks, c = t - k * chunks;
+      const int u = sloc[e.list[U.list + k]];
+      int32_t x[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const int v = rows[4 * c + r].y;
+        x[r] = v < 0 ? kInf : __ldg(Fp + (int64_t)v * pd.ldf + u);
+      }
+      s32[coef + t] = make_int4(x[0], x[1], x[2], x[3]);
+#pragma unroll
+      for (int r = 0; r < 4; r++) x[r] = min(x[r], kMergeCap) * 0x10001;
+      s16[coef + t] = make_int4(x[0], x[1], x[2], x[3]);
+    }
+  }
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < (P.s - P.b) * P.b; t += gridDim.x * blockDim.x) {
+    const int32_t x = __ldg(Fp + (int64_t)(P.b + t / P.b) * pd.ldf + t % P.b);
+    if (x < kInf) far = max(far, x);
+  }
+  far = __reduce_max_sync(0xffffffffu, far);
+  if (lane == 0 && far > 0) atomicMax(m.maxA + w.x, far);
+}
+
+// How a strip sits in shared memory: kMergePacked, a lane's word is two
+// columns in 16 unsigned bits (shifted by the column's offset and clamped at
+// kMergeCap); kMergePair, a lane holds two columns as int32; kMergeOne, one.
+enum MergeMode { kMergeOne, kMergePair, kMergePacked };
+
+// Where a strip's rows go: the lane's column or columns of the block's rows in
+// D, with the own-part columns taken from F (jx, jy: local index or -1).
+struct MergeOut {
+  char *D;       // first row, the lane's first column
+  int32_t ld;    // bytes between rows
+  const int32_t *F;
+  int32_t ldf;
+  int jx, jy, ox, oy;  // ox, oy: packed columns' offsets
+};
+
+// One unit of NR rows on a warp.  Per list entry one load of the strip serves
+// NR rows; body: the unit's rows, list and coefficients in shared memory; st:
+// the lane's place in row 0.  OWN: the strip has own-part columns; their values
+// are asked for before the relaxations, which hide the latency.
+template <int MODE, int NR, bool OWN>
+__device__ __forceinline__ void merge_unit(char *st, const int4 *body, int nu, const MergeOut &o) {
+  constexpr bool PK = MODE == kMergePacked, TWO = MODE == kMergePair;
+  constexpr int LD = TWO ? 256 : 128;  // bytes of a strip's row; the lists are in units of 128
+  const int4 *list = body + kElimUnitRows / 2, *coef = list + nu / 4;
+  int acc[NR], acc2[TWO ? NR : 1], fx[OWN ? NR : 1], fy[OWN && MODE != kMergeOne ? NR : 1];
+  if (OWN) {
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+      const int v = max(reinterpret_cast<const int2 *>(body)[r].y, 0);
+      const int32_t *f = o.F + (int64_t)v * o.ldf;
+      if (o.jx >= 0) fx[r] = __ldg(f + o.jx);
+      if (MODE != kMergeOne && o.jy >= 0) fy[MODE != kMergeOne ? r : 0] = __ldg(f + o.jy);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < NR; r++) {
+    acc[r] = PK ? kMergeCap * 0x10001 : kInf;
+    if (TWO) acc2[TWO ? r : 0] = kInf;
+  }
+  auto relax = [](int x, int y, int z) -> int {
+    if (PK) return (int)__viaddmin_u16x2((unsigned)x, (unsigned)y, (unsigned)z);
+    return __viaddmin_s32(x, y, z);
+  };
+  auto step = [&](int u, const int4 *f) {
+    int x, y = 0;
+    if (TWO) {
+      const int2 t = *reinterpret_cast<const int2 *>(st + 2 * u);
+      x = t.x;
+      y = t.y;
+    } else {
+      x = *reinterpret_cast<const int *>(st + u);
+    }
+#pragma unroll
+    for (int g = 0; g < NR / 4; g++) {
+      const int4 a = f[g];
+      const int c[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        acc[4 * g + r] = relax(c[r], x, acc[4 * g + r]);
+        if (TWO) acc2[TWO ? 4 * g + r : 0] = relax(c[r], y, acc2[TWO ? 4 * g + r : 0]);
+      }
+    }
+  };
+#pragma unroll 1
+  for (const int4 *end = coef; list < end; list++, coef += NR) {
+    const int4 u = *list;
+    step(u.x, coef);
+    step(u.y, coef + NR / 4);
+    step(u.z, coef + 2 * (NR / 4));
+    step(u.w, coef + 3 * (NR / 4));
+  }
+#pragma unroll
+  for (int r = 0; r < NR; r++) {
+    const int2 v = reinterpret_cast<const int2 *>(body)[r];
+    if (v.y < 0) break;
+    int2 d = make_int2(acc[r], acc2[TWO ? r : 0]);
+    if (v.x >= 0) {
+      if (TWO) *reinterpret_cast<int2 *>(st + v.x * LD) = d;
+      else *reinterpret_cast<int *>(st + v.x * LD) = d.x;
+    }
+    if (PK) {
+      const int x = acc[r] & 0xffff, y = (int)((uint32_t)acc[r] >> 16);
+      d = make_int2(__viaddmin_s32(x, o.ox, kInf), __viaddmin_s32(y, o.oy, kInf));
+      if (x >= kMergeCap) d.x = kInf;
+      if (y >= kMergeCap) d.y = kInf;
+    }
+    if (OWN && o.jx >= 0) d.x = fx[r];
+    if (OWN && MODE != kMergeOne && o.jy >= 0) d.y = fy[MODE != kMergeOne ? r : 0];
+    char *row = o.D + (int64_t)v.y * o.ld;
+    if (MODE == kMergeOne) __stcs(reinterpret_cast<int *>(row), d.x);
+    else __stcs(reinterpret_cast<int2 *>(row), d);
+  }
+}
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// The part's chunks through a ring of kMergeRing buffers in shared memory,
+// copied asynchronously two chunks ahead; a chunk's units are independent, a
+// barrier ends every chunk.
+constexpr int kMergeRing = 3;
+template <int MODE, bool OWN>
+__device__ __forceinline__ void merge_stream(char *st, int4 *ring, int buf16, const ElimChunk *chunks, int nchunks,
+                                             const int4 *__restrict__ stream, const MergeOut &o) {
+  const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  auto fetch = [&](int c) {
+    if (c < nchunks) {
+      const ElimChunk k = chunks[c];
+      for (int i = threadIdx.x; i < k.n16; i += blockDim.x) cp_async16(ring + (c % kMergeRing) * buf16 + i, stream + k.off + i);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0);
+  fetch(1);
+  for (int c = 0; c < nchunks; c++) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // chunk c is here, and every warp is done with chunk c - 1
+    fetch(c + 2);
+    const int4 *buf = ring + (c % kMergeRing) * buf16;
+    const int n = chunks[c].nunits;
+    for (int i = warp; i < n; i += nwarps) {
+      const int2 head = reinterpret_cast<const int2 *>(buf)[i];
+      if (head.y & kElimWide) merge_unit<MODE, 8, OWN>(st, buf + head.x, head.y & ~kElimWide, o);
+      else merge_unit<MODE, 4, OWN>(st, buf + head.x, head.y, o);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+}
+
+constexpr int kMergeThreads = 384;
+constexpr int kMergeCols = 64;
+__host__ __device__ inline size_t merge_smem(int slots, int slot_bytes, int chunk16, int chunks) {
+  return (size_t)slots * slot_bytes + ((size_t)kMergeRing * chunk16 + chunks) * 16;
+}
+
+// Inner rows.  CTA (strip of 64 columns, listed part).  The boundary rows of
+// the strip give every column its least finite entry (off) and the strip its
+// range; the rows are relaxed in packed 16 bits where maxA + range < kMergeCap
+// (every inner row's shifted value is at most that sum, two values of at most
+// kMergeCap do not overflow, and one at kMergeCap means no path), else in
+// int32: two columns a lane (pair) where two CTAs still fit on an SM, else as
+// two strips of 32 columns.  A grid part's row takes 28 relaxations (its
+// boundary: 164), a geometric graph's 5 (27).  Bound by issue: about 100
+// instructions per packed row of 64 columns, of which 39 relax.  Merge of a
+// 256 x 256 grid 22.4 -> 12.8 ms, of a 60,000-vertex geometric graph 9.3 -> 5.7
+// (the min-plus tiles before); 384 threads of 85 registers, since at 56 the
+// pair form spills (9.7 ms).
+__global__ void __launch_bounds__(kMergeThreads, 2)
+    elim_merge_kernel(ElimDev e, ElimMerge m, const PartDesc *__restrict__ parts, const int32_t *__restrict__ F,
+                      int n, int32_t *D, int64_t ldD, const int32_t *__restrict__ graph_id,
+                      const int32_t *__restrict__ ed2st, int max_slots, int pair) {
+  extern __shared__ __align__(16) int32_t st[];
+  __shared__ int32_t lo[kMergeCols], hi[kMergeCols], own[kMergeCols];
+  __shared__ int range, any_own;
+  int4 *ring = reinterpret_cast<int4 *>(st + (size_t)max_slots * (pair ? 64 : 32));
+  ElimChunk *chunks = reinterpret_cast<ElimChunk *>(ring + (size_t)kMergeRing * e.max_chunk16);
+  const int2 w = m.list[blockIdx.y];
+  const ElimPart P = e.parts[w.x];
+  const PartDesc pd = parts[w.y];
+  const int64_t c0 = (int64_t)blockIdx.x * kMergeCols;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  int32_t *Dp = D + pd.row_base * ldD + c0;
+  for (int i = threadIdx.x; i < P.nchunks; i += blockDim.x) chunks[i] = e.chunks[P.chunk_off + i];
+  if (threadIdx.x == 0) range = any_own = 0;
+  if (threadIdx.x < kMergeCols) {
+    lo[threadIdx.x] = kInf;
+    hi[threadIdx.x] = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x < kMergeCols) {
+    const int64_t v = c0 + threadIdx.x;
+    int j = -1;
+    if (v < n && __ldg(graph_id + v) == pd.part) {
+      j = __ldg(ed2st + v) - pd.start;
+      any_own = 1;
+    }
+    own[threadIdx.x] = j;
+  }
+  if (m.tiles != nullptr) {
+    int mn[2] = {kInf, kInf}, mx[2] = {0, 0};
+#pragma unroll 4
+    for (int k = warp; k < P.b; k += nwarps) {
+      const int2 x = reinterpret_cast<const int2 *>(Dp + (int64_t)k * ldD)[lane];
+      mn[0] = min(mn[0], x.x);
+      mn[1] = min(mn[1], x.y);
+      if (x.x < kInf) mx[0] = max(mx[0], x.x);
+      if (x.y < kInf) mx[1] = max(mx[1], x.y);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+      atomicMin(&lo[2 * lane + t], mn[t]);
+      atomicMax(&hi[2 * lane + t], mx[t]);
+    }
+    __syncthreads();
+    if (threadIdx.x < kMergeCols && lo[threadIdx.x] < kInf) atomicMax(&range, hi[threadIdx.x] - lo[threadIdx.x]);
+  }
+  __syncthreads();
+  const bool pk = m.tiles != nullptr && range < kMergeCap && m.maxA[w.x] + range < kMergeCap;
+  if (threadIdx.x == 0 && m.tiles != nullptr) {
+    atomicAdd(m.tiles + 1, 1ull);
+    if (pk) atomicAdd(m.tiles, 1ull);
+  }
+  MergeOut o{reinterpret_cast<char *>(Dp + 2 * lane), (int32_t)(ldD * 4), F + pd.f_off, pd.ldf, 0, 0, 0, 0};
+  o.jx = own[2 * lane];
+  o.jy = own[2 * lane + 1];
+  char *lst = reinterpret_cast<char *>(st + lane);
+  if (pk) {
+    o.ox = lo[2 * lane];
+    o.oy = lo[2 * lane + 1];
+#pragma unroll 4
+    for (int k = warp; k < P.b; k += nwarps) {
+      const int2 x = reinterpret_cast<const int2 *>(Dp + (int64_t)k * ldD)[lane];
+      const int a = x.x >= kInf ? kMergeCap : min(x.x - o.ox, kMergeCap);
+      const int b = x.y >= kInf ? kMergeCap : min(x.y - o.oy, kMergeCap);
+      st[k * 32 + lane] = a | b << 16;
+    }
+    if (any_own) merge_stream<kMergePacked, true>(lst, ring, e.max_chunk16, chunks, P.nchunks, m.s16 + P.stream_off, o);
+    else merge_stream<kMergePacked, false>(lst, ring, e.max_chunk16, chunks, P.nchunks, m.s16 + P.stream_off, o);
+    return;
+  }
+  if (pair) {
+#pragma unroll 4
+    for (int k = warp; k < P.b; k += nwarps)
+      reinterpret_cast<int2 *>(st)[k * 32 + lane] = reinterpret_cast<const int2 *>(Dp + (int64_t)k * ldD)[lane];
+    lst = reinterpret_cast<char *>(st + 2 * lane);
+    if (any_own) merge_stream<kMergePair, true>(lst, ring, e.max_chunk16, chunks, P.nchunks, m.s32 + P.stream_off, o);
+    else merge_stream<kMergePair, false>(lst, ring, e.max_chunk16, chunks, P.nchunks, m.s32 + P.stream_off, o);
+    return;
+  }
+  for (int h = 0; h < 2; h++) {
+#pragma unroll 4
+    for (int k = warp; k < P.b; k += nwarps) st[k * 32 + lane] = Dp[(int64_t)k * ldD + 32 * h + lane];
+    o.D = reinterpret_cast<char *>(Dp + 32 * h + lane);
+    o.jx = own[32 * h + lane];
+    if (any_own) merge_stream<kMergeOne, true>(lst, ring, e.max_chunk16, chunks, P.nchunks, m.s32 + P.stream_off, o);
+    else merge_stream<kMergeOne, false>(lst, ring, e.max_chunk16, chunks, P.nchunks, m.s32 + P.stream_off, o);
+  }
+}
+
 template <class K>
 cudaError_t allow_smem(K kern, size_t smem) {
   return smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
@@ -353,6 +647,36 @@ cudaError_t launch_elim_expand(const ElimDev &e, const int64_t *rows, int nrows,
     *launches += 1;
     return cudaGetLastError();
   });
+}
+
+bool elim_merge_fits(const ElimPlan &p, int slots) {
+  return merge_smem(slots, 128, p.max_chunk16, p.max_chunks) <= kElimSmem;
+}
+
+cudaError_t launch_elim_coef(const ElimDev &e, const ElimMerge &m, const PartDesc *parts, const int32_t *F,
+                             int max_units, cudaStream_t stream, int64_t *launches) {
+  if (m.count <= 0) return cudaSuccess;
+  cudaError_t err = cudaMemsetAsync(m.maxA, 0, (size_t)e.nparts * sizeof(int32_t), stream);
+  if (err != cudaSuccess) return err;
+  elim_coef_kernel<<<dim3(std::max(1, std::min(16, (max_units + 7) / 8)), m.count), 256, 0, stream>>>(e, m, parts, F);
+  *launches += 1;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_elim_merge(const ElimDev &e, const ElimMerge &m, const PartDesc *parts, const int32_t *F, int n,
+                              int32_t *D, int64_t ldD, const int32_t *graph_id, const int32_t *ed2st, int max_slots,
+                              cudaStream_t stream, int64_t *launches) {
+  if (m.count <= 0) return cudaSuccess;
+  if (ldD % kMergeCols != 0 || ldD > INT32_MAX / 4) return cudaErrorInvalidValue;
+  const bool pair = merge_smem(max_slots, 256, e.max_chunk16, e.max_chunks) <= kElimHalf;
+  const size_t smem = merge_smem(max_slots, pair ? 256 : 128, e.max_chunk16, e.max_chunks);
+  if (smem > kElimSmem) return cudaErrorInvalidValue;
+  cudaError_t err = allow_smem(elim_merge_kernel, smem);
+  if (err != cudaSuccess) return err;
+  elim_merge_kernel<<<dim3((unsigned)(ldD / kMergeCols), m.count), kMergeThreads, smem, stream>>>(
+      e, m, parts, F, n, D, ldD, graph_id, ed2st, max_slots, pair ? 1 : 0);
+  *launches += 1;
+  return cudaGetLastError();
 }
 
 }  // namespace fapb

@@ -20,6 +20,8 @@
 #include <functional>
 #include <vector>
 
+#include "fap_internal.h"
+
 namespace fapb {
 
 // One part of the plan.  Its vertices are renumbered: 0..b-1 the boundary
@@ -35,7 +37,47 @@ struct ElimPart {
   int32_t lev_off;     // nlev + 1 level starts, first level = highest (next to the boundary)
   int32_t nlev;
   int32_t boff;        // first boundary index of the part
+  int32_t glev_off;    // gnlev + 1 level starts in units
+  int32_t gnlev;
+  int32_t stream_off;  // of the streams, in 16-byte words
+  int32_t chunk_off, nchunks;
+  int32_t nslots, sloc_off;
 };
+
+// Separator groups of the merge.  Rows eliminated one after the other are
+// gathered while that costs no more: a group G shares the list U = N+ of its
+// last vertex, which separates all of G from the rest, so with the parts'
+// closed distances F
+//   D[v][x] = min over u in U of F[v][u] + D[u][x]    for every v in G
+// and the rows of a group are independent of one another: about ten levels
+// instead of a hundred on grid parts, and every row u read serves four rows.
+// Only boundary rows and rows that a list names (slots: boundary vertices
+// first) stay in shared memory; the others, about two thirds on grid parts, go
+// to memory straight from registers.  A unit is up to eight rows of a group;
+// its list (slots) is padded to a multiple of four by repeating its last entry.
+//
+// The merge reads a part's units as a stream of chunks (consecutive units of
+// one level, about kElimChunk16 * 16 bytes): the units' heads (body's offset in
+// the chunk in 16-byte words, nu), then their bodies (rows, list as byte
+// offsets into the strip, coefficients; elim_body16 words).  launch_elim_coef writes the stream.
+struct ElimUnit {
+  int32_t rows;   // first of kElimUnitRows rows: slot or -1, local index or -1
+  int32_t list;   // first list entry
+  int32_t nu;     // list entries, a multiple of four; kElimWide: eight rows, else at most four
+  int32_t head;   // of the stream, in 8-byte words
+  int32_t body;   // of the stream, in 16-byte words
+  int32_t chunk;  // start of its chunk in the stream, in 16-byte words
+};
+struct ElimChunk {
+  int32_t off, n16, nunits, pad_;  // in 16-byte words
+};
+constexpr int32_t kElimChunk16 = 512;
+constexpr int32_t kElimWide = 1 << 30;
+constexpr int kElimUnitRows = 8;
+__host__ __device__ inline int32_t elim_body16(int32_t nu) {
+  const int32_t k = nu & ~kElimWide;
+  return kElimUnitRows / 2 + k / 4 + k * (nu & kElimWide ? 2 : 1);
+}
 
 struct ElimPlan {
   bool ok = false;
@@ -46,7 +88,15 @@ struct ElimPlan {
   std::vector<int32_t> eend;       // end of the entry's vertex, relative to ent_off
   std::vector<int32_t> w0;         // weight of the edge (v, u), or the sentinel
   std::vector<int32_t> lev;
-  int32_t max_s = 0, max_b = 0, max_nent = 0, max_nlev = 0;
+  std::vector<ElimUnit> units;
+  std::vector<int32_t> glev, rows8;  // rows8: pairs (slot, local index)
+  std::vector<uint16_t> list;
+  std::vector<int32_t> sloc;  // local index of every slot, parts one after the other (sloc_off)
+  std::vector<ElimChunk> chunks;
+  int64_t stream16 = 0;
+  int32_t max_chunk16 = 0, max_chunks = 0;
+  std::vector<int64_t> group_work;  // per part: list entries times padded rows
+  int32_t max_s = 0, max_b = 0, max_nent = 0, max_nlev = 0, max_units = 0, max_slots = 0;
   int64_t nent = 0;
 };
 
@@ -72,8 +122,12 @@ void elim_offsets(int64_t ld, ElimPlan *plan);
 struct ElimDev {
   const ElimPart *parts;
   const int32_t *loc, *inv, *eptr, *ecol, *eend, *w0, *lev;
+  const ElimUnit *units;
+  const int32_t *glev, *rows8, *sloc;
+  const uint16_t *list;
+  const ElimChunk *chunks;
   int2 *ent;  // {plan number of u, W(v, u)}, written by launch_elim_up
-  int32_t nparts, max_s, max_b, max_nent, max_nlev;
+  int32_t nparts, max_s, max_b, max_nent, max_nlev, max_chunk16, max_chunks;
 };
 
 // M (ld): the sentinel on nfill x nfill, 0 on the first nb diagonal entries,
@@ -100,5 +154,28 @@ cudaError_t launch_elim_close(const ElimDev &e, const int32_t *list, const int64
 cudaError_t launch_elim_expand(const ElimDev &e, const int64_t *rows, int nrows, const int32_t *dB, int64_t ldB,
                                const int32_t *vid, int n, int32_t *D, int64_t ldD, cudaStream_t stream,
                                int64_t *launches);
+
+// The listed parts' (pairs plan part, batch index of its PartDesc) streams:
+// coefficients F[v][u] as int32 in s32 and, clamped at kMergeCap with both
+// halves equal, in s16; maxA[plan part] = the largest finite distance from an
+// inner to a boundary vertex.
+constexpr int32_t kMergeCap = 32767;  // twice fits in 16 unsigned bits
+struct ElimMerge {
+  const int2 *list;
+  int32_t count;
+  int4 *s32, *s16;
+  int32_t *maxA;
+  unsigned long long *tiles;  // [2] strips run packed, strips run; null: int32 only
+};
+cudaError_t launch_elim_coef(const ElimDev &e, const ElimMerge &m, const PartDesc *parts, const int32_t *F,
+                             int max_units, cudaStream_t stream, int64_t *launches);
+
+// Inner rows of the listed parts' blocks from their boundary rows in D
+// (stage 3); own columns from F.
+cudaError_t launch_elim_merge(const ElimDev &e, const ElimMerge &m, const PartDesc *parts, const int32_t *F, int n,
+                              int32_t *D, int64_t ldD, const int32_t *graph_id, const int32_t *ed2st, int max_slots,
+                              cudaStream_t stream, int64_t *launches);
+// Whether a part with that many slots fits in a CTA's shared memory.
+bool elim_merge_fits(const ElimPlan &p, int slots);
 
 }  // namespace fapb

@@ -37,6 +37,17 @@ def _zeros():
     return el
 
 
+def _grid_heavy():
+    """Distances too long for the packed rows, on 2,048-vertex parts."""
+    el = G.grid_graph(64, 64, wmin=1, wmax=200000, seed=30)
+    return el
+
+
+def _grid_forest():
+    """A grid without a third of its edges: unreachable vertices beside wide boundaries."""
+    return G.grid_graph(60, 61, drop_frac=0.33, wmin=1, wmax=50, seed=31)
+
+
 CASES = {  # name: (graph, parts)
     "road": (lambda: G.road_graph(3001, seed=20), 5),
     "tiny_parts": (lambda: G.road_graph(97, seed=24), 16),
@@ -46,6 +57,8 @@ CASES = {  # name: (graph, parts)
     "rgg": (lambda: G.random_geometric_graph(5000, 3.7, seed=25), 6),
     "grid_small_parts": (lambda: G.grid_graph(40, 37, extra_frac=0.01, wmin=1, wmax=100, seed=26), 9),
     "grid_wide": (lambda: G.grid_graph(64, 64, wmin=1, wmax=100, seed=27), 2),   # 2,048-vertex parts
+    "grid_heavy": (_grid_heavy, 2),
+    "grid_forest": (_grid_forest, 4),
     "grid_floyd": (lambda: G.grid_graph(100, 100, extra_frac=0.01, wmin=1, wmax=100, seed=28), 40),
 }
 
