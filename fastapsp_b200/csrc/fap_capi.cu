@@ -1322,7 +1322,8 @@ int run_elim(fap_dgraph *G, const PartDesc *dp, int count, int max_s, int32_t *F
     FAP_CK(launch_elim_up(G->el2.dev, dB, nullptr, 0, st, L));
     FAP_CK(launch_elim_close(G->el2.dev, nullptr, off, 1, nb, nullptr, 0, dB, G->ldB, st, L));
   } else {
-    FAP_CK(launch_floyd_matrix<int32_t>(dB, G->ldB, (int)ceil_div(nb, kFloydTile), status, st, L, nb));
+    FAP_CK(launch_floyd_matrix<int32_t>(dB, G->ldB, (int)ceil_div(nb, kFloydTile), status, st, L, nb,
+                                        true));
   }
   FAP_CK(record_event(ev2, st));
   FAP_CK(launch_elim_close(G->el.dev, G->d_elist.as<const int32_t>(), off + 1, count, max_s, dB, G->ldB, F, ldf, st, L));
@@ -2226,19 +2227,15 @@ extern "C" int fap_op_floyd(fap_ctx *c, int dtype, int32_t s, void *mat, int64_t
   FAP_CK(cudaMemsetAsync(c->status.p, 0, sizeof(int), st));
   FAP_TRY(c->scratch.ensure((size_t)ldp * ldp * 4));
   int64_t L = 0;
-  // padded copy: sentinel everywhere, then the matrix
-  if (dtype == FAP_DTYPE_I32)
-    FAP_CK(launch_fill<int32_t>(c->scratch.as<int32_t>(), ldp, ldp, ldp, kInfI32, st, &L));
-  else
-    FAP_CK(launch_fill<float>(c->scratch.as<float>(), ldp, ldp, ldp, kInfF32, st, &L));
-  FAP_CK(cudaMemcpy2DAsync(c->scratch.p, (size_t)ldp * 4, mat, (size_t)ld * 4, (size_t)s * 4, (size_t)s,
-                           cudaMemcpyDeviceToDevice, st));
-  if (dtype == FAP_DTYPE_I32)
-    FAP_CK(launch_floyd_matrix<int32_t>(c->scratch.as<int32_t>(), ldp, (int)(ldp / kFloydTile),
-                                        c->status.as<int>(), st, &L));
-  else
-    FAP_CK(launch_floyd_matrix<float>(c->scratch.as<float>(), ldp, (int)(ldp / kFloydTile),
-                                      c->status.as<int>(), st, &L));
+  if (dtype == FAP_DTYPE_I32) {
+    int32_t *p = c->scratch.as<int32_t>();
+    FAP_CK(launch_pad_copy<int32_t>(p, ldp, static_cast<const int32_t *>(mat), ld, s, st, &L));
+    FAP_CK(launch_floyd_matrix<int32_t>(p, ldp, (int)(ldp / kFloydTile), c->status.as<int>(), st, &L, s));
+  } else {
+    float *p = c->scratch.as<float>();
+    FAP_CK(launch_pad_copy<float>(p, ldp, static_cast<const float *>(mat), ld, s, st, &L));
+    FAP_CK(launch_floyd_matrix<float>(p, ldp, (int)(ldp / kFloydTile), c->status.as<int>(), st, &L, s));
+  }
   FAP_CK(cudaMemcpy2DAsync(mat, (size_t)ld * 4, c->scratch.p, (size_t)ldp * 4, (size_t)s * 4, (size_t)s,
                            cudaMemcpyDeviceToDevice, st));
   c->launches += L;

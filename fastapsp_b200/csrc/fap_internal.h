@@ -203,10 +203,19 @@ cudaError_t launch_floyd_parts_multi(const PartDesc *parts, int nparts, int max_
 // Plain: one padded matrix (ld a multiple of kFloydTile, nb tiles per side
 // in use), one launch per phase per pivot block.  status may be null.  s:
 // the real rows and columns (the rest is padding holding the sentinel,
-// whose pivots and tile halves are skipped); -1 = all of the nb tiles.
+// whose pivots and tile halves are skipped); -1 = all of the nb tiles.  sym: the
+// matrix is symmetric (a hint: half of the tiles may be left out).
+// dst (side ld_dst, a multiple of 4): the s x s matrix src, the sentinel around it.
+template <typename T>
+cudaError_t launch_pad_copy(T *dst, int64_t ld_dst, const T *src, int64_t ld_src, int s, cudaStream_t stream,
+                            int64_t *launches);
+
+// launch_floyd_matrix in pivot blocks of 64; sym: the matrix is symmetric.
+template <typename T>
+cudaError_t launch_floyd64(T *mat, int64_t ld, int s, bool sym, cudaStream_t stream, int64_t *launches);
 template <typename T>
 cudaError_t launch_floyd_matrix(T *mat, int64_t ld, int nb, int *status, cudaStream_t stream,
-                                int64_t *launches, int s = -1);
+                                int64_t *launches, int s = -1, bool sym = false);
 
 // Boundary rows of the listed parts: F[i][j] -> D[row_base+i][st2ed[start+j]].
 template <typename T>
