@@ -1247,13 +1247,14 @@ constexpr int kThinK = kThinBoundary;
 constexpr int kThinThreads = 256;
 constexpr int kThinCols = 8 * kThinThreads;
 constexpr int kThinHalf = kThinCols / 2;
-constexpr int kThinOwnMax = 64;
+constexpr int kThinRows = 32;   // a CTA's rows are a multiple of this
+constexpr int kThinOwn = 8192;  // own-part values staged at a time (rows x own columns of the strip)
 
 template <typename T>
 struct ThinShared {
   __align__(16) T As[kMinplusBM][kThinK];
-  T Own[kMinplusBM][kThinOwnMax];
-  int32_t own_col[kThinOwnMax];
+  T Own[kThinOwn];
+  uint16_t own_col[kThinCols];  // (parts of more than 65,535 vertices have no Floyd matrix)
   int nown;
 };
 
@@ -1278,26 +1279,28 @@ __device__ __forceinline__ void thin_rows(ThinShared<T> &sh, const PartDesc &pd,
       sv[k][4 * g + 0] = v.x; sv[k][4 * g + 1] = v.y; sv[k][4 * g + 2] = v.z; sv[k][4 * g + 3] = v.w;
     }
   const T *Fp = F + pd.f_off;
-  // Own-part columns (the decode): staged slot per column, or -1.  Own
-  // columns are scattered over the strip, so the replacement is done with
-  // selects (no divergent branch per row) whenever any lane of the warp has
-  // one; a column whose value was not staged (more own columns than
-  // kThinOwnMax in the strip) takes the rare global-load path.
+  // Own-part columns (the decode): slot per column, or -1.  Own columns are
+  // scattered over the strip, so the replacement is done with selects (no
+  // divergent branch per row) whenever any lane of the warp has one.  A block
+  // is as many rows as have room for all of the strip's own values (128 up to
+  // 64 own columns; a graph of few parts has hundreds, and loading those that
+  // did not fit row by row took 0.09 of road20k's 0.62 ms and most of the
+  // merge of graphs of five parts).
   const bool warp_own = __any_sync(0xffffffffu, any_own);
-  const bool cta_unstaged = sh.nown > kThinOwnMax;  // same in every thread
-  for (int m0 = mb; m0 < me; m0 += kMinplusBM) {
-    const int rows = min(kMinplusBM, me - m0);
+  const int nown = sh.nown;  // same in every thread
+  const int block = nown <= kThinOwn / kMinplusBM ? kMinplusBM : kThinOwn / nown;
+  for (int m0 = mb; m0 < me; m0 += block) {
+    const int rows = min(block, me - m0);
     const T *Fr = Fp + (int64_t)(pd.b + m0) * pd.ldf;
     // stage this block's A values and own-part values
     __syncthreads();
-    for (int t = threadIdx.x; t < kMinplusBM * kThinK; t += blockDim.x) {
+    for (int t = threadIdx.x; t < rows * kThinK; t += blockDim.x) {
       const int r = t / kThinK, k = t % kThinK;
-      sh.As[r][k] = (r < rows && k < B) ? __ldg(Fr + (int64_t)r * pd.ldf + k) : inf;
+      sh.As[r][k] = k < B ? __ldg(Fr + (int64_t)r * pd.ldf + k) : inf;
     }
-    const int nown = min(sh.nown, kThinOwnMax);
     for (int t = threadIdx.x; t < rows * nown; t += blockDim.x) {
-      const int r = t / nown, o = t % nown;
-      sh.Own[r][o] = __ldg(Fr + (int64_t)r * pd.ldf + sh.own_col[o]);
+      const int r = t / nown, o = t - r * nown;
+      sh.Own[t] = __ldg(Fr + (int64_t)r * pd.ldf + sh.own_col[o]);
     }
     __syncthreads();
     T *Cm = D + (pd.row_base + pd.b + m0) * ldD + c0;
@@ -1321,17 +1324,9 @@ __device__ __forceinline__ void thin_rows(ThinShared<T> &sh, const PartDesc &pd,
       if (warp_own) {
 #pragma unroll
         for (int q = 0; q < 4 * G; q++) {
-          const int o = own[4 * g0 + q];  // -1, or (part-local column << 7) | (slot + 1)
-          const int sl = o >= 0 ? (o & 127) - 1 : -1;
-          const T st = sh.Own[r][sl >= 0 ? sl : 0];
+          const int sl = own[4 * g0 + q];
+          const T st = sh.Own[r * nown + max(sl, 0)];
           acc[q] = sl >= 0 ? st : acc[q];
-        }
-        if (cta_unstaged) {
-#pragma unroll
-          for (int q = 0; q < 4 * G; q++) {
-            const int o = own[4 * g0 + q];
-            if (o >= 0 && (o & 127) == 0) acc[q] = Fr[(int64_t)r * pd.ldf + (o >> 7)];
-          }
         }
       }
 #pragma unroll
@@ -1363,7 +1358,7 @@ __device__ __forceinline__ void thin_dispatch(ThinShared<T> &sh, const PartDesc 
 
 // grid (ceil(ldD / kThinCols), number of thin parts, row chunks);
 // blockIdx.y indexes thin_parts (batch indices), blockIdx.z the chunk of
-// row_chunk inner rows (a multiple of kMinplusBM) the CTA walks, so that a
+// row_chunk inner rows (a multiple of kThinRows) the CTA walks, so that a
 // batch of few parts still spreads over every SM.
 template <typename T>
 __global__ void __launch_bounds__(kThinThreads, 2)
@@ -1390,15 +1385,12 @@ __global__ void __launch_bounds__(kThinThreads, 2)
     if (live[q >> 2] && c < n && __ldg(graph_id + c) == pd.part) {
       const int j = __ldg(ed2st + c) - pd.start;
       const int sl = atomicAdd(&sh.nown, 1);
-      int staged = 0;
-      if (sl < kThinOwnMax) {
-        sh.own_col[sl] = j;
-        staged = sl + 1;
-      }
-      own[q] = (j << 7) | staged;
+      sh.own_col[sl] = (uint16_t)j;
+      own[q] = sl;
       any_own = true;
     }
   }
+  __syncthreads();  // the strip's own columns are counted
   switch (pd.b) {
 #define FAPB_THIN_CASE(NB) \
   case NB: thin_dispatch<T, NB>(sh, pd, mb, me, c0, F, D, ldD, own, any_own, live); break;
@@ -1484,13 +1476,14 @@ cudaError_t launch_minplus_thin(const PartDesc *parts, const int32_t *thin_parts
                                 int n, const T *F, T *D, int64_t ldD, const int32_t *graph_id,
                                 const int32_t *ed2st, cudaStream_t stream, int64_t *launches) {
   if (nthin <= 0 || max_m <= 0) return cudaSuccess;
-  // Enough CTAs for about four per SM: split the parts' inner rows into
-  // chunks of whole kMinplusBM blocks when the column strips alone are few.
+  // Enough CTAs for about 16 per SM (two run at a time, so the last wave is a
+  // small share; road20k 0.62 -> 0.53 ms against four per SM): split the parts' inner rows into
+  // chunks of whole kThinRows blocks when the column strips alone are few.
   const int64_t col_ctas = ceil_div(ldD, kThinCols) * (int64_t)nthin;
-  const int64_t blocks = ceil_div(max_m, kMinplusBM);
-  const int64_t want = 4 * (int64_t)device_sm_count();
+  const int64_t blocks = ceil_div(max_m, kThinRows);
+  const int64_t want = 16 * (int64_t)device_sm_count();
   const int64_t zc = std::min<int64_t>(blocks, std::max<int64_t>(1, ceil_div(want, col_ctas)));
-  const int row_chunk = (int)(ceil_div(blocks, zc) * kMinplusBM);
+  const int row_chunk = (int)(ceil_div(blocks, zc) * kThinRows);
   const unsigned gz = (unsigned)ceil_div(max_m, row_chunk);
   dim3 grid((unsigned)ceil_div(ldD, kThinCols), (unsigned)nthin, gz);
   minplus_thin_kernel<T><<<grid, kThinThreads, 0, stream>>>(parts, thin_parts, n, F, D, ldD,

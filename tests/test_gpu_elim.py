@@ -50,6 +50,7 @@ def _grid_forest():
 
 CASES = {  # name: (graph, parts)
     "road": (lambda: G.road_graph(3001, seed=20), 5),
+    "two_parts": (lambda: G.road_graph(2600, seed=32), 2),   # a strip's own columns by the hundred
     "tiny_parts": (lambda: G.road_graph(97, seed=24), 16),
     "forest": (_forest, 4),
     "heavy": (_heavy, 3),
