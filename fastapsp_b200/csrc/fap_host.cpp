@@ -11,6 +11,8 @@
 //   fapGraph                     fap/fap.cpp:27-277
 #include "fap/fap.h"
 
+#include <future>
+#include <system_error>
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -521,12 +523,20 @@ int32_t fapGraph::solve(bool path_needed) {
   ensure_device();
   set_paths(path_needed);
   const int64_t n = num_vertexs;
-  dist.assign((size_t)(n * n), 0.0f);
-  path.assign((size_t)(n * n), -1);
+  dist.resize((size_t)(n * n));  // every entry is copied below
   path_ready_ = false;
+  // the -1 of `path` are written while the device solves and copies (the
+  // future's destructor waits for them, whatever happens below)
+  std::future<void> blank;
+  try {
+    blank = std::async(std::launch::async, [this, n] { path.assign((size_t)(n * n), -1); });
+  } catch (const std::system_error &) {  // no thread to be had
+    path.assign((size_t)(n * n), -1);
+  }
   const int rc = solve_all(static_cast<int>(mode_));
   if (rc == FAP_OK) {
     check(fap_graph_check(dg_), "fap_graph_check");
+    if (path_needed && blank.valid()) blank.get();
     for (int32_t p = 1; p <= K; p++) {
       copy_block(p, dist.data() + (size_t)C_BlockVer_offset[p] * n);
       if (path_needed) copy_path_block(p, path.data() + (size_t)C_BlockVer_offset[p] * n);
@@ -534,6 +544,7 @@ int32_t fapGraph::solve(bool path_needed) {
   } else if (rc == FAP_ERR_NOMEM) {
     // Fewer than n rows fit on the device: solve and copy group by group.
     const int64_t rows = reserve_group_rows(max_subgraph_vertexs);
+    if (path_needed && blank.valid()) blank.get();
     for (int32_t p = 1; p <= K;) {
       const int32_t next = run_group(p, rows);
       for (; p < next; p++) {
@@ -544,6 +555,7 @@ int32_t fapGraph::solve(bool path_needed) {
   } else {
     check(rc, "fap_solve");
   }
+  if (blank.valid()) blank.get();
   path_ready_ = path_needed;
   return 0;
 }
@@ -595,12 +607,16 @@ int32_t fapGraph::solveSubGraph(int32_t id, bool path_needed) {
 // ---------------------------------------------------------------------------
 std::vector<int32_t> fapGraph::getMapping() { return st2ed; }
 
-std::vector<float> fapGraph::getAllDistance() {
+std::vector<float> fapGraph::getAllDistance() { return allDistance(); }
+
+const std::vector<float> &fapGraph::allDistance() const {
   if (is_split) raise(FAP_ERR_STATE, "getAllDistance on a split graph");
   return dist;
 }
 
-std::vector<int32_t> fapGraph::getAllPath() {
+std::vector<int32_t> fapGraph::getAllPath() { return allPath(); }
+
+const std::vector<int32_t> &fapGraph::allPath() const {
   if (is_split) raise(FAP_ERR_STATE, "getAllPath on a split graph");
   return path;
 }
@@ -613,12 +629,16 @@ std::vector<int32_t> fapGraph::getSubGraphIndex(int32_t id) {
 
 int32_t fapGraph::getCurrentSubGraphId() { return current_subgraph_id; }
 
-std::vector<float> fapGraph::getSubGraphDistance(int32_t id) {
+std::vector<float> fapGraph::getSubGraphDistance(int32_t id) { return subGraphDistance(id); }
+
+const std::vector<float> &fapGraph::subGraphDistance(int32_t id) const {
   if (id != current_subgraph_id) raise(FAP_ERR_STATE, "part is not the current one");
   return subgraph_dist;
 }
 
-std::vector<int32_t> fapGraph::getSubGraphPath(int32_t id) {
+std::vector<int32_t> fapGraph::getSubGraphPath(int32_t id) { return subGraphPath(id); }
+
+const std::vector<int32_t> &fapGraph::subGraphPath(int32_t id) const {
   if (id != current_subgraph_id) raise(FAP_ERR_STATE, "part is not the current one");
   return subgraph_path;
 }
@@ -733,6 +753,28 @@ int h_invalid(const char *msg) {
 }  // namespace
 
 // Every pointer argument of a wrapper is checked: NULL is FAP_ERR_INVALID.
+namespace {
+// memcpy into a caller's matrix, which is usually fresh memory: the page faults
+// dominate (67 MB: 14 ms on one thread, 4 on four), so large copies are split.
+void copy_out(void *dst, const void *src, size_t bytes) {
+  constexpr size_t kPiece = size_t(4) << 20;
+  constexpr size_t kThreads = 4;
+  std::future<void> done[kThreads];
+  const size_t step = bytes < 2 * kPiece ? bytes : (bytes / kThreads + 4095) / 4096 * 4096;
+  size_t at = 0;
+  for (size_t t = 0; at + step < bytes && t + 1 < kThreads; t++, at += step) {
+    char *d = static_cast<char *>(dst) + at;
+    const char *s = static_cast<const char *>(src) + at;
+    try {
+      done[t] = std::async(std::launch::async, [d, s, step] { std::memcpy(d, s, step); });
+    } catch (const std::system_error &) {  // no thread to be had
+      std::memcpy(d, s, step);
+    }
+  }
+  std::memcpy(static_cast<char *>(dst) + at, static_cast<const char *>(src) + at, bytes - at);
+}
+}  // namespace
+
 #define FAPH_NEED(cond) \
   if (!(cond)) return h_invalid("NULL argument")
 
@@ -899,16 +941,16 @@ int fap_host_current_subgraph(fap::fapGraph *g) {
 int fap_host_subgraph_distance(fap::fapGraph *g, int id, float *out) {
   FAPH_NEED(g && out);
   FAPH_BODY({
-    auto v = g->getSubGraphDistance(id);
-    std::memcpy(out, v.data(), v.size() * sizeof(float));
+    const auto &v = g->subGraphDistance(id);
+    copy_out(out, v.data(), v.size() * sizeof(float));
   })
 }
 
 int fap_host_all_distance(fap::fapGraph *g, float *out) {
   FAPH_NEED(g && out);
   FAPH_BODY({
-    auto v = g->getAllDistance();
-    std::memcpy(out, v.data(), v.size() * sizeof(float));
+    const auto &v = g->allDistance();
+    copy_out(out, v.data(), v.size() * sizeof(float));
   })
 }
 
@@ -928,16 +970,16 @@ int fap_host_distance_p2p(fap::fapGraph *g, int from, int to, float *out) {
 int fap_host_subgraph_path(fap::fapGraph *g, int id, int32_t *out) {
   FAPH_NEED(g && out);
   FAPH_BODY({
-    auto v = g->getSubGraphPath(id);
-    std::memcpy(out, v.data(), v.size() * sizeof(int32_t));
+    const auto &v = g->subGraphPath(id);
+    copy_out(out, v.data(), v.size() * sizeof(int32_t));
   })
 }
 
 int fap_host_all_path(fap::fapGraph *g, int32_t *out) {
   FAPH_NEED(g && out);
   FAPH_BODY({
-    auto v = g->getAllPath();
-    std::memcpy(out, v.data(), v.size() * sizeof(int32_t));
+    const auto &v = g->allPath();
+    copy_out(out, v.data(), v.size() * sizeof(int32_t));
   })
 }
 

@@ -179,6 +179,12 @@ class __attribute__((visibility("default"))) fapGraph {
   int32_t getK() const { return K; }
   fap_dgraph *deviceGraph() { return dg_; }
 
+  // The same matrices without a copy (valid until the next solve).
+  const std::vector<float> &allDistance() const;
+  const std::vector<int32_t> &allPath() const;
+  const std::vector<float> &subGraphDistance(int32_t sub_graph_id) const;
+  const std::vector<int32_t> &subGraphPath(int32_t sub_graph_id) const;
+
   // Sampled self-check (fap/utils/checkResult.h:38-82): 20 random rows x 10
   // random columns of `dist` (rows = source[]) against shortest-path rows
   // recomputed by the GPU SSSP stage; |diff| <= 1e-5 or both unreachable.
