@@ -288,16 +288,18 @@ struct ElimBuf {
     buf.release();
     plan = ElimPlan{};
   }
-  int upload() {
+  int upload(bool directed) {
     const struct { const void *p; size_t bytes; } src[] = {
         {plan.parts.data(), plan.parts.size() * sizeof(ElimPart)},
         {plan.loc.data(), plan.loc.size() * 4},   {plan.inv.data(), plan.inv.size() * 4},
         {plan.eptr.data(), plan.eptr.size() * 4}, {plan.ecol.data(), plan.ecol.size() * 4},
         {plan.eend.data(), plan.eend.size() * 4}, {plan.w0.data(), plan.w0.size() * 4},
-        {plan.lev.data(), plan.lev.size() * 4},   {plan.units.data(), plan.units.size() * sizeof(ElimUnit)},
+        {plan.w0b.data(), directed ? plan.w0b.size() * 4 : 0}, {plan.lev.data(), plan.lev.size() * 4},
+        {plan.units.data(), plan.units.size() * sizeof(ElimUnit)},
         {plan.glev.data(), plan.glev.size() * 4}, {plan.rows8.data(), plan.rows8.size() * 4},
-        {plan.list.data(), plan.list.size() * 2}, {plan.sloc.data(), plan.sloc.size() * 4},
-        {plan.chunks.data(), plan.chunks.size() * sizeof(ElimChunk)}, {nullptr, plan.ecol.size() * sizeof(int2)}};
+        {plan.sloc.data(), plan.sloc.size() * 4}, {plan.list.data(), plan.list.size() * 2},
+        {plan.chunks.data(), plan.chunks.size() * sizeof(ElimChunk)},
+        {nullptr, plan.ecol.size() * sizeof(int2)}, {nullptr, directed ? plan.ecol.size() * 4 : 0}};
     constexpr int N = sizeof(src) / sizeof(src[0]);
     size_t off[N], bytes = 0;
     for (int i = 0; i < N; i++) {
@@ -305,17 +307,37 @@ struct ElimBuf {
       bytes += (src[i].bytes + 255) / 256 * 256;
     }
     FAP_TRY(buf.ensure(std::max<size_t>(bytes, 256)));
-    std::vector<char> host(off[N - 1]);
-    for (int i = 0; i + 1 < N; i++)
+    std::vector<char> host(off[N - 2]);
+    for (int i = 0; i + 2 < N; i++)
       if (src[i].bytes > 0) std::memcpy(host.data() + off[i], src[i].p, src[i].bytes);
     FAP_CK(cudaMemcpy(buf.p, host.data(), host.size(), cudaMemcpyHostToDevice));
     char *d = buf.as<char>();
     auto at = [&](int i) { return reinterpret_cast<const int32_t *>(d + off[i]); };
-    dev = ElimDev{reinterpret_cast<const ElimPart *>(d), at(1), at(2), at(3), at(4), at(5), at(6), at(7),
-                  reinterpret_cast<const ElimUnit *>(d + off[8]), at(9), at(10), at(12),
-                  reinterpret_cast<const uint16_t *>(d + off[11]),
-                  reinterpret_cast<const ElimChunk *>(d + off[13]), reinterpret_cast<int2 *>(d + off[N - 1]), (int32_t)plan.parts.size(), plan.max_s, plan.max_b,
-                  plan.max_nent, plan.max_nlev, plan.max_chunk16, plan.max_chunks};
+    dev = ElimDev{};
+    dev.parts = reinterpret_cast<const ElimPart *>(d);
+    dev.loc = at(1);
+    dev.inv = at(2);
+    dev.eptr = at(3);
+    dev.ecol = at(4);
+    dev.eend = at(5);
+    dev.w0 = at(6);
+    dev.w0b = directed ? at(7) : nullptr;
+    dev.lev = at(8);
+    dev.units = reinterpret_cast<const ElimUnit *>(d + off[9]);
+    dev.glev = at(10);
+    dev.rows8 = at(11);
+    dev.sloc = at(12);
+    dev.list = reinterpret_cast<const uint16_t *>(d + off[13]);
+    dev.chunks = reinterpret_cast<const ElimChunk *>(d + off[14]);
+    dev.ent = reinterpret_cast<int2 *>(d + off[15]);
+    dev.entb = directed ? reinterpret_cast<int32_t *>(d + off[16]) : nullptr;
+    dev.nparts = (int32_t)plan.parts.size();
+    dev.max_s = plan.max_s;
+    dev.max_b = plan.max_b;
+    dev.max_nent = plan.max_nent;
+    dev.max_nlev = plan.max_nlev;
+    dev.max_chunk16 = plan.max_chunk16;
+    dev.max_chunks = plan.max_chunks;
     return FAP_OK;
   }
 };
@@ -433,6 +455,7 @@ struct fap_dgraph {
   // kElimGraphMax vertices; larger ones are closed by Floyd), barcs the arcs
   // between boundary vertices as (boundary index, boundary index, weight).
   bool eliminate = true;   // parameter "eliminate"
+  bool el_sym = false;     // the plans of the boundary-graph form exist
   bool last_elim = false;  // the prepared batch uses it
   ElimBuf el, el2;
   std::vector<int32_t> barcs;
@@ -440,7 +463,7 @@ struct fap_dgraph {
   // Parts of the prepared batch whose inner rows the group merge makes
   // (plan part, batch index), and its coefficients (ElimMerge).
   std::vector<int2> merge;
-  bool last_merge = false;
+  bool last_merge = false, last_given = false;
   int32_t merge_units = 0, merge_slots = 0;
   DevBuf d_merge, d_coef32, d_coef16, d_far;
   std::vector<int32_t> boff;
@@ -699,15 +722,20 @@ namespace {
 constexpr int64_t kElimGraphMax = 2048;
 constexpr int64_t kElimGraphEntries = 24576;
 
-// The elimination plans of the parts and of the boundary graph, for
-// undirected int32 graphs (every arc has its reverse with the same weight)
-// without duplicate arcs inside a part.  Host work of some milliseconds on
-// up to 16 threads.
+// The elimination plans: of the parts, for every graph with boundary vertices
+// whose parts eliminate with short lists, and on undirected int32 graphs
+// (el_sym: every arc has its reverse with the same weight, no duplicate arcs
+// inside a part) of the boundary graph.  Host work of some milliseconds on up
+// to 16 threads.
 int build_elim(fap_dgraph *G) {
   G->el.release();
   G->el2.release();
   G->barcs.clear();
-  if (G->dtype != FAP_DTYPE_I32 || !G->sym_local || G->total_b <= 0) return FAP_OK;
+  G->el_sym = false;
+  if (G->total_b <= 0) return FAP_OK;
+  const bool i32 = G->dtype == FAP_DTYPE_I32;
+  const int32_t inf = i32 ? kInfI32 : 0x4cbebc20;  // (bits of 1e8f)
+  const int threads = std::min(16, (int)std::thread::hardware_concurrency());
   const int32_t K = (int32_t)G->vnum.size() - 1;
   auto bidx = [&](int32_t v) { return G->boff[G->gid[v]] + (G->ed2st[v] - G->voff[G->gid[v]]); };
   auto weight = [&](int32_t e) {
@@ -733,6 +761,12 @@ int build_elim(fap_dgraph *G) {
       g->ptr.push_back((int32_t)g->adj.size());
     }
   };
+  elim_build(K, part_graph, threads, inf, i32, &G->el.plan);
+  if (!G->el.plan.ok) return FAP_OK;
+  // (float32 parts keep min-plus over the boundary, which distance rows from
+  // the resident cache match bit for bit; their symmetry is sym_local's)
+  FAP_TRY(G->el.upload(!G->sym_local));
+  if (!i32 || !G->sym_local) return FAP_OK;
   std::vector<std::array<int32_t, 3>> cross;
   for (int32_t p = 1; p <= K; p++)
     for (int32_t i = 0; i < G->bnum[p]; i++) {
@@ -756,9 +790,7 @@ int build_elim(fap_dgraph *G) {
   }
   for (const auto &a : cross) G->barcs.insert(G->barcs.end(), a.begin(), a.end());
   if (G->barcs.size() > (size_t)INT32_MAX) return FAP_OK;
-  elim_build(K, part_graph, std::min(16, (int)std::thread::hardware_concurrency()), &G->el.plan);
-  if (!G->el.plan.ok) return FAP_OK;
-  FAP_TRY(G->el.upload());
+  G->el_sym = true;
   FAP_TRY(G->d_barcs.ensure(std::max<size_t>(G->barcs.size(), 4) * 4));
   if (!G->barcs.empty())
     FAP_CK(cudaMemcpy(G->d_barcs.p, G->barcs.data(), G->barcs.size() * 4, cudaMemcpyHostToDevice));
@@ -775,11 +807,11 @@ int build_elim(fap_dgraph *G) {
         g->ptr.push_back((int32_t)g->adj.size());
       }
   };
-  elim_build(1, boundary_graph, 1, &G->el2.plan);
+  elim_build(1, boundary_graph, 1, inf, false, &G->el2.plan);
   if (G->el2.plan.nent > kElimGraphEntries) G->el2.plan = ElimPlan{};
   if (!G->el2.plan.ok) return FAP_OK;
   elim_offsets(round_up(G->total_b, kFloydTile), &G->el2.plan);
-  return G->el2.upload();
+  return G->el2.upload(false);
 }
 
 // Whether solves close the boundary graph and the parts by elimination:
@@ -791,12 +823,16 @@ int build_elim(fap_dgraph *G) {
 // graph: 0.17 ms instead of 4.6.
 constexpr int64_t kElimBatchElems = int64_t(1) << 20;
 bool elim_ok(const fap_dgraph *G, int64_t sources) {
-  if (!G->eliminate || !G->el.plan.ok || G->dtype != FAP_DTYPE_I32 || G->stage1 == 1 || G->bgraph_form != 0 ||
+  if (!G->eliminate || !G->el_sym || G->stage1 == 1 || G->bgraph_form != 0 ||
       !G->floyd_queue || !G->floyd_sym || G->floyd_per_cta || G->total_b > kBgraphFloydMax)
     return false;
   const int64_t ldB = round_up(G->total_b, kFloydTile);
   return sources < 0 || (G->el2.plan.ok && ldB * ldB <= std::max<int64_t>(sources * G->n, kElimBatchElems));
 }
+
+// Whether the SSSP form closes the parts by elimination from its boundary rows
+// (any dtype, directed or not) instead of Floyd-Warshall.
+bool elim_given_ok(const fap_dgraph *G) { return G->eliminate && G->el.plan.ok && !G->floyd_per_cta; }
 }  // namespace
 
 extern "C" int fap_graph_destroy(fap_dgraph *G) try {
@@ -1278,10 +1314,12 @@ int expand_bgraph(fap_dgraph *G, const PartDesc *dp, int np, int max_s, const T 
 
 // Device state of the elimination form for the listed parts (row_base and
 // f_off final): the plans, dB, the parts to close and, for a batch of some of
-// the parts, the boundary rows to write.
-int prepare_elim(fap_dgraph *G, const std::vector<PartDesc> &parts) {
-  G->ldB = round_up(std::max<int64_t>(G->total_b, 1), kFloydTile);
-  FAP_TRY(G->d_dB.ensure((size_t)G->ldB * G->ldB * 4));
+// the parts, the boundary rows to write.  given: for run_elim_given only.
+int prepare_elim(fap_dgraph *G, const std::vector<PartDesc> &parts, bool given = false) {
+  if (!given) {
+    G->ldB = round_up(std::max<int64_t>(G->total_b, 1), kFloydTile);
+    FAP_TRY(G->d_dB.ensure((size_t)G->ldB * G->ldB * 4));
+  }
   std::vector<int32_t> list;
   std::vector<int64_t> off{0}, rows;  // (the first offset is the boundary graph's own)
   for (const PartDesc &d : parts) {
@@ -1294,10 +1332,27 @@ int prepare_elim(fap_dgraph *G, const std::vector<PartDesc> &parts) {
   }
   FAP_TRY(G->d_elist.ensure(list.size() * 4));
   FAP_TRY(G->d_eoff.ensure(off.size() * 8));
+  if (given) {
+    FAP_CK(cudaMemcpy(G->d_elist.p, list.data(), list.size() * 4, cudaMemcpyHostToDevice));
+    FAP_CK(cudaMemcpy(G->d_eoff.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice));
+    return FAP_OK;
+  }
   FAP_TRY(G->d_brows.ensure(std::max<size_t>(rows.size(), 2) * 8));
   FAP_CK(cudaMemcpy(G->d_elist.p, list.data(), list.size() * 4, cudaMemcpyHostToDevice));
   FAP_CK(cudaMemcpy(G->d_eoff.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice));
   if (!rows.empty()) FAP_CK(cudaMemcpy(G->d_brows.p, rows.data(), rows.size() * 8, cudaMemcpyHostToDevice));
+  return FAP_OK;
+}
+
+// F = the listed parts' exact closures from their boundary rows in D.
+template <typename T>
+int run_elim_given(fap_dgraph *G, const PartDesc *dp, int count, int max_s, T *F, int64_t ldf, const T *D, int64_t *L) {
+  cudaStream_t st = G->ctx->stream;
+  const int32_t *list = G->d_elist.as<const int32_t>();
+  FAP_CK(launch_elim_up<T>(G->el.dev, list, count, nullptr, nullptr, 0, st, L));
+  FAP_CK(launch_elim_close<T>(G->el.dev, list, G->d_eoff.as<const int64_t>() + 1, count, max_s,
+                              ElimBoundary<T>{nullptr, 0, dp, D, G->ldD, G->d_st2ed.as<const int32_t>()}, F, ldf, st,
+                              L));
   return FAP_OK;
 }
 
@@ -1316,17 +1371,18 @@ int run_elim(fap_dgraph *G, const PartDesc *dp, int count, int max_s, int32_t *F
     for (const PartDesc &d : G->parts) nrows += d.b;
   FAP_CK(launch_elim_seed(dB, G->ldB, nb, G->el2.plan.ok ? nb : (int)G->ldB, G->d_barcs.as<const int32_t>(),
                           (int)(G->barcs.size() / 3), st, L));
-  FAP_CK(launch_elim_up(G->el.dev, nullptr, dB, G->ldB, st, L));
+  FAP_CK(launch_elim_up<int32_t>(G->el.dev, nullptr, 0, nullptr, dB, G->ldB, st, L));
   FAP_CK(record_event(ev1, st));
   if (G->el2.plan.ok) {
-    FAP_CK(launch_elim_up(G->el2.dev, dB, nullptr, 0, st, L));
-    FAP_CK(launch_elim_close(G->el2.dev, nullptr, off, 1, nb, nullptr, 0, dB, G->ldB, st, L));
+    FAP_CK(launch_elim_up<int32_t>(G->el2.dev, nullptr, 0, dB, nullptr, 0, st, L));
+    FAP_CK(launch_elim_close<int32_t>(G->el2.dev, nullptr, off, 1, nb, ElimBoundary<int32_t>{}, dB, G->ldB, st, L));
   } else {
     FAP_CK(launch_floyd_matrix<int32_t>(dB, G->ldB, (int)ceil_div(nb, kFloydTile), status, st, L, nb,
                                         true));
   }
   FAP_CK(record_event(ev2, st));
-  FAP_CK(launch_elim_close(G->el.dev, G->d_elist.as<const int32_t>(), off + 1, count, max_s, dB, G->ldB, F, ldf, st, L));
+  FAP_CK(launch_elim_close<int32_t>(G->el.dev, G->d_elist.as<const int32_t>(), off + 1, count, max_s,
+                                    ElimBoundary<int32_t>{dB, G->ldB, nullptr, nullptr, 0, nullptr}, F, ldf, st, L));
   FAP_CK(record_event(ev3, st));
   if (all) {
     FAP_TRY(expand_bgraph<int32_t>(G, dp, count, max_s, F, Dout, ldf, status, L));
@@ -1361,9 +1417,9 @@ int run_merge(fap_dgraph *G, const PartDesc *dp, const int32_t *F, int64_t *L) {
 
 // Builds (or reuses) the batch descriptors for the requested parts.
 int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, bool bmethod, bool elim,
-                  bool merge) {
+                  bool given, bool merge) {
   const bool same = (ids == G->last_ids) && (cached == G->last_cached) && (bmethod == G->last_bmethod) &&
-                    (elim == G->last_elim) && (merge == G->last_merge);
+                    (elim == G->last_elim) && (given == G->last_given) && (merge == G->last_merge);
   if (same) return FAP_OK;
   // The descriptors change from here on: until they are complete no batch
   // counts as prepared, so a failure below forces a full rebuild next time.
@@ -1522,7 +1578,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
     }
   }
   std::vector<QItem> qitems;
-  if (!cached && !elim) {
+  if (!cached && !elim && !given) {
     int32_t mnb = 0;
     // (the local closures of the boundary-graph form are symmetric when the
     // parts are; the SSSP form's matrices hold boundary rows and are not)
@@ -1537,7 +1593,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
   FAP_CK(cudaStreamSynchronize(st));
   if (!qitems.empty())
     FAP_CK(cudaMemcpy(G->q.items.p, qitems.data(), qitems.size() * sizeof(QItem), cudaMemcpyHostToDevice));
-  if (elim) FAP_TRY(prepare_elim(G, G->parts));
+  if (elim || given) FAP_TRY(prepare_elim(G, G->parts, given));
   if (bmethod && (int32_t)ids.size() == G->K) FAP_TRY(prepare_bgraph(G, G->parts, true));
   FAP_CK(cudaMemcpy(G->d_parts.p, G->parts.data(), G->parts.size() * sizeof(PartDesc), cudaMemcpyHostToDevice));
   if (!G->work.empty())
@@ -1558,6 +1614,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
   G->last_cached = cached;
   G->last_bmethod = bmethod;
   G->last_elim = elim;
+  G->last_given = given;
   G->last_merge = merge;
   G->epoch++;
   return FAP_OK;
@@ -1757,13 +1814,16 @@ int run_solve(fap_dgraph *G, int mode) {
     FAP_CK(record_event(c->ev[0], st));
     FAP_TRY(run_stage1_sssp<T>(G, src, srow, (int)G->src.size(), D, status, max_rounds, &L));
     FAP_CK(record_event(c->ev[1], st));
-    FAP_CK(launch_gather<T>(dp, np, G->max_ldf, ro, col, w, gid, st2ed, ed2st, D, G->ldD, F, st, &L));
+    if (!G->last_given)
+      FAP_CK(launch_gather<T>(dp, np, G->max_ldf, ro, col, w, gid, st2ed, ed2st, D, G->ldD, F, st, &L));
     FAP_CK(record_event(c->ev[2], st));
     // With the work queue, the min-plus tiles run in the same launch as the
     // Floyd (each part's as soon as its closure and boundary rows are done)
     // unless they use the packed form, whose bounds need every boundary row.
     int mp_in_queue = 0;
-    if (G->floyd_per_cta) {
+    if (G->last_given) {
+      FAP_TRY(run_elim_given<T>(G, dp, np, G->max_s, F, G->max_ldf, D, &L));
+    } else if (G->floyd_per_cta) {
       FAP_CK(launch_floyd_parts<T>(dp, np, F, G->max_ldf, D, G->ldD, st2ed, status, st, &L));
     } else if (G->floyd_queue) {
       mp_in_queue = pack16_of(G) == nullptr ? (int)G->work.size() : 0;
@@ -1864,8 +1924,9 @@ extern "C" int fap_solve(fap_dgraph *G, const int32_t *parts, int32_t count, int
     for (const int32_t p : ids) sources += G->bnum[p];
   const bool elim = !cached && mode == FAP_MODE_BATCHED && elim_ok(G, sources);
   const bool bmethod = elim || (!cached && mode == FAP_MODE_BATCHED && all_parts && bmethod_ok(G));
-  const bool merge = mode == FAP_MODE_BATCHED && G->eliminate && G->el.plan.ok;
-  FAP_TRY(prepare_batch(G, ids, cached, bmethod, elim, merge));
+  const bool given = !cached && !bmethod && mode == FAP_MODE_BATCHED && elim_given_ok(G);
+  const bool merge = mode == FAP_MODE_BATCHED && G->eliminate && G->el.plan.ok && G->dtype == FAP_DTYPE_I32;
+  FAP_TRY(prepare_batch(G, ids, cached, bmethod, elim, given, merge));
   int rc = FAP_OK;
   cudaStream_t st = G->ctx->stream;
   // (the tiled SSSP form tests convergence on the host: not capturable)
@@ -2793,7 +2854,8 @@ int cache_build_impl(fap_dgraph *G) {
   if (!bm && !use_msbf(G))  // (the tiled form sizes its own tiles)
     FAP_TRY(G->sssp_scratch.ensure(
         (size_t)std::max(sssp_scratch_rows(G->n, (int)src.size()), 1) * (size_t)G->n * 4));
-  if (!elim) {
+  const bool given = !bm && elim_given_ok(G);
+  if (!elim && !given) {
     int32_t mnb = 0;
     G->cq.sym = bm && G->sym_local && G->floyd_sym;
     const std::vector<QItem> qitems = floyd_queue_items(G->cparts, G->cq.sym, &G->cq.nfloyd, &mnb);
@@ -2861,11 +2923,15 @@ int cache_build_impl(fap_dgraph *G) {
   FAP_TRY(run_stage1_sssp<T>(G, G->d_src.as<const int32_t>(), G->d_srcrows.as<const int64_t>(),
                              (int)src.size(), Bd, status, rounds, &L));
   FAP_CK(cudaEventRecord(G->cev[1], st));
-  FAP_CK(launch_gather<T>(dp, K, cs.ldf, G->ro.as<const int32_t>(), G->col.as<const int32_t>(),
-                          G->w.as<const T>(), gid, st2ed, ed2st, Bd, G->ldD, F, st, &L));
+  if (!given)
+    FAP_CK(launch_gather<T>(dp, K, cs.ldf, G->ro.as<const int32_t>(), G->col.as<const int32_t>(),
+                            G->w.as<const T>(), gid, st2ed, ed2st, Bd, G->ldD, F, st, &L));
   FAP_CK(cudaEventRecord(G->cev[2], st));
   G->cache_bmethod = false;
-  if (G->floyd_per_cta) {
+  if (given) {
+    FAP_TRY(prepare_elim(G, G->cparts, true));
+    FAP_TRY(run_elim_given<T>(G, dp, K, cs.max_s, F, cs.ldf, Bd, &L));
+  } else if (G->floyd_per_cta) {
     FAP_CK(launch_floyd_parts<T>(dp, K, F, cs.ldf, Bd, G->ldD, st2ed, status, st, &L));
   } else if (G->floyd_queue) {
     FAP_CK(run_floyd_queue<T>(G, G->cq, dp, F, cs.ldf, true, nullptr, 0, Bd, 0, status, &L));

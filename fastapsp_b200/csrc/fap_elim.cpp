@@ -9,12 +9,10 @@
 namespace fapb {
 namespace {
 
-constexpr int32_t kInf = 100000000;
-
 struct PartPlan {
   bool ok = false;
   int32_t b = 0, boff = 0;
-  std::vector<int32_t> loc, inv, eptr, ecol, w0, lev;
+  std::vector<int32_t> loc, inv, eptr, ecol, w0, w0b, lev;
   std::vector<ElimUnit> units;
   std::vector<int32_t> glev, rows8;
   std::vector<uint16_t> list;
@@ -30,7 +28,7 @@ struct PartPlan {
 // their levels, and pendant paths and chains are then taken every other
 // vertex instead of end to end (road114k: 17 levels instead of 53 with 1.46
 // entries per vertex instead of 1.36; a 256 x 256 grid 101 instead of 113).
-void eliminate(const ElimGraph &g, PartPlan *out) {
+void eliminate(const ElimGraph &g, int32_t inf, PartPlan *out) {
   const int32_t s = g.s, b = g.b;
   const int W = (s + 63) / 64;
   std::vector<uint64_t> A((size_t)s * W, 0);
@@ -106,23 +104,24 @@ void eliminate(const ElimGraph &g, PartPlan *out) {
   for (int32_t e = 0; e < s; e++)
     out->eptr[e + 1] = out->eptr[e] + (e < b ? 0 : ncnt[out->loc[e]]);
   out->ecol.resize(nnz);
-  out->w0.assign(nnz, kInf);
+  out->w0.assign(nnz, inf);
+  out->w0b.assign(nnz, inf);
   for (int32_t e = b; e < s; e++) {
     const int32_t v = out->loc[e];
     int32_t *c = &out->ecol[out->eptr[e]];
     int32_t k = 0;
     for (int32_t i = 0; i < ncnt[v]; i++) c[k++] = out->inv[nbr[nptr[v] + i]];
     std::sort(c, c + k, std::greater<int32_t>());
-    if (g.w.empty()) continue;
-    for (int32_t a = g.ptr[v]; a < g.ptr[v + 1]; a++) {
-      const int32_t u = out->inv[g.adj[a]];
-      int32_t *p = std::lower_bound(c, c + k, u, std::greater<int32_t>());
-      if (p != c + k && *p == u) {
-        int32_t &x = out->w0[out->eptr[e] + (p - c)];
-        x = std::min(x, g.w[a]);
-      }
-    }
   }
+  if (!g.w.empty())
+    for (int32_t i = 0; i < s; i++)
+      for (int32_t a = g.ptr[i]; a < g.ptr[i + 1]; a++) {
+        const int32_t x = out->inv[i], y = out->inv[g.adj[a]], v = std::max(x, y), u = std::min(x, y);
+        if (v < b) continue;
+        const int32_t *c = &out->ecol[out->eptr[v]], *end = &out->ecol[0] + out->eptr[v + 1];
+        const auto at = std::lower_bound(c, end, u, std::greater<int32_t>()) - &out->ecol[0];
+        (x > y ? out->w0 : out->w0b)[at] = g.w[a];
+      }
   out->ok = true;
 }
 
@@ -215,7 +214,8 @@ void group_rows(PartPlan *q) {
 
 }  // namespace
 
-void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, int threads, ElimPlan *out) {
+void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, int threads, int32_t inf,
+                bool groups, ElimPlan *out) {
   *out = ElimPlan{};
   const int K = nparts;
   std::vector<PartPlan> pp(K);
@@ -229,9 +229,9 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
         graph(p, &g);
         pp[p].boff = g.boff;
         pp[p].b = g.b;
-        if (g.s <= kElimMaxS) eliminate(g, &pp[p]);
+        if (g.s <= kElimMaxS) eliminate(g, inf, &pp[p]);
         if (!pp[p].ok) dense = true;
-        else if (g.b > 0) group_rows(&pp[p]);
+        else if (groups && g.b > 0) group_rows(&pp[p]);
       }
     } catch (...) {
       failed = true;
@@ -255,7 +255,7 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
   out->loc.reserve(nv);
   out->inv.reserve(nv);
   out->eptr.reserve(nv + K);
-  for (auto *a : {&out->ecol, &out->eend, &out->w0}) a->reserve(ne);
+  for (auto *a : {&out->ecol, &out->eend, &out->w0, &out->w0b}) a->reserve(ne);
   for (int p = 0; p < K; p++) {
     const PartPlan &q = pp[p];
     ElimPart d{};
@@ -299,6 +299,7 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
     out->eptr.insert(out->eptr.end(), q.eptr.begin(), q.eptr.end());
     out->ecol.insert(out->ecol.end(), q.ecol.begin(), q.ecol.end());
     out->w0.insert(out->w0.end(), q.w0.begin(), q.w0.end());
+    out->w0b.insert(out->w0b.end(), q.w0b.begin(), q.w0b.end());
     out->lev.insert(out->lev.end(), q.lev.begin(), q.lev.end());
     for (int32_t e = 0; e < d.s; e++)
       out->eend.insert(out->eend.end(), q.eptr[e + 1] - q.eptr[e], q.eptr[e + 1]);

@@ -54,24 +54,39 @@ __global__ void elim_seed_arcs_kernel(int32_t *M, int64_t ld, const int32_t *__r
 // starts and the levels' entry ranges (a 670-vertex boundary graph: 140 us
 // with only W there, 58 us).  Otherwise the entries sit in L2 and are read
 // past L1.
-template <bool SM>
+// Directed parts (entb): an entry carries both weights, and a pair lowers both.
+template <typename T, bool SM>
 __global__ void __launch_bounds__(kElimUpThreads)
-    elim_up_kernel(ElimDev e, const int32_t *__restrict__ from, int32_t *M, int64_t ldM) {
+    elim_up_kernel(ElimDev e, const int32_t *__restrict__ list, const T *__restrict__ from, T *M, int64_t ldM) {
   extern __shared__ int2 up_smem[];
-  const ElimPart P = e.parts[blockIdx.x];
+  const ElimPart P = e.parts[list ? list[blockIdx.x] : blockIdx.x];
   const int32_t *eptr = e.eptr + P.eptr_off, *lev = e.lev + P.lev_off;
   const int32_t *ecol = e.ecol + P.ent_off, *eend = e.eend + P.ent_off, *w0 = e.w0 + P.ent_off;
+  const T inf = Dist<T>::inf();
+  const bool directed = e.entb != nullptr;
   int2 *gent = e.ent + P.ent_off;
+  int32_t *gentb = directed ? e.entb + P.ent_off : nullptr;
   int2 *ent = SM ? up_smem : gent;
   int32_t *sptr = reinterpret_cast<int32_t *>(up_smem + (SM ? P.nent : 0));  // s + 1 list starts
   int32_t *slev = sptr + P.s + 1;                                            // nlev + 1 entry ranges
+  int32_t *entb = SM ? slev + P.nlev + 1 : gentb;
   const int lane = threadIdx.x % kUpLanes, group = threadIdx.x / kUpLanes, ngroups = blockDim.x / kUpLanes;
+  auto value = [](int32_t bits) -> T {
+    if constexpr (std::is_same<T, float>::value) return __int_as_float(bits);
+    else return bits;
+  };
+  auto bits = [](T x) -> int32_t {
+    if constexpr (std::is_same<T, float>::value) return __float_as_int(x);
+    else return x;
+  };
   if (SM) {
     for (int v = threadIdx.x; v <= P.s; v += blockDim.x) sptr[v] = eptr[v];
     for (int l = threadIdx.x; l <= P.nlev; l += blockDim.x) slev[l] = eptr[lev[l]];
   }
-  for (int i = threadIdx.x; i < P.nent; i += blockDim.x)
-    ent[i] = make_int2(SM ? ecol[i] | (eend[i] - i - 1) << 16 : ecol[i], from ? from[w0[i]] : w0[i]);
+  for (int i = threadIdx.x; i < P.nent; i += blockDim.x) {
+    ent[i] = make_int2(SM ? ecol[i] | (eend[i] - i - 1) << 16 : ecol[i], from ? bits(from[w0[i]]) : w0[i]);
+    if (directed) entb[i] = e.w0b[P.ent_off + i];
+  }
   if (!SM) __threadfence();
   __syncthreads();
   for (int l = P.nlev - 1; l >= 0; l--) {
@@ -80,7 +95,9 @@ __global__ void __launch_bounds__(kElimUpThreads)
       const int2 a = SM ? ent[i] : __ldcg(ent + i);
       const int ui = SM ? a.x & 0xffff : a.x;
       const int end = SM ? i + 1 + (int)((uint32_t)a.x >> 16) : eend[i];
-      if (a.y >= kInf) continue;
+      if (ui < P.b && M == nullptr) continue;  // (pairs of boundary vertices are not wanted)
+      const T out = value(a.y), in = directed ? value(SM ? entb[i] : __ldcg(entb + i)) : out;
+      if (out >= inf && in >= inf) continue;
       int lo = 0, hi = 0;
       if (ui >= P.b) {
         lo = SM ? sptr[ui] : eptr[ui];
@@ -89,11 +106,12 @@ __global__ void __launch_bounds__(kElimUpThreads)
       for (int j = i + 1 + lane; j < end; j += kUpLanes) {
         const int2 c = SM ? ent[j] : __ldcg(ent + j);
         const int uj = SM ? c.x & 0xffff : c.x;
-        const int32_t w = a.y + c.y;
-        if (w >= kInf) continue;
+        const T fwd = in + value(c.y);  // u_i -> v -> u_j
+        const T back = directed ? value(SM ? entb[j] : __ldcg(entb + j)) + out : fwd;
+        if (fwd >= inf && back >= inf) continue;
         if (ui < P.b) {
-          atomicMin(M + (int64_t)(P.boff + ui) * ldM + P.boff + uj, w);
-          atomicMin(M + (int64_t)(P.boff + uj) * ldM + P.boff + ui, w);
+          Dist<T>::atomic_min(M + (int64_t)(P.boff + ui) * ldM + P.boff + uj, fwd);
+          Dist<T>::atomic_min(M + (int64_t)(P.boff + uj) * ldM + P.boff + ui, fwd);
           continue;
         }
         int x = lo, y = hi - 1;  // descending; u_j is in the list
@@ -102,37 +120,50 @@ __global__ void __launch_bounds__(kElimUpThreads)
           if ((SM ? ent[m].x & 0xffff : ecol[m]) > uj) x = m + 1;
           else y = m;
         }
-        atomicMin(&ent[x].y, w);
+        // (non-negative float bits order like int32)
+        if (fwd < inf) atomicMin(&ent[x].y, bits(fwd));
+        if (directed && back < inf) atomicMin(entb + x, bits(back));
       }
     }
     __syncthreads();
   }
   if (SM)
-    for (int i = threadIdx.x; i < P.nent; i += blockDim.x) gent[i] = make_int2(ent[i].x & 0xffff, ent[i].y);
+    for (int i = threadIdx.x; i < P.nent; i += blockDim.x) {
+      gent[i] = make_int2(ent[i].x & 0xffff, ent[i].y);
+      if (directed) gentb[i] = entb[i];
+    }
 }
 
 // What a sweep reads of a part's plan: the entries, the lists' starts and the
 // levels, in shared memory behind the strip (SM) or in global memory.
 struct SweepPlan {
   const int2 *ent;
+  const int32_t *entb;
   const int32_t *eptr, *lev;
 };
 template <int CW, bool SM>
-__device__ __forceinline__ SweepPlan stage_plan(const ElimDev &e, const ElimPart &P, int32_t *st) {
-  SweepPlan p{e.ent + P.ent_off, e.eptr + P.eptr_off, e.lev + P.lev_off};
+__device__ __forceinline__ SweepPlan stage_plan(const ElimDev &e, const ElimPart &P, void *strip) {
+  SweepPlan p{e.ent + P.ent_off, e.entb ? e.entb + P.ent_off : nullptr, e.eptr + P.eptr_off, e.lev + P.lev_off};
   if (!SM) return p;
-  int2 *ent = reinterpret_cast<int2 *>(st + ((P.s * kStripLd<CW> + 1) & ~1));
-  int32_t *eptr = reinterpret_cast<int32_t *>(ent + P.nent), *lev = eptr + P.s + 1;
+  int2 *ent = reinterpret_cast<int2 *>(static_cast<int32_t *>(strip) + ((P.s * kStripLd<CW> + 1) & ~1));
+  int32_t *eptr = reinterpret_cast<int32_t *>(ent + P.nent), *lev = eptr + P.s + 1, *entb = lev + P.nlev + 1;
   for (int i = threadIdx.x; i < P.nent; i += blockDim.x) ent[i] = __ldg(p.ent + i);
   for (int i = threadIdx.x; i <= P.s; i += blockDim.x) eptr[i] = __ldg(p.eptr + i);
   for (int i = threadIdx.x; i <= P.nlev; i += blockDim.x) lev[i] = __ldg(p.lev + i);
-  return SweepPlan{ent, eptr, lev};
+  if (p.entb)
+    for (int i = threadIdx.x; i < P.nent; i += blockDim.x) entb[i] = __ldg(p.entb + i);
+  return SweepPlan{ent, p.entb ? entb : nullptr, eptr, lev};
 }
 template <int CW>
 size_t sweep_bytes(const ElimDev &e, int max_s, bool plan) {
   size_t words = ((size_t)max_s * kStripLd<CW> + 1) & ~size_t(1);
-  if (plan) words += 2 * (size_t)e.max_nent + (size_t)max_s + 1 + e.max_nlev + 1;
+  if (plan) words += (e.entb ? 3 : 2) * (size_t)e.max_nent + (size_t)max_s + 1 + e.max_nlev + 1;
   return words * sizeof(int32_t);
+}
+template <typename T>
+__device__ __forceinline__ T weight_of(int32_t bits) {
+  if constexpr (std::is_same<T, float>::value) return __int_as_float(bits);
+  else return bits;
 }
 
 // Rows of the inner vertices, level by level away from the boundary.  The
@@ -143,8 +174,8 @@ size_t sweep_bytes(const ElimDev &e, int max_s, bool plan) {
 // parts: 1.46 ms without, 0.69 ms with).  Parts with short lists (at most 8
 // entries on average) take whole lists: road114k 0.42 ms without the split,
 // 0.52 with it.
-template <int CW>
-__device__ __forceinline__ void sweep_down(int32_t *st, const ElimPart &P, const SweepPlan &p) {
+template <typename T, int CW>
+__device__ __forceinline__ void sweep_down(T *st, const ElimPart &P, const SweepPlan &p) {
   static_assert(32 % CW == 0, "a warp holds whole rows");
   const int c = threadIdx.x % CW, first = threadIdx.x / CW, step = blockDim.x / CW;
   const bool split = P.nent > 8 * (P.s - P.b);
@@ -153,25 +184,25 @@ __device__ __forceinline__ void sweep_down(int32_t *st, const ElimPart &P, const
     const int sh = split ? 31 - __clz(max(step / (v1 - v0), 1)) : 0;  // (no level is empty)
     if (sh == 0) {
       for (int v = v0 + first; v < v1; v += step) {
-        int32_t *q = st + v * kStripLd<CW> + c;
-        int32_t acc = *q;
+        T *q = st + v * kStripLd<CW> + c;
+        T acc = *q;
         const int e1 = p.eptr[v + 1];
 #pragma unroll 4
         for (int i = p.eptr[v]; i < e1; i++) {
           const int2 x = p.ent[i];
-          acc = __viaddmin_s32(x.y, st[x.x * kStripLd<CW> + c], acc);
+          acc = Dist<T>::relax(weight_of<T>(x.y), st[x.x * kStripLd<CW> + c], acc);
         }
         *q = acc;
       }
     } else if (const int v = v0 + (first >> sh); v < v1) {
-      int32_t acc = kInf;
+      T acc = Dist<T>::inf();
       const int e1 = p.eptr[v + 1];
 #pragma unroll 2
       for (int i = p.eptr[v] + (first & ((1 << sh) - 1)); i < e1; i += 1 << sh) {
         const int2 x = p.ent[i];
-        acc = __viaddmin_s32(x.y, st[x.x * kStripLd<CW> + c], acc);
+        acc = Dist<T>::relax(weight_of<T>(x.y), st[x.x * kStripLd<CW> + c], acc);
       }
-      if (acc < kInf) atomicMin(st + v * kStripLd<CW> + c, acc);
+      if (acc < Dist<T>::inf()) Dist<T>::atomic_min(st + v * kStripLd<CW> + c, acc);
     }
     __syncthreads();
   }
@@ -188,11 +219,14 @@ __device__ __forceinline__ void sweep_down(int32_t *st, const ElimPart &P, const
 // of the levels (road parts: ~50 of each): the plan sits in shared memory
 // when three CTAs still fit on an SM with it (road114k: 827 us with a level
 // barrier in the forward sweep and the plan in L1, 428 us).
-template <int CW, bool SM>
+// Boundary rows given in D (parts != null) are taken as they are.
+template <typename T, int CW, bool SM>
 __global__ void __launch_bounds__(kElimSweepThreads)
     elim_close_kernel(ElimDev e, const int32_t *__restrict__ list, const int64_t *__restrict__ out_off,
-                      const int32_t *dB, int64_t ldB, int32_t *out, int64_t ld) {
-  extern __shared__ __align__(16) int32_t st[];
+                      ElimBoundary<T> bd, T *out, int64_t ld) {
+  extern __shared__ __align__(16) int32_t close_smem[];
+  T *st = reinterpret_cast<T *>(close_smem);
+  const T inf = Dist<T>::inf();
   const ElimPart P = e.parts[list ? list[blockIdx.y] : blockIdx.y];
   const int x0 = blockIdx.x * CW;
   if (x0 >= P.s) return;
@@ -201,41 +235,46 @@ __global__ void __launch_bounds__(kElimSweepThreads)
   const int c = threadIdx.x % CW, first = threadIdx.x / CW, step = blockDim.x / CW;
   const int lane = threadIdx.x & 31;
   const SweepPlan p = stage_plan<CW, SM>(e, P, st);
-  for (int i = threadIdx.x; i < P.s * kStripLd<CW>; i += blockDim.x) st[i] = kInf;
+  for (int i = threadIdx.x; i < P.s * kStripLd<CW>; i += blockDim.x) st[i] = inf;
   __syncthreads();
   for (int x = threadIdx.x >> 5; x < nx; x += blockDim.x >> 5) {
     int v = inv[x0 + x];
-    if (lane == 0) st[v * kStripLd<CW> + x] = 0;
+    if (lane == 0) st[v * kStripLd<CW> + x] = T(0);
     __syncwarp();
     while (v >= P.b) {
       const int e0 = p.eptr[v], e1 = p.eptr[v + 1];
       if (e0 == e1) break;
-      const int32_t y = st[v * kStripLd<CW> + x];
+      const T y = st[v * kStripLd<CW> + x];
       const int up = p.ent[e0].x;
-      if (y < kInf)
+      if (y < inf)
         for (int i = e0 + lane; i < e1; i += 32) {
           const int2 a = p.ent[i];
-          int32_t *q = st + a.x * kStripLd<CW> + x;
-          *q = __viaddmin_s32(a.y, y, *q);
+          T *q = st + a.x * kStripLd<CW> + x;
+          *q = Dist<T>::relax(weight_of<T>(p.entb ? p.entb[i] : a.y), y, *q);
         }
       __syncwarp();
       v = up;
     }
   }
   __syncthreads();
-  if (P.b > 0) {
+  if (bd.parts != nullptr) {
+    const PartDesc pd = bd.parts[blockIdx.y];
+    const T *D = bd.D + pd.row_base * bd.ldD + (c < nx ? __ldg(bd.vid + pd.start + x0 + c) : 0);
+    for (int k = first; k < P.b; k += step) st[k * kStripLd<CW> + c] = D[k * bd.ldD];
+    __syncthreads();
+  } else if (P.b > 0) {
     for (int k = first; k < P.b; k += step) {
-      const int32_t *row = dB + (int64_t)(P.boff + k) * ldB + P.boff;
-      int32_t acc = st[k * kStripLd<CW> + c];
+      const T *row = bd.dB + (int64_t)(P.boff + k) * bd.ldB + P.boff;
+      T acc = st[k * kStripLd<CW> + c];
 #pragma unroll 4
-      for (int q = 0; q < P.b; q++) acc = __viaddmin_s32(__ldg(row + q), st[q * kStripLd<CW> + c], acc);
+      for (int q = 0; q < P.b; q++) acc = Dist<T>::relax(__ldg(row + q), st[q * kStripLd<CW> + c], acc);
       st[k * kStripLd<CW> + c] = acc;
     }
     __syncthreads();
   }
-  sweep_down<CW>(st, P, p);
+  sweep_down<T, CW>(st, P, p);
   if (c < nx) {
-    int32_t *o = out + out_off[blockIdx.y] + x0 + c;
+    T *o = out + out_off[blockIdx.y] + x0 + c;
     for (int v = first; v < P.s; v += step) o[loc[v] * ld] = st[v * kStripLd<CW> + c];
   }
 }
@@ -259,7 +298,7 @@ __global__ void __launch_bounds__(kElimSweepThreads)
     st[k * kStripLd<CW> + r] = __ldg(dB + rows[2 * (r0 + r)] * ldB + P.boff + k);
   }
   __syncthreads();
-  sweep_down<CW>(st, P, p);
+  sweep_down<int32_t, CW>(st, P, p);
   const int32_t *inv = e.inv + P.voff;
   const int lane = threadIdx.x & 31;
   for (int r = threadIdx.x >> 5; r < nr; r += blockDim.x >> 5) {
@@ -600,37 +639,50 @@ cudaError_t launch_elim_seed(int32_t *M, int64_t ld, int nb, int nfill, const in
   return cudaGetLastError();
 }
 
-cudaError_t launch_elim_up(const ElimDev &e, const int32_t *from, int32_t *M, int64_t ldM,
+template <typename T>
+cudaError_t launch_elim_up(const ElimDev &e, const int32_t *list, int count, const T *from, T *M, int64_t ldM,
                            cudaStream_t stream, int64_t *launches) {
-  if (e.nparts <= 0) return cudaSuccess;
-  const size_t smem = (size_t)e.max_nent * sizeof(int2) + ((size_t)e.max_s + e.max_nlev + 2) * sizeof(int32_t);
+  if (list == nullptr) count = e.nparts;
+  if (count <= 0) return cudaSuccess;
+  if (M != nullptr && e.entb != nullptr) return cudaErrorInvalidValue;
+  const size_t smem = ((size_t)e.max_nent * (e.entb ? 3 : 2) + (size_t)e.max_s + e.max_nlev + 2) * sizeof(int32_t);
   if (smem <= kElimSmem) {
-    cudaError_t err = allow_smem(elim_up_kernel<true>, smem);
+    cudaError_t err = allow_smem(elim_up_kernel<T, true>, smem);
     if (err != cudaSuccess) return err;
-    elim_up_kernel<true><<<e.nparts, kElimUpThreads, smem, stream>>>(e, from, M, ldM);
+    elim_up_kernel<T, true><<<count, kElimUpThreads, smem, stream>>>(e, list, from, M, ldM);
   } else {
-    elim_up_kernel<false><<<e.nparts, kElimUpThreads, 0, stream>>>(e, from, M, ldM);
+    elim_up_kernel<T, false><<<count, kElimUpThreads, 0, stream>>>(e, list, from, M, ldM);
   }
   *launches += 1;
   return cudaGetLastError();
 }
 
+template <typename T>
 cudaError_t launch_elim_close(const ElimDev &e, const int32_t *list, const int64_t *out_off, int count, int max_s,
-                              const int32_t *dB, int64_t ldB, int32_t *out, int64_t ld, cudaStream_t stream,
+                              const ElimBoundary<T> &bd, T *out, int64_t ld, cudaStream_t stream,
                               int64_t *launches) {
   if (count <= 0 || max_s <= 0) return cudaSuccess;
   return for_strip(e, max_s, [&](auto cw, auto sm) -> cudaError_t {
     constexpr int CW = decltype(cw)::value;
     constexpr bool SM = decltype(sm)::value;
     const size_t smem = sweep_bytes<CW>(e, max_s, SM);
-    cudaError_t err = allow_smem(elim_close_kernel<CW, SM>, smem);
+    cudaError_t err = allow_smem(elim_close_kernel<T, CW, SM>, smem);
     if (err != cudaSuccess) return err;
-    elim_close_kernel<CW, SM><<<dim3((max_s + CW - 1) / CW, count), kElimSweepThreads, smem, stream>>>(
-        e, list, out_off, dB, ldB, out, ld);
+    elim_close_kernel<T, CW, SM><<<dim3((max_s + CW - 1) / CW, count), kElimSweepThreads, smem, stream>>>(
+        e, list, out_off, bd, out, ld);
     *launches += 1;
     return cudaGetLastError();
   });
 }
+
+#define FAPB_ELIM(T)                                                                                             \
+  template cudaError_t launch_elim_up<T>(const ElimDev &, const int32_t *, int, const T *, T *, int64_t,        \
+                                         cudaStream_t, int64_t *);                                              \
+  template cudaError_t launch_elim_close<T>(const ElimDev &, const int32_t *, const int64_t *, int, int,        \
+                                            const ElimBoundary<T> &, T *, int64_t, cudaStream_t, int64_t *);
+FAPB_ELIM(int32_t)
+FAPB_ELIM(float)
+#undef FAPB_ELIM
 
 cudaError_t launch_elim_expand(const ElimDev &e, const int64_t *rows, int nrows, const int32_t *dB, int64_t ldB,
                                const int32_t *vid, int n, int32_t *D, int64_t ldD, cudaStream_t stream,

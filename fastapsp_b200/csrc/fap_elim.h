@@ -9,7 +9,9 @@
 // shortest path from v to u through vertices eliminated earlier,
 //   D[v][x] = min over u in N+(v) of W(v, u) + D[u][x]
 // for every x that is not eliminated before v.  Sums and minima of int32 are
-// exact, so the values are those of Floyd-Warshall.  On road-shaped parts
+// exact, so the values are those of Floyd-Warshall (float32 sums associate
+// differently, with fewer roundings on a path than edge after edge).  Directed
+// parts keep both weights of an entry, W(v, u) and W(u, v).  On road-shaped parts
 // N+(v) holds 1.4 vertices on average (a part of 830 vertices: 1,300
 // relaxations per column instead of 830^2), on grid parts about 20.
 #pragma once
@@ -86,7 +88,7 @@ struct ElimPlan {
   std::vector<int32_t> eptr;       // entries of a vertex, relative to ent_off
   std::vector<int32_t> ecol;       // N+(v), plan numbers, descending
   std::vector<int32_t> eend;       // end of the entry's vertex, relative to ent_off
-  std::vector<int32_t> w0;         // weight of the edge (v, u), or the sentinel
+  std::vector<int32_t> w0, w0b;    // weight (bits) of the arc v -> u, of u -> v, or the sentinel
   std::vector<int32_t> lev;
   std::vector<ElimUnit> units;
   std::vector<int32_t> glev, rows8;  // rows8: pairs (slot, local index)
@@ -100,8 +102,8 @@ struct ElimPlan {
   int64_t nent = 0;
 };
 
-// Adjacency of part p (0-based) for the plan: local indices and weights of
-// the undirected edges, both directions listed, no self loops.
+// Arcs of part p (0-based) for the plan: heads (local indices) and weights
+// (bits), no self loops; of two arcs joining the same pair the later one counts.
 struct ElimGraph {
   int32_t s = 0, b = 0, boff = 0;
   std::vector<int32_t> ptr, adj, w;  // w empty: weights come from a dense matrix
@@ -113,7 +115,9 @@ struct ElimGraph {
 // columns fills the shared memory) or more than s^2 / kElimDense entries.
 constexpr int32_t kElimMaxS = 6144;
 constexpr int64_t kElimDense = 16;
-void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, int threads, ElimPlan *out);
+// inf: bits of the sentinel; groups: also build the separator groups.
+void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, int threads, int32_t inf,
+                bool groups, ElimPlan *out);
 // w0 of a one-part plan := offsets of the entries in a matrix whose rows and
 // columns are the part's local indices.
 void elim_offsets(int64_t ld, ElimPlan *plan);
@@ -121,12 +125,13 @@ void elim_offsets(int64_t ld, ElimPlan *plan);
 // Device arrays of a plan.
 struct ElimDev {
   const ElimPart *parts;
-  const int32_t *loc, *inv, *eptr, *ecol, *eend, *w0, *lev;
+  const int32_t *loc, *inv, *eptr, *ecol, *eend, *w0, *w0b, *lev;
   const ElimUnit *units;
   const int32_t *glev, *rows8, *sloc;
   const uint16_t *list;
   const ElimChunk *chunks;
-  int2 *ent;  // {plan number of u, W(v, u)}, written by launch_elim_up
+  int2 *ent;      // {plan number of u, W(v, u)}, written by launch_elim_up
+  int32_t *entb;  // W(u, v); null: symmetric
   int32_t nparts, max_s, max_b, max_nent, max_nlev, max_chunk16, max_chunks;
 };
 
@@ -135,18 +140,32 @@ struct ElimDev {
 cudaError_t launch_elim_seed(int32_t *M, int64_t ld, int nb, int nfill, const int32_t *arcs, int narcs, cudaStream_t stream,
                              int64_t *launches);
 
-// W of every part of the plan, and into M (boundary indices) the shortest
-// paths between a part's boundary vertices through its inner ones.  from:
-// the edges' weights are the elements of this matrix that w0 names (offsets,
+// W of the listed parts (0-based plan parts; null: every part), and into M
+// (boundary indices, symmetric parts only; null: not wanted) the shortest
+// paths between a part's boundary vertices through its inner ones.  from: the
+// edges' weights are the elements of this matrix that w0 names (offsets,
 // elim_offsets) instead of w0 itself.
-cudaError_t launch_elim_up(const ElimDev &e, const int32_t *from, int32_t *M, int64_t ldM,
+template <typename T>
+cudaError_t launch_elim_up(const ElimDev &e, const int32_t *list, int count, const T *from, T *M, int64_t ldM,
                            cudaStream_t stream, int64_t *launches);
 
-// Exact closures of the listed parts (0-based plan parts; list null: all of
-// them in order) from the closed boundary matrix dB (null: the parts have no
-// boundary): out_off[i] + local row * ld + local column.
+// Exact closures of the listed parts (as above) into out_off[i] + local row *
+// ld + local column, from the exact distances of their boundary vertices: the
+// closed boundary matrix dB (null with no rows: the parts have no boundary), or
+// with `parts` (the listed parts' descriptors) the boundary rows of D, which
+// hold every column (sorted position -> column: vid).
+template <typename T>
+struct ElimBoundary {
+  const T *dB;
+  int64_t ldB;
+  const PartDesc *parts;
+  const T *D;
+  int64_t ldD;
+  const int32_t *vid;
+};
+template <typename T>
 cudaError_t launch_elim_close(const ElimDev &e, const int32_t *list, const int64_t *out_off, int count, int max_s,
-                              const int32_t *dB, int64_t ldB, int32_t *out, int64_t ld, cudaStream_t stream,
+                              const ElimBoundary<T> &bd, T *out, int64_t ld, cudaStream_t stream,
                               int64_t *launches);
 
 // Rows of D for the listed boundary vertices (pairs boundary index, row of

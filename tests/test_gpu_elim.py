@@ -113,7 +113,7 @@ def test_elimination_equals_general_path(cuda_ok, name):
     assert np.array_equal(want[p][rows].astype(np.int64), ref)
     # some of the parts, packed and in another order
     some = every[::-2]
-    dg.reserve(int(sum(vn[q] for q in some)))
+    dg.reserve(int(max(sum(vn[q] for q in some), vn[p])))
     for batch in (some, [p]):
         dg.solve(batch, FAP_MODE_BATCHED)
         _same(_blocks(dg, batch), want)
@@ -142,6 +142,54 @@ def test_elimination_gives_the_same_predecessors(cuda_ok, name):
         out.append([dg.copy_path_block(p) for p in range(1, K + 1)])
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def _directed_int():
+    el = G.rmat_graph(11, 9000, seed=33)          # duplicate arcs, hubs, unreachable pairs
+    el.weights = np.ceil(el.weights)
+    el.integral = True
+    return el
+
+
+def _float_rgg():
+    el = G.random_geometric_graph(2100, 3.0, seed=34)
+    el.weights = np.random.default_rng(34).uniform(0.5, 100.0, el.weights.shape[0]).astype(np.float32)
+    return el
+
+
+@pytest.mark.parametrize("name", ["directed_int", "float_rgg", "float_rmat"])
+def test_closures_from_given_boundary_rows(cuda_ok, name):
+    """The SSSP form's closures by elimination (any dtype, directed parts):
+    int32 bit-identical to the Floyd-Warshall closures; float32 within 1e-5 (the
+    sums associate differently) with reachability exact, and the same bits from
+    batches of some of the parts and from the resident cache."""
+    el, K = {"directed_int": (_directed_int(), 4), "float_rgg": (_float_rgg(), 3),
+             "float_rmat": (G.rmat_graph(11, 9000, seed=35), 4)}[name]
+    dg, st2ed, vn, vo, _ = _device(el, K)
+    every = list(range(1, K + 1))
+    dg.set_param("stage1", 1)
+    dg.set_param("eliminate", 0)
+    dg.solve(mode=FAP_MODE_BATCHED)
+    want = _blocks(dg, every)
+    dg.set_param("eliminate", 1)
+    dg.solve(mode=FAP_MODE_BATCHED)
+    got = _blocks(dg, every)
+    for p in every:
+        if name == "directed_int":
+            assert np.array_equal(got[p], want[p]), p
+        else:
+            reach = want[p] < INF
+            assert np.array_equal(got[p] < INF, reach)
+            assert np.all(np.abs(got[p] - want[p])[reach] <= 1e-5 * want[p][reach])
+    dg.reserve(int(vn[1:].max()))
+    for p in every:
+        dg.solve([p], FAP_MODE_BATCHED)
+        assert np.array_equal(dg.copy_block(p).view(np.int32), got[p].view(np.int32))
+    dg.cache_build()
+    for p in every:
+        dg.solve([p], FAP_MODE_BATCHED)
+        assert dg.last_stage1() == 3
+        assert np.array_equal(dg.copy_block(p).view(np.int32), got[p].view(np.int32))
 
 
 def test_asymmetric_weights_keep_the_general_path(cuda_ok):
