@@ -2920,6 +2920,96 @@ cudaError_t launch_minplus_generic(int M, int N, int K, const T *A, int64_t lda,
   return cudaGetLastError();
 }
 
+// The same product from operands copied into padded scratch, whatever their
+// alignment: A to rows of Kp (a multiple of 16), B to rows of Np (a multiple of
+// 128).  The tiles then come by TMA (the generic kernel stages them through
+// registers, element by element when B's rows are not 16-byte aligned), and
+// the result leaves through shared memory in whole rows.  Padding is never
+// stored, and padded rows and columns of a tile are skipped by halves.
+template <typename T>
+__global__ void pack_operand_kernel(T *dst, int64_t ldd, const T *__restrict__ src, int64_t lds, int rows, int cols) {
+  const int i = blockIdx.y;
+  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < ldd; j += (int64_t)gridDim.x * blockDim.x)
+    dst[i * ldd + j] = i < rows && j < cols ? __ldg(src + i * lds + j) : Dist<T>::inf();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(FloydCfg<T, kFloydTile>::THREADS, 2)
+    minplus_packed_kernel(int M, int N, int K, T *__restrict__ Cp, int64_t ldc,
+                          const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                          int *status) {
+  using TC = typename FloydCfg<T, kFloydTile>::TC;
+  using V = typename Vec4<T>::type;
+  extern __shared__ __align__(128) unsigned char mk_smem_raw[];
+  auto sm = tma_smem_init<T, TC>(mk_smem_raw);
+  const int m0 = blockIdx.y * TC::BM, n0 = blockIdx.x * TC::BN;
+  T acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int j = 0; j < 8; j++) acc[i][j] = Dist<T>::inf();
+  if (!tma_minplus_tile<T, TC, true>(&mapA, 0, m0, 0, &mapB, n0, 0, 0, K, acc, sm, M - m0, N - n0)) {
+    if (threadIdx.x == 0) set_status(status, kDevTmaTimeout);
+    return;
+  }
+  constexpr int LD = TC::BN + 4;
+  static_assert(64 * LD * sizeof(T) <= TC::RING_BYTES, "half a tile fits in the ring");
+  T *buf = sm.ring;
+  const int ty = threadIdx.x / TC::TX, tx = threadIdx.x % TC::TX;
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+#pragma unroll
+  for (int g = 0; g < 2; g++) {
+    __syncthreads();
+#pragma unroll
+    for (int l = 0; l < 4; l++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        V v;
+        v.x = acc[4 * g + l][4 * h]; v.y = acc[4 * g + l][4 * h + 1];
+        v.z = acc[4 * g + l][4 * h + 2]; v.w = acc[4 * g + l][4 * h + 3];
+        *reinterpret_cast<V *>(buf + (4 * ty + l) * LD + 64 * h + 4 * tx) = v;
+      }
+    __syncthreads();
+    for (int r = warp; r < 64; r += TC::THREADS / 32) {
+      const int m = m0 + 64 * g + r;
+      if (m >= M) break;
+#pragma unroll
+      for (int c = 0; c < TC::BN; c += 32)
+        if (n0 + c + lane < N) __stcs(Cp + m * ldc + n0 + c + lane, buf[r * LD + c + lane]);
+    }
+  }
+}
+
+int64_t minplus_packed_elems(int M, int N, int K) {
+  const int64_t kp = round_up(K, 16);
+  return round_up(M, kMinplusBM) * kp + kp * round_up(N, kMinplusBN);
+}
+
+template <typename T>
+cudaError_t launch_minplus_packed(int M, int N, int K, const T *A, int64_t lda, const T *B, int64_t ldb, T *C,
+                                  int64_t ldc, T *scratch, int *status, cudaStream_t stream, int64_t *launches) {
+  using FC = FloydCfg<T, kFloydTile>;
+  const int64_t kp = round_up(K, 16), mp = round_up(M, kMinplusBM), np = round_up(N, kMinplusBN);
+  T *Ap = scratch, *Bp = scratch + mp * kp;
+  pack_operand_kernel<T><<<dim3((unsigned)std::min<int64_t>(ceil_div(kp, 256), 64), (unsigned)mp), 256, 0, stream>>>(
+      Ap, kp, A, lda, M, K);
+  pack_operand_kernel<T><<<dim3((unsigned)std::min<int64_t>(ceil_div(np, 256), 64), (unsigned)kp), 256, 0, stream>>>(
+      Bp, np, B, ldb, K, N);
+  *launches += 2;
+  const bool f = Dist<T>::kDtype == FAP_DTYPE_F32;
+  CUtensorMap mapA, mapB;
+  cudaError_t e = make_tmap_3d(&mapA, Ap, f, kp, mp, 1, FC::TC::BK, FC::TC::BM);
+  if (e == cudaSuccess) e = make_tmap_3d(&mapB, Bp, f, np, kp, 1, FC::TC::BN, FC::TC::BK);
+  if (e != cudaSuccess) return e;
+  const size_t smem = FC::SMEM_BYTES;
+  e = cudaFuncSetAttribute(minplus_packed_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  minplus_packed_kernel<T><<<dim3((unsigned)(np / FC::TC::BN), (unsigned)(mp / FC::TC::BM)), FC::THREADS, smem, stream>>>(
+      M, N, K, C, ldc, mapA, mapB, status);
+  *launches += 1;
+  return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // Utilities
 // ---------------------------------------------------------------------------
@@ -3074,6 +3164,9 @@ cudaError_t launch_relax_peak(T *sink, int blocks, int iters, cudaStream_t strea
                                               const int32_t *, cudaStream_t, int64_t *);          \
   template cudaError_t launch_minplus_generic<T>(int, int, int, const T *, int64_t, const T *,    \
                                                  int64_t, T *, int64_t, cudaStream_t, int64_t *); \
+  template cudaError_t launch_minplus_packed<T>(int, int, int, const T *, int64_t, const T *,     \
+                                                int64_t, T *, int64_t, T *, int *, cudaStream_t,  \
+                                                int64_t *);                                       \
   template cudaError_t launch_fill<T>(T *, int64_t, int64_t, int64_t, T, cudaStream_t, int64_t *); \
   template cudaError_t launch_bgraph<T>(const PartDesc *, int, int, const T *, T *, int64_t,       \
                                         const int32_t *, const int32_t *, const T *, int,          \

@@ -370,6 +370,12 @@ cudaError_t launch_minplus_rows(const PartDesc *parts, const RowGroup *groups, i
                                 int64_t *launches);
 
 // Generic C = min(INF, A (x) B).
+// ... with the operands first copied into padded scratch
+// (minplus_packed_elems(M, N, K) elements).
+int64_t minplus_packed_elems(int M, int N, int K);
+template <typename T>
+cudaError_t launch_minplus_packed(int M, int N, int K, const T *A, int64_t lda, const T *B, int64_t ldb, T *C,
+                                  int64_t ldc, T *scratch, int *status, cudaStream_t stream, int64_t *launches);
 template <typename T>
 cudaError_t launch_minplus_generic(int M, int N, int K, const T *A, int64_t lda, const T *B,
                                    int64_t ldb, T *C, int64_t ldc, cudaStream_t stream,
