@@ -424,7 +424,7 @@ __device__ __forceinline__ void merge_unit(char *st, const int4 *body, int nu, c
       }
     }
   };
-#pragma unroll 1
+#pragma unroll 2
   for (const int4 *end = coef; list < end; list++, coef += NR) {
     const int4 u = *list;
     step(u.x, coef);
@@ -461,9 +461,9 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
 }
 
 // The part's chunks through a ring of kMergeRing buffers in shared memory,
-// copied asynchronously two chunks ahead; a chunk's units are independent, a
+// copied asynchronously a chunk ahead; a chunk's units are independent, a
 // barrier ends every chunk.
-constexpr int kMergeRing = 3;
+constexpr int kMergeRing = 2;
 template <int MODE, bool OWN>
 __device__ __forceinline__ void merge_stream(char *st, int4 *ring, int buf16, const ElimChunk *chunks, int nchunks,
                                              const int4 *__restrict__ stream, const MergeOut &o) {
@@ -476,11 +476,10 @@ __device__ __forceinline__ void merge_stream(char *st, int4 *ring, int buf16, co
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   fetch(0);
-  fetch(1);
   for (int c = 0; c < nchunks; c++) {
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();  // chunk c is here, and every warp is done with chunk c - 1
-    fetch(c + 2);
+    fetch(c + 1);
     const int4 *buf = ring + (c % kMergeRing) * buf16;
     const int n = chunks[c].nunits;
     for (int i = warp; i < n; i += nwarps) {
@@ -508,7 +507,7 @@ __host__ __device__ inline size_t merge_smem(int slots, int slot_bytes, int chun
 // two strips of 32 columns.  A grid part's row takes 28 relaxations (its
 // boundary: 164), a geometric graph's 5 (27).  Bound by issue: about 100
 // instructions per packed row of 64 columns, of which 39 relax.  Merge of a
-// 256 x 256 grid 22.4 -> 12.8 ms, of a 60,000-vertex geometric graph 9.3 -> 5.7
+// 256 x 256 grid 22.4 -> 9.8 ms, of a 60,000-vertex geometric graph 9.3 -> 5.5
 // (the min-plus tiles before); 384 threads of 85 registers, since at 56 the
 // pair form spills (9.7 ms).
 __global__ void __launch_bounds__(kMergeThreads, 2)

@@ -73,7 +73,10 @@ struct ElimUnit {
 struct ElimChunk {
   int32_t off, n16, nunits, pad_;  // in 16-byte words
 };
-constexpr int32_t kElimChunk16 = 512;
+// (18 KB: a barrier ends every chunk, and one of 8 KB held as few as two units of
+// a grid part's first levels for 12 warps; merge of a 256 x 256 grid 12.8 ms at
+// 8 KB, 9.8 at 18; two buffers of more would leave one CTA on an SM)
+constexpr int32_t kElimChunk16 = 1152;
 constexpr int32_t kElimWide = 1 << 30;
 constexpr int kElimUnitRows = 8;
 __host__ __device__ inline int32_t elim_body16(int32_t nu) {
