@@ -31,7 +31,7 @@ CUDA_LIB = os.path.join(CUDA_HOME, "targets", "x86_64-linux", "lib")
 METIS_A = os.path.join(CUDA_LIB, "libmetis_static.a")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden",
+COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden,-mpopcnt",
           "-I" + INCLUDE, "-I" + CSRC]
 SOURCES = ["fap_device.cu", "fap_capi.cu", "fap_elim.cu", "fap_elim.cpp", "fap_floyd64.cu", "fap_legacy.cu", "fap_noalloc.cu", "fap_host.cpp",
            "fap_serve.cpp"]

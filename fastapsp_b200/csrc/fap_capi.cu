@@ -307,11 +307,9 @@ struct ElimBuf {
       bytes += (src[i].bytes + 255) / 256 * 256;
     }
     FAP_TRY(buf.ensure(std::max<size_t>(bytes, 256)));
-    std::vector<char> host(off[N - 2]);
-    for (int i = 0; i + 2 < N; i++)
-      if (src[i].bytes > 0) std::memcpy(host.data() + off[i], src[i].p, src[i].bytes);
-    FAP_CK(cudaMemcpy(buf.p, host.data(), host.size(), cudaMemcpyHostToDevice));
     char *d = buf.as<char>();
+    for (int i = 0; i + 2 < N; i++)
+      if (src[i].bytes > 0) FAP_CK(cudaMemcpy(d + off[i], src[i].p, src[i].bytes, cudaMemcpyHostToDevice));
     auto at = [&](int i) { return reinterpret_cast<const int32_t *>(d + off[i]); };
     dev = ElimDev{};
     dev.parts = reinterpret_cast<const ElimPart *>(d);
@@ -1397,7 +1395,7 @@ int run_elim(fap_dgraph *G, const PartDesc *dp, int count, int max_s, int32_t *F
 // min-plus tiles: its padded relaxations have to be at most half of the
 // tiles' inner x b.
 bool merge_ok(const fap_dgraph *G, int32_t p) {
-  return elim_merge_fits(G->el.plan, G->el.plan.parts[p - 1].nslots) && G->vnum[p] > G->bnum[p] &&
+  return G->bnum[p] > kThinBoundary && elim_merge_fits(G->el.plan, G->el.plan.parts[p - 1].nslots) && G->vnum[p] > G->bnum[p] &&
          2 * G->el.plan.group_work[p - 1] <= (int64_t)(G->vnum[p] - G->bnum[p]) * G->bnum[p];
 }
 

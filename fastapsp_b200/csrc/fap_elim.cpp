@@ -56,6 +56,7 @@ void eliminate(const ElimGraph &g, int32_t inf, PartPlan *out) {
   };
   for (int32_t i = b; i < s; i++) push(i);
   std::vector<int32_t> nptr(s, 0), ncnt(s, 0), nbr;  // N+ of the eliminated vertices
+  std::vector<int> words;
   std::vector<char> gone(s, 0);
   std::vector<int32_t> order;
   order.reserve(std::max(0, s - b));
@@ -73,15 +74,21 @@ void eliminate(const ElimGraph &g, int32_t inf, PartPlan *out) {
       for (uint64_t x = rv[w]; x != 0; x &= x - 1) nbr.push_back(w * 64 + __builtin_ctzll(x));
     ncnt[v] = (int32_t)nbr.size() - nptr[v];
     if (nbr.size() > limit) return;
+    words.clear();  // (the neighbours sit in a few words of the row)
+    for (int w = 0; w < W; w++)
+      if (rv[w] != 0) words.push_back(w);
     for (int32_t i = 0; i < ncnt[v]; i++) {
       const int32_t u = nbr[nptr[v] + i];
       uint64_t *ru = &A[(size_t)u * W];
       int32_t d = 0;
-      for (int w = 0; w < W; w++) d += __builtin_popcountll(ru[w] |= rv[w]);
+      for (int w : words) {
+        d += __builtin_popcountll(rv[w] & ~ru[w]);
+        ru[w] |= rv[w];
+      }
       ru[v / 64] &= ~(uint64_t(1) << (v % 64));
       ru[u / 64] &= ~(uint64_t(1) << (u % 64));
       if (u < b) continue;
-      deg[u] = d - 2;  // (v and u itself, both set by rv or before)
+      deg[u] += d - 2;  // (u's own bit came with rv, v is gone)
       up[u] = std::max(up[u], up[v] + 1);
       push(u);
     }
@@ -231,7 +238,7 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
         pp[p].b = g.b;
         if (g.s <= kElimMaxS) eliminate(g, inf, &pp[p]);
         if (!pp[p].ok) dense = true;
-        else if (groups && g.b > 0) group_rows(&pp[p]);
+        else if (groups && g.b > kThinBoundary) group_rows(&pp[p]);  // (the others take the thin merge)
       }
     } catch (...) {
       failed = true;
