@@ -532,10 +532,10 @@ __global__ void __launch_bounds__(FloydCfg<T, kFloydTile>::THREADS, 2)
 
 // Pivot blocks of 64 (fap_floyd64.cu) or 128.  Measured, int32, us: s = 64
 // 45 / 65, 100 77 / 73 (two blocks against one), 129 96 / 134, 500 211 / 430,
-// 1,500 731 / 1,243, 4,000 6,190 / 6,800, 5,538 15,500 / 14,100: from there the
+// 1,500 731 / 1,243, 4,000 5,690 / 6,800, 5,538 15,500 / 14,100: from there the
 // remainder bounds both, and with 64 pivots a pass over the matrix it is read
 // and written twice as often.  A symmetric matrix (half of the tiles) stays
-// ahead: 5,538 12,100 / 15,600.
+// ahead: 5,538 10,900 / 15,600.
 constexpr int kFloyd64Min = 112, kFloyd64Max = 4608, kFloyd64MaxSym = 8192;
 
 template <typename T>

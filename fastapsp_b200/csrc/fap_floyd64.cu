@@ -172,9 +172,12 @@ __global__ void __launch_bounds__(kThreads) floyd64_panel_kernel(T *mat, int64_t
 // Remainder of pivot block kb: CTA (column tile, pair of row tiles) of the
 // tiles outside the pivot's row and column; the last CTA of x = 0 closes the
 // diagonal tile in place (the panels closed it for themselves).  SYM: only row
-// tiles up to the column tile, each also stored transposed.
-template <typename T, bool SYM>
-__global__ void __launch_bounds__(kThreads, 2) floyd64_rest_kernel(T *mat, int64_t ld, int kb, int nb) {
+// tiles up to the column tile, each also stored transposed.  CTAS: per SM; a
+// grid of more than two waves takes three at 80 registers (s = 4,000 6.19 ->
+// 5.69 ms; symmetric 5,538 12.1 -> 10.9), a smaller one two without spills
+// (1,500 732 us, 784 with three).
+template <typename T, bool SYM, int CTAS>
+__global__ void __launch_bounds__(kThreads, CTAS) floyd64_rest_kernel(T *mat, int64_t ld, int kb, int nb) {
   extern __shared__ __align__(16) unsigned char f64_smem[];
   T *A = reinterpret_cast<T *>(f64_smem), *B = A + 2 * kB * kLd;
   if (blockIdx.y == gridDim.y - 1) {
@@ -220,8 +223,11 @@ __global__ void __launch_bounds__(kThreads, 2) floyd64_rest_kernel(T *mat, int64
 
 template <typename T, bool SYM>
 cudaError_t run(T *mat, int64_t ld, int nb, cudaStream_t stream, int64_t *launches) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t smem = (size_t)3 * kB * kLd * sizeof(T);
-  auto rest = floyd64_rest_kernel<T, SYM>;
+  const bool many = (int64_t)(nb - 1) * (nb / 2) / (SYM ? 2 : 1) > 4 * (int64_t)sms;
+  auto rest = many ? floyd64_rest_kernel<T, SYM, 3> : floyd64_rest_kernel<T, SYM, 2>;
   cudaError_t e = cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   for (int kb = 0; kb < nb; kb++) {
