@@ -764,6 +764,11 @@ int build_elim(fap_dgraph *G) {
   // (float32 parts keep min-plus over the boundary, which distance rows from
   // the resident cache match bit for bit; their symmetry is sym_local's)
   FAP_TRY(G->el.upload(!G->sym_local));
+  if (G->el.plan.stream16 > 0) {  // (with the plan, so that a server counts them as held)
+    FAP_TRY(G->d_coef32.ensure((size_t)G->el.plan.stream16 * 16));
+    FAP_TRY(G->d_coef16.ensure((size_t)G->el.plan.stream16 * 16));
+    FAP_TRY(G->d_far.ensure(G->el.plan.parts.size() * 4));
+  }
   if (!i32 || !G->sym_local) return FAP_OK;
   std::vector<std::array<int32_t, 3>> cross;
   for (int32_t p = 1; p <= K; p++)
@@ -1514,11 +1519,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
     FAP_TRY(G->sssp_scratch.ensure_async(
         (size_t)std::max(sssp_scratch_rows(G->n, (int)G->src.size()), 1) * (size_t)G->n * 4, st));
   if (!G->merge.empty()) {
-    const ElimPlan &pl = G->el.plan;
     FAP_TRY(G->d_merge.ensure_async(G->merge.size() * sizeof(int2), st));
-    FAP_TRY(G->d_coef32.ensure_async(std::max<size_t>((size_t)pl.stream16, 1) * 16, st));
-    FAP_TRY(G->d_coef16.ensure_async(std::max<size_t>((size_t)pl.stream16, 1) * 16, st));
-    FAP_TRY(G->d_far.ensure_async(pl.parts.size() * 4, st));
     if (G->pack16 && !G->d_pk_tiles.p) {
       FAP_TRY(G->d_pk_tiles.ensure_async(2 * sizeof(unsigned long long), st));
       FAP_CK(cudaMemsetAsync(G->d_pk_tiles.p, 0, 2 * sizeof(unsigned long long), st));
