@@ -191,7 +191,9 @@ FAP_API int fap_graph_sssp_rows(fap_dgraph *g, const int32_t *sources, int32_t c
  * boundary-row column is shifted by its least finite entry and the part's
  * largest finite inner-to-boundary distance plus the tile's largest shifted
  * entry is below 16383; other tiles run in int32; the results are the same
- * int32 values either way; 0: int32 everywhere); "minplus_prepack" (default
+ * int32 values either way; 0: int32 everywhere; with "eliminate" a 64-column
+ * strip of a separator group is such a tile, unsigned, with 32767 as its
+ * bound); "minplus_prepack" (default
  * 1: the packed tiles read operands packed once per solve, the boundary rows
  * as 16-bit columns and the inner-to-boundary distances with both halves
  * equal, and the packed tiles of the boundary graph's tiled expansion read
@@ -225,7 +227,8 @@ FAP_API int fap_graph_set_param(fap_dgraph *g, const char *key, double value);
 FAP_API int fap_queue_order_check(const int32_t *part_sizes, int32_t nparts, int sym);
 
 /* Min-plus tiles run in the packed 16-bit form and in all, counted over
- * every solve of g so far (see "minplus_pack16").  Synchronous. */
+ * every solve of g so far, 64-column strips of the separator-group merge
+ * among them (see "minplus_pack16").  Synchronous. */
 FAP_API int fap_graph_pack16_tiles(fap_dgraph *g, int64_t *packed, int64_t *total);
 /* The same for the tiles of the boundary graph's tiled expansion (int32,
  * Bellman-Ford closure of the boundary graph): rows of the closed boundary
