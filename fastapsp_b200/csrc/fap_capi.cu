@@ -833,6 +833,16 @@ bool elim_ok(const fap_dgraph *G, int64_t sources) {
   return sources < 0 || (G->el2.plan.ok && ldB * ldB <= std::max<int64_t>(sources * G->n, kElimBatchElems));
 }
 
+// Words of dB, with the work space of its Floyd closure after it from 1,024
+// vertices on, where the 96 KB are at most 2% of dB (the size that a cache build
+// announces does not grow for small graphs).
+bool bgraph_has_work(int64_t ldB) { return ldB > 1024 && ldB <= round_up(kBgraphFloydMax, kFloydTile); }
+int64_t bgraph_words(int64_t ldB) { return ldB * ldB + (bgraph_has_work(ldB) ? kFloyd64Work : 0); }
+template <typename T>
+T *bgraph_work(T *dB, int64_t ldB) {
+  return bgraph_has_work(ldB) ? dB + ldB * ldB : nullptr;
+}
+
 // Whether the SSSP form closes the parts by elimination from its boundary rows
 // (any dtype, directed or not) instead of Floyd-Warshall.
 bool elim_given_ok(const fap_dgraph *G) { return G->eliminate && G->el.plan.ok && !G->floyd_per_cta; }
@@ -1195,7 +1205,7 @@ int prepare_bgraph(fap_dgraph *G, const std::vector<PartDesc> &parts, bool col_t
   // (the Bellman-Ford closure writes dB's columns padded per part, so that
   // the expansion's TMA boxes start on 16-byte boundaries)
   G->ldB = round_up(std::max<int64_t>(bgraph_bf(G) ? G->bpcol[G->K + 1] : G->total_b, 1), kFloydTile);
-  FAP_TRY(G->d_dB.ensure((size_t)G->ldB * G->ldB * 4));
+  FAP_TRY(G->d_dB.ensure((size_t)bgraph_words(G->ldB) * 4));
   const int64_t ldFB = parts.empty() ? kFloydTile : parts[0].ldf;
   FAP_TRY(G->d_FB.ensure((size_t)std::max<int64_t>(G->total_b, 1) * ldFB * 4));
   FAP_TRY(G->d_bpart.ensure(bp.size() * sizeof(BPart)));
@@ -1236,7 +1246,7 @@ int close_bgraph(fap_dgraph *G, const PartDesc *dp, int np, int max_b, const T *
                             G->w.as<const T>(), G->n, G->d_gid.as<const int32_t>(),
                             G->d_ed2st.as<const int32_t>(), G->d_bpart.as<const BPart>(), st, L));
     FAP_CK(launch_floyd_matrix<T>(dB, G->ldB, (int)ceil_div(G->total_b, kFloydTile), status, st, L,
-                                  (int)G->total_b));
+                                  (int)G->total_b, false, bgraph_work(dB, G->ldB)));
     return FAP_OK;
   }
   const int z = bgraph_ztiles(G);
@@ -1321,7 +1331,7 @@ int expand_bgraph(fap_dgraph *G, const PartDesc *dp, int np, int max_s, const T 
 int prepare_elim(fap_dgraph *G, const std::vector<PartDesc> &parts, bool given = false) {
   if (!given) {
     G->ldB = round_up(std::max<int64_t>(G->total_b, 1), kFloydTile);
-    FAP_TRY(G->d_dB.ensure((size_t)G->ldB * G->ldB * 4));
+    FAP_TRY(G->d_dB.ensure((size_t)bgraph_words(G->ldB) * 4));
   }
   std::vector<int32_t> list;
   std::vector<int64_t> off{0}, rows;  // (the first offset is the boundary graph's own)
@@ -1381,7 +1391,7 @@ int run_elim(fap_dgraph *G, const PartDesc *dp, int count, int max_s, int32_t *F
     FAP_CK(launch_elim_close<int32_t>(G->el2.dev, nullptr, off, 1, nb, ElimBoundary<int32_t>{}, dB, G->ldB, st, L));
   } else {
     FAP_CK(launch_floyd_matrix<int32_t>(dB, G->ldB, (int)ceil_div(nb, kFloydTile), status, st, L, nb,
-                                        true));
+                                        true, bgraph_work(dB, G->ldB)));
   }
   FAP_CK(record_event(ev2, st));
   FAP_CK(launch_elim_close<int32_t>(G->el.dev, G->d_elist.as<const int32_t>(), off + 1, count, max_s,
@@ -2285,16 +2295,18 @@ extern "C" int fap_op_floyd(fap_ctx *c, int dtype, int32_t s, void *mat, int64_t
   cudaStream_t st = c->stream;
   const int64_t ldp = round_up(s, kFloydTile);
   FAP_CK(cudaMemsetAsync(c->status.p, 0, sizeof(int), st));
-  FAP_TRY(c->scratch.ensure((size_t)ldp * ldp * 4));
+  FAP_TRY(c->scratch.ensure(((size_t)ldp * ldp + kFloyd64Work) * 4));
   int64_t L = 0;
   if (dtype == FAP_DTYPE_I32) {
     int32_t *p = c->scratch.as<int32_t>();
     FAP_CK(launch_pad_copy<int32_t>(p, ldp, static_cast<const int32_t *>(mat), ld, s, st, &L));
-    FAP_CK(launch_floyd_matrix<int32_t>(p, ldp, (int)(ldp / kFloydTile), c->status.as<int>(), st, &L, s));
+    FAP_CK(launch_floyd_matrix<int32_t>(p, ldp, (int)(ldp / kFloydTile), c->status.as<int>(), st, &L, s,
+                                        false, p + ldp * ldp));
   } else {
     float *p = c->scratch.as<float>();
     FAP_CK(launch_pad_copy<float>(p, ldp, static_cast<const float *>(mat), ld, s, st, &L));
-    FAP_CK(launch_floyd_matrix<float>(p, ldp, (int)(ldp / kFloydTile), c->status.as<int>(), st, &L, s));
+    FAP_CK(launch_floyd_matrix<float>(p, ldp, (int)(ldp / kFloydTile), c->status.as<int>(), st, &L, s,
+                                        false, p + ldp * ldp));
   }
   FAP_CK(cudaMemcpy2DAsync(mat, (size_t)ld * 4, c->scratch.p, (size_t)ldp * 4, (size_t)s * 4, (size_t)s,
                            cudaMemcpyDeviceToDevice, st));
@@ -3322,7 +3334,7 @@ extern "C" int fap_graph_cache_bytes(const fap_dgraph *G, int64_t *bytes, int *b
     if (bmethod_ok(G)) {
       const int64_t ldB =
           round_up(std::max<int64_t>(bgraph_bf(G) ? G->bpcol[G->K + 1] : G->total_b, 1), kFloydTile);
-      *bytes = cs.bytes(G) + (int64_t)alloc_size((size_t)(ldB * ldB * 4)) +
+      *bytes = cs.bytes(G) + (int64_t)alloc_size((size_t)bgraph_words(ldB) * 4) +
                (int64_t)alloc_size((size_t)std::max<int64_t>(G->total_b, 1) * cs.ldf * 4) +
                (int64_t)alloc_size((size_t)(G->K + 1) * sizeof(BPart)) +
                (int64_t)alloc_size((size_t)std::max<int64_t>(2 * G->total_b, 2) * 8);

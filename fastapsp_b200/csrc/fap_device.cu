@@ -531,22 +531,22 @@ __global__ void __launch_bounds__(FloydCfg<T, kFloydTile>::THREADS, 2)
 }
 
 // Pivot blocks of 64 (fap_floyd64.cu) or 128.  Measured, int32, us: s = 64
-// 45 / 65, 100 77 / 73 (two blocks against one), 129 96 / 134, 500 211 / 430,
-// 1,500 731 / 1,243, 4,000 5,690 / 6,800, 5,538 15,500 / 14,100: from there the
-// remainder bounds both, and with 64 pivots a pass over the matrix it is read
+// 45 / 65, 129 89 / 134, 500 185 / 430, 1,500 544 / 1,243, 4,000 5,420 / 6,800;
+// without work space 100 77 / 73 (two blocks against one), 1,500 731 / 1,243,
+// 5,538 15,500 / 14,100: from there the remainder bounds both, and with 64 pivots a pass over the matrix it is read
 // and written twice as often.  A symmetric matrix (half of the tiles) stays
-// ahead: 5,538 10,900 / 15,600.
+// ahead: 5,538 10,900 / 15,600 without work space.
 constexpr int kFloyd64Min = 112, kFloyd64Max = 4608, kFloyd64MaxSym = 8192;
 
 template <typename T>
 cudaError_t launch_floyd_matrix(T *mat, int64_t ld, int nb, int *status, cudaStream_t stream,
-                                int64_t *launches, int s, bool sym) {
+                                int64_t *launches, int s, bool sym, T *work) {
   using FC = FloydCfg<T, kFloydTile>;
   if (nb <= 0) return cudaSuccess;
   if (s < 0 || s > nb * kFloydTile) s = nb * kFloydTile;
   if (s <= (nb - 1) * kFloydTile) return cudaErrorInvalidValue;  // the last block holds real rows
   if (s <= (sym ? kFloyd64MaxSym : kFloyd64Max) && (s <= kFloydTile / 2 || s > kFloyd64Min))
-    return launch_floyd64<T>(mat, ld, s, sym, stream, launches);
+    return launch_floyd64<T>(mat, ld, s, sym, work, stream, launches);
   CUtensorMap mapA, mapB;
   cudaError_t e = make_arena_tmaps<T>(mat, ld, 1, &mapA, &mapB);
   if (e != cudaSuccess) return e;
@@ -3252,7 +3252,7 @@ cudaError_t launch_relax_peak(T *sink, int blocks, int iters, cudaStream_t strea
                                         cudaStream_t, int64_t *);                                 \
   template cudaError_t launch_floyd_parts<T>(const PartDesc *, int, T *, int64_t, T *, int64_t,   \
                                              const int32_t *, int *, cudaStream_t, int64_t *);    \
-  template cudaError_t launch_floyd_matrix<T>(T *, int64_t, int, int *, cudaStream_t, int64_t *, int, bool); \
+  template cudaError_t launch_floyd_matrix<T>(T *, int64_t, int, int *, cudaStream_t, int64_t *, int, bool, T *); \
   template cudaError_t launch_floyd_parts_multi<T>(const PartDesc *, int, int, T *, int64_t, int *, \
                                                    cudaStream_t, int64_t *);                      \
   template cudaError_t launch_floyd_queue<T>(const PartDesc *, int, T *, int64_t, const FloydQueue &, \

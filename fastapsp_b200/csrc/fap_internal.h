@@ -211,11 +211,14 @@ cudaError_t launch_pad_copy(T *dst, int64_t ld_dst, const T *src, int64_t ld_src
                             int64_t *launches);
 
 // launch_floyd_matrix in pivot blocks of 64; sym: the matrix is symmetric.
+// work: kFloyd64Work words of the call's own, 16-byte aligned (panels then run
+// beside the remainder of the block before), or NULL.
+constexpr int64_t kFloyd64Work = 6 * 64 * 64;
 template <typename T>
-cudaError_t launch_floyd64(T *mat, int64_t ld, int s, bool sym, cudaStream_t stream, int64_t *launches);
+cudaError_t launch_floyd64(T *mat, int64_t ld, int s, bool sym, T *work, cudaStream_t stream, int64_t *launches);
 template <typename T>
 cudaError_t launch_floyd_matrix(T *mat, int64_t ld, int nb, int *status, cudaStream_t stream,
-                                int64_t *launches, int s = -1, bool sym = false);
+                                int64_t *launches, int s = -1, bool sym = false, T *work = nullptr);
 
 // Boundary rows of the listed parts: F[i][j] -> D[row_base+i][st2ed[start+j]].
 template <typename T>

@@ -44,3 +44,59 @@ def test_floyd_blocks_of_64(cuda_ok, s, dtype):
         reach = want < INF
         assert np.array_equal(got < INF, reach)
         assert np.all(np.abs(got - want)[reach] <= s * 2.0 ** -24 * want[reach])
+
+
+@pytest.mark.parametrize("dtype", ["i32", "f32"])
+@pytest.mark.parametrize("s", [66, 255, 2240, 2369])
+def test_floyd_panels_beside_the_remainder(cuda_ok, s, dtype):
+    """Two pivot blocks, an even and an odd number of them, and both launch
+    shapes of the remainder (35 and 38 blocks), against pivots one by one on
+    the device; tolerance as above."""
+    import torch
+    rng = np.random.default_rng(s)
+    w = rng.uniform(0.0, 1000.0, (s, 6))
+    m = np.full((s, s), INF)
+    np.minimum.at(m, (np.repeat(np.arange(s), 6), rng.integers(0, s, 6 * s)),
+                  (np.floor(w) if dtype == "i32" else w.astype(np.float32)).ravel())
+    np.fill_diagonal(m, 0.0)
+    want = torch.from_numpy(m).cuda()
+    for k in range(s):
+        torch.minimum(want, want[:, k:k + 1] + want[k:k + 1], out=want)
+    want.clamp_(max=INF)
+    got = torch.from_numpy(m).to(torch.int32 if dtype == "i32" else torch.float32).cuda()
+    ctx = Context(0)
+    torch.cuda.synchronize()
+    ctx.floyd(got, FAP_DTYPE_I32 if dtype == "i32" else FAP_DTYPE_F32)
+    ctx.sync()
+    got = got.double()
+    if dtype == "i32":
+        assert torch.equal(got, want)
+    else:
+        reach = want < INF
+        assert torch.equal(got < INF, reach)
+        assert bool(((got - want).abs()[reach] <= s * 2.0 ** -24 * want[reach]).all())
+
+
+def test_symmetric_boundary_graph_panels_beside_the_remainder(cuda_ok):
+    """A boundary graph of more than 2,048 vertices (symmetric tiles) after the
+    elimination, bit for bit against the general path."""
+    from fastapsp_b200 import DeviceGraph, fapGraph
+    from fastapsp_b200 import generators as G
+    el = G.grid_graph(112, 111, extra_frac=0.01, wmin=1, wmax=100, drop_frac=0.0, seed=3)
+    ro, col, w = G.edges_to_csr(el)
+    K = 30
+    g = fapGraph.from_csr(el.n, int(col.shape[0]), ro, col, w, K, directed=el.directed)
+    g.preCondition()
+    vn, vo, bn = g.partInfo()
+    assert 2048 < int(np.asarray(bn).sum()) <= 8192
+    dg = DeviceGraph(Context(0), ro, col, w)
+    dg.set_parts(K, g.getGraphId(), g.getMapping(), vn, vo, bn)
+    dg.reserve()
+    out = []
+    for eliminate in (1, 0):
+        dg.set_param("eliminate", eliminate)
+        dg.solve()
+        assert ("elimination" in dg.stage1_name()) == bool(eliminate)
+        out.append([dg.copy_block(p) for p in range(1, K + 1)])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
