@@ -55,6 +55,9 @@ struct Dist<float> {
   }
 };
 
+// Blocks a grid may have in y (and z); rows beyond it are walked by a stride.
+constexpr int64_t kMaxGridY = 65535;
+
 __host__ __device__ inline int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 __host__ __device__ inline int64_t ceil_div(int64_t x, int64_t m) { return (x + m - 1) / m; }
 

@@ -3033,10 +3033,11 @@ cudaError_t launch_minplus_generic(int M, int N, int K, const T *A, int64_t lda,
 // the result leaves through shared memory in whole rows.  Padding is never
 // stored, and padded rows and columns of a tile are skipped by halves.
 template <typename T>
-__global__ void pack_operand_kernel(T *dst, int64_t ldd, const T *__restrict__ src, int64_t lds, int rows, int cols) {
-  const int i = blockIdx.y;
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < ldd; j += (int64_t)gridDim.x * blockDim.x)
-    dst[i * ldd + j] = i < rows && j < cols ? __ldg(src + i * lds + j) : Dist<T>::inf();
+__global__ void pack_operand_kernel(T *dst, int64_t ldd, const T *__restrict__ src, int64_t lds, int64_t dst_rows,
+                                    int rows, int cols) {
+  for (int64_t i = blockIdx.y; i < dst_rows; i += gridDim.y)
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < ldd; j += (int64_t)gridDim.x * blockDim.x)
+      dst[i * ldd + j] = i < rows && j < cols ? __ldg(src + i * lds + j) : Dist<T>::inf();
 }
 
 template <typename T>
@@ -3097,14 +3098,19 @@ cudaError_t launch_minplus_packed(int M, int N, int K, const T *A, int64_t lda, 
   using FC = FloydCfg<T, kFloydTile>;
   const int64_t kp = round_up(K, 16), mp = round_up(M, kMinplusBM), np = round_up(N, kMinplusBN);
   T *Ap = scratch, *Bp = scratch + mp * kp;
-  pack_operand_kernel<T><<<dim3((unsigned)std::min<int64_t>(ceil_div(kp, 256), 64), (unsigned)mp), 256, 0, stream>>>(
-      Ap, kp, A, lda, M, K);
-  pack_operand_kernel<T><<<dim3((unsigned)std::min<int64_t>(ceil_div(np, 256), 64), (unsigned)kp), 256, 0, stream>>>(
-      Bp, np, B, ldb, K, N);
-  *launches += 2;
+  // (tall and deep products have more rows than a grid's 65,535 in y)
+  auto pack = [&](T *dst, int64_t ldd, const T *src, int64_t lds, int64_t dst_rows, int rows, int cols) -> cudaError_t {
+    const dim3 grid((unsigned)std::min<int64_t>(ceil_div(ldd, 256), 64), (unsigned)std::min<int64_t>(dst_rows, kMaxGridY));
+    pack_operand_kernel<T><<<grid, 256, 0, stream>>>(dst, ldd, src, lds, dst_rows, rows, cols);
+    *launches += 1;
+    return cudaGetLastError();
+  };
+  cudaError_t e = pack(Ap, kp, A, lda, mp, M, K);
+  if (e == cudaSuccess) e = pack(Bp, np, B, ldb, kp, K, N);
+  if (e != cudaSuccess) return e;
   const bool f = Dist<T>::kDtype == FAP_DTYPE_F32;
   CUtensorMap mapA, mapB;
-  cudaError_t e = make_tmap_3d(&mapA, Ap, f, kp, mp, 1, FC::TC::BK, FC::TC::BM);
+  e = make_tmap_3d(&mapA, Ap, f, kp, mp, 1, FC::TC::BK, FC::TC::BM);
   if (e == cudaSuccess) e = make_tmap_3d(&mapB, Bp, f, np, kp, 1, FC::TC::BN, FC::TC::BK);
   if (e != cudaSuccess) return e;
   const size_t smem = FC::SMEM_BYTES;

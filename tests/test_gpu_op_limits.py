@@ -1,0 +1,32 @@
+"""Operators on matrices with more rows than a grid has blocks in y (65,535):
+the shapes an operator takes do not depend on how its operands are staged."""
+import pytest
+
+from fastapsp_b200 import FAP_DTYPE_F32, FAP_DTYPE_I32, Context
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,M,N,K", [("i32", 70000, 1000, 16),      # tall
+                                         ("i32", 130, 130, 66000),      # deep
+                                         ("f32", 70000, 1001, 16),      # (unaligned rows)
+                                         ("f32", 130, 131, 66000)])
+def test_tall_and_deep_minplus(cuda_ok, dtype, M, N, K):
+    """Products of at least 1e9 relaxations: minima of exact int32 sums, or of
+    float32 sums rounded once, are the same in any order."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M)
+    t = torch.int32 if dtype == "i32" else torch.float32
+    a = (torch.rand((M, K), generator=g, device="cuda") * 1000).to(t)
+    b = (torch.rand((K, N), generator=g, device="cuda") * 1000).to(t)
+    far = torch.rand((M, K), generator=g, device="cuda") < 0.1
+    a.masked_fill_(far, 100000000)
+    want = torch.full((M, N), 100000000, dtype=t, device="cuda")
+    step = max(1, 100000000 // (M * N))
+    for k in range(0, K, step):
+        torch.minimum(want, (a[:, k:k + step, None] + b[None, k:k + step]).amin(1), out=want)
+    c = torch.full((M, N), 7, dtype=t, device="cuda")
+    ctx = Context(0)
+    torch.cuda.synchronize()
+    ctx.minplus(a, b, c, FAP_DTYPE_I32 if dtype == "i32" else FAP_DTYPE_F32)
+    assert torch.equal(c, want)
