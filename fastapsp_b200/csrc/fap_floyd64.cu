@@ -370,15 +370,16 @@ cudaError_t run(T *mat, int64_t ld, int nb, T *work, cudaStream_t stream, int64_
 template <typename T>
 __global__ void pad_copy_kernel(T *dst, int64_t ldd, const T *__restrict__ src, int64_t lds, int s) {
   using V = typename Vec4<T>::type;
-  const int i = blockIdx.y;
-  for (int j = 4 * (blockIdx.x * blockDim.x + threadIdx.x); j < ldd; j += 4 * gridDim.x * blockDim.x) {
-    T a[4];
+  for (int64_t i = blockIdx.y; i < ldd; i += gridDim.y)
+    for (int64_t j = 4 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); j < ldd;
+         j += 4 * (int64_t)gridDim.x * blockDim.x) {
+      T a[4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) a[q] = i < s && j + q < s ? __ldg(src + i * lds + j + q) : Dist<T>::inf();
-    V v;
-    v.x = a[0]; v.y = a[1]; v.z = a[2]; v.w = a[3];
-    *reinterpret_cast<V *>(dst + i * ldd + j) = v;
-  }
+      for (int q = 0; q < 4; q++) a[q] = i < s && j + q < s ? __ldg(src + i * lds + j + q) : Dist<T>::inf();
+      V v;
+      v.x = a[0]; v.y = a[1]; v.z = a[2]; v.w = a[3];
+      *reinterpret_cast<V *>(dst + i * ldd + j) = v;
+    }
 }
 
 }  // namespace
@@ -386,8 +387,8 @@ __global__ void pad_copy_kernel(T *dst, int64_t ldd, const T *__restrict__ src, 
 template <typename T>
 cudaError_t launch_pad_copy(T *dst, int64_t ldd, const T *src, int64_t lds, int s, cudaStream_t stream,
                             int64_t *launches) {
-  pad_copy_kernel<T><<<dim3((unsigned)ceil_div(ldd, 4 * kThreads), (unsigned)ldd), kThreads, 0, stream>>>(dst, ldd, src,
-                                                                                                          lds, s);
+  const dim3 grid((unsigned)ceil_div(ldd, 4 * kThreads), (unsigned)std::min<int64_t>(ldd, kMaxGridY));
+  pad_copy_kernel<T><<<grid, kThreads, 0, stream>>>(dst, ldd, src, lds, s);
   *launches += 1;
   return cudaGetLastError();
 }

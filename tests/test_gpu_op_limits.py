@@ -30,3 +30,28 @@ def test_tall_and_deep_minplus(cuda_ok, dtype, M, N, K):
     torch.cuda.synchronize()
     ctx.minplus(a, b, c, FAP_DTYPE_I32 if dtype == "i32" else FAP_DTYPE_F32)
     assert torch.equal(c, want)
+
+
+def test_floyd_of_more_rows_than_a_grid_has(cuda_ok):
+    """A 65,473 x 65,473 matrix (17 GB, and as much scratch): the ring of unit
+    arcs with one chord closes to known distances."""
+    import torch
+    s, far = 65473, 40000
+    free, _ = torch.cuda.mem_get_info()
+    if free < 45 << 30:
+        pytest.skip("needs 45 GB of device memory")
+    m = torch.full((s, s), 100000000, dtype=torch.int32, device="cuda")
+    at = torch.arange(s, device="cuda")
+    m[at, at] = 0
+    m[at, (at + 1) % s] = 1
+    m[0, far] = 7
+    ctx = Context(0)
+    torch.cuda.synchronize()
+    ctx.floyd(m, FAP_DTYPE_I32)
+    for lo in range(0, s, 8192):
+        i = at[lo:lo + 8192, None]
+        ring = (at - i) % s
+        chord = (-i) % s + 7 + (at - far) % s       # from i to 0, over the chord, on to j
+        assert torch.equal(m[lo:lo + 8192].long(), torch.minimum(ring, chord)), lo
+    del m
+    torch.cuda.empty_cache()
