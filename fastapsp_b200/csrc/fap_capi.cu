@@ -732,7 +732,12 @@ int build_elim(fap_dgraph *G) {
   G->el_sym = false;
   if (G->total_b <= 0) return FAP_OK;
   const bool i32 = G->dtype == FAP_DTYPE_I32;
-  const int32_t inf = i32 ? kInfI32 : 0x4cbebc20;  // (bits of 1e8f)
+  // A float32 arc heavier than the sentinel keeps its weight in a closure
+  // where no path is shorter; the sweeps start from the sentinel and would lose it.
+  if (!i32)
+    for (const uint32_t bits : G->h_w)
+      if (bits > kInfBitsF32) return FAP_OK;  // (weights are finite and at least 0; -0.0 is left to the general path too)
+  const int32_t inf = i32 ? kInfI32 : (int32_t)kInfBitsF32;
   const int threads = std::min(16, (int)std::thread::hardware_concurrency());
   const int32_t K = (int32_t)G->vnum.size() - 1;
   auto bidx = [&](int32_t v) { return G->boff[G->gid[v]] + (G->ed2st[v] - G->voff[G->gid[v]]); };

@@ -1,0 +1,37 @@
+"""What the general path answers, elimination answers too: inputs at the limits
+of the elimination's plans and kernels, with "eliminate" on (the default)
+against 0."""
+import numpy as np
+import pytest
+
+from fastapsp_b200 import FAP_DTYPE_F32, FAP_MODE_BATCHED, Context, DeviceGraph, fapGraph
+from fastapsp_b200 import generators as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("directed", [False, True])
+def test_float_weights_beyond_the_sentinel(cuda_ok, directed):
+    """Arcs of weight 1.5e8 and 3e8 (unreachable is 1e8 and more): whole small
+    weights otherwise, so float32 sums are exact in any order and the blocks
+    have to be the same bits."""
+    el = G.rmat_graph(9, 3000, seed=41) if directed else G.road_graph(900, seed=41)
+    rng = np.random.default_rng(41)
+    el.weights = rng.integers(1, 50, el.weights.shape[0]).astype(np.float32)
+    el.weights[::7] = 1.5e8
+    el.weights[3::11] = 3e8
+    ro, col, w = G.edges_to_csr(el)
+    K = 3
+    fg = fapGraph.from_csr(el.n, int(ro[-1]), ro, col, w, K, directed=el.directed)
+    fg.preCondition()
+    dg = DeviceGraph(Context(0), ro, col, w, FAP_DTYPE_F32)
+    vn, vo, bn = fg.partInfo()
+    dg.set_parts(K, fg.getGraphId(), fg.getMapping(), vn, vo, bn)
+    out = []
+    for eliminate in (0, 1):
+        dg.set_param("eliminate", eliminate)
+        dg.solve(mode=FAP_MODE_BATCHED)
+        out.append([dg.copy_block(p) for p in range(1, K + 1)])
+    assert any((b > 1e8).any() for b in out[0])
+    for p, (a, b) in enumerate(zip(*out), 1):
+        assert np.array_equal(a.view(np.int32), b.view(np.int32)), f"part {p}"
