@@ -533,29 +533,39 @@ int32_t fapGraph::solve(bool path_needed) {
   } catch (const std::system_error &) {  // no thread to be had
     path.assign((size_t)(n * n), -1);
   }
-  const int rc = solve_all(static_cast<int>(mode_));
-  if (rc == FAP_OK) {
-    check(fap_graph_check(dg_), "fap_graph_check");
-    if (path_needed && blank.valid()) blank.get();
-    for (int32_t p = 1; p <= K; p++) {
-      copy_block(p, dist.data() + (size_t)C_BlockVer_offset[p] * n);
-      if (path_needed) copy_path_block(p, path.data() + (size_t)C_BlockVer_offset[p] * n);
-    }
-  } else if (rc == FAP_ERR_NOMEM) {
-    // Fewer than n rows fit on the device: solve and copy group by group.
-    const int64_t rows = reserve_group_rows(max_subgraph_vertexs);
-    if (path_needed && blank.valid()) blank.get();
-    for (int32_t p = 1; p <= K;) {
-      const int32_t next = run_group(p, rows);
-      for (; p < next; p++) {
+  int32_t copied = 0;  // parts 1..copied of dist are this solve's
+  try {
+    const int rc = solve_all(static_cast<int>(mode_));
+    if (rc == FAP_OK) {
+      check(fap_graph_check(dg_), "fap_graph_check");
+      if (path_needed && blank.valid()) blank.get();
+      for (int32_t p = 1; p <= K; p++) {
         copy_block(p, dist.data() + (size_t)C_BlockVer_offset[p] * n);
+        copied = p;
         if (path_needed) copy_path_block(p, path.data() + (size_t)C_BlockVer_offset[p] * n);
       }
+    } else if (rc == FAP_ERR_NOMEM) {
+      // Fewer than n rows fit on the device: solve and copy group by group.
+      const int64_t rows = reserve_group_rows(max_subgraph_vertexs);
+      if (path_needed && blank.valid()) blank.get();
+      for (int32_t p = 1; p <= K;) {
+        const int32_t next = run_group(p, rows);
+        for (; p < next; p++) {
+          copy_block(p, dist.data() + (size_t)C_BlockVer_offset[p] * n);
+          copied = p;
+          if (path_needed) copy_path_block(p, path.data() + (size_t)C_BlockVer_offset[p] * n);
+        }
+      }
+    } else {
+      check(rc, "fap_solve");
     }
-  } else {
-    check(rc, "fap_solve");
+    if (blank.valid()) blank.get();
+  } catch (...) {
+    // no rows of an earlier solve are left behind
+    const size_t done = copied < K ? (size_t)C_BlockVer_offset[copied + 1] * n : dist.size();
+    std::fill(dist.begin() + done, dist.end(), 0.0f);
+    throw;
   }
-  if (blank.valid()) blank.get();
   path_ready_ = path_needed;
   return 0;
 }
