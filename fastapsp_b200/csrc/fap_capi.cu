@@ -828,14 +828,15 @@ int build_elim(fap_dgraph *G) {
 // takes it where elimination closes the whole boundary graph too, and dB
 // needs no more memory than the SSSP scratch rows it replaces, or 4 MB (the
 // server admits such batches by that size).  One part of a 50,001-vertex road
-// graph: 0.17 ms instead of 4.6.
+// graph: 0.17 ms instead of 4.6.  (Its rows are written by one grid row per
+// part of the graph, which a batch of few of very many parts does not fit.)
 constexpr int64_t kElimBatchElems = int64_t(1) << 20;
 bool elim_ok(const fap_dgraph *G, int64_t sources) {
   if (!G->eliminate || !G->el_sym || G->stage1 == 1 || G->bgraph_form != 0 ||
       !G->floyd_queue || !G->floyd_sym || G->floyd_per_cta || G->total_b > kBgraphFloydMax)
     return false;
   const int64_t ldB = round_up(G->total_b, kFloydTile);
-  return sources < 0 || (G->el2.plan.ok && ldB * ldB <= std::max<int64_t>(sources * G->n, kElimBatchElems));
+  return sources < 0 || (G->el2.plan.ok && G->K <= kMaxGridY && ldB * ldB <= std::max<int64_t>(sources * G->n, kElimBatchElems));
 }
 
 // Words of dB, with the work space of its Floyd closure after it from 1,024

@@ -35,3 +35,35 @@ def test_float_weights_beyond_the_sentinel(cuda_ok, directed):
     assert any((b > 1e8).any() for b in out[0])
     for p, (a, b) in enumerate(zip(*out), 1):
         assert np.array_equal(a.view(np.int32), b.view(np.int32)), f"part {p}"
+
+
+def test_some_of_more_parts_than_a_grid_has_rows(cuda_ok):
+    """66,001 parts: a batch of a few of them (a path through four parts of two
+    vertices, the other vertices alone)."""
+    K, n = 66001, 66005
+    gid = np.concatenate([np.repeat(np.arange(1, 5), 2), np.arange(5, K + 1)]).astype(np.int32)
+    path = np.arange(8)
+    edges = np.stack([path[:-1], path[1:]], 1)
+    el = G.EdgeList(n, np.concatenate([edges, edges[:, ::-1]]), np.full(14, 3.0, np.float32), directed=True,
+                    weighted=True, integral=True)
+    ro, col, w = G.edges_to_csr(el)
+    vn = np.zeros(K + 1, np.int32)
+    vn[1:] = np.bincount(gid)[1:]
+    bn = np.zeros(K + 1, np.int32)
+    bn[1:5] = [1, 2, 2, 1]
+    vo = np.concatenate([[0, 0], np.cumsum(vn[1:-1])]).astype(np.int32)
+    st2ed = np.arange(n, dtype=np.int32)
+    st2ed[:2] = [1, 0]                       # part 1: its boundary vertex first
+    dg = DeviceGraph(Context(0), ro, col, w)
+    dg.set_parts(K, gid, st2ed, vn, vo, bn)
+    dg.reserve(64)
+    some = [3, 1, 4, 700]
+    dg.solve(some, FAP_MODE_BATCHED)
+    for p in some:
+        b = dg.copy_block(p)
+        for r, v in enumerate(st2ed[vo[p]:vo[p] + vn[p]]):
+            want = np.full(n, 100000000)
+            want[v] = 0
+            if v < 8:
+                want[:8] = 3 * np.abs(path - v)
+            assert np.array_equal(b[r], want), (p, r)
