@@ -36,7 +36,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hi
 SOURCES = ["fap_device.cu", "fap_capi.cu", "fap_elim.cu", "fap_elim.cpp", "fap_floyd64.cu", "fap_legacy.cu", "fap_noalloc.cu", "fap_host.cpp",
            "fap_serve.cpp"]
 HEADERS = ["fap_common.cuh", "minplus_tile.cuh", "floyd.cuh", "sssp.cuh", "tma.cuh", "tma_tile.cuh",
-           "fap_internal.h", "fap_elim.h"]
+           "fap_internal.h", "fap_elim.h", "floyd64_tiles.h"]
 
 
 def _stale(target: str, deps: list[str]) -> bool:

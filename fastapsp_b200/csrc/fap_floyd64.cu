@@ -17,6 +17,7 @@
 
 #include "fap_common.cuh"
 #include "fap_internal.h"
+#include "floyd64_tiles.h"
 #include "minplus_tile.cuh"
 
 namespace fapb {
@@ -173,12 +174,13 @@ __global__ void __launch_bounds__(kThreads) floyd64_panel_kernel(T *mat, int64_t
   if (SYM) store_transposed<T, 4>(acc, 0, tile, mat + (int64_t)t * kB * ld + (int64_t)kb * kB, ld);
 }
 
-// Remainder tiles (i0, jx) and, with ni = 2, (i0 + 1, jx) of pivot block kb,
-// counted without the `skip` rows and columns from kb on.  SYM: only row tiles
-// up to the column tile, each also stored transposed.
+// Remainder tiles (i0, jx) and (i0 + 1, jx) of pivot block kb, as far as they
+// are this CTA's (floyd64_pair_rows), of nr rows and columns counted without the
+// `skip` ones from kb on.  SYM: each is also stored transposed.
 template <typename T, bool SYM>
-__device__ __forceinline__ void rest_tiles(T *mat, int64_t ld, int kb, int jx, int i0, int ni, int skip, T *A, T *B) {
-  if (SYM && i0 > jx) return;
+__device__ __forceinline__ void rest_tiles(T *mat, int64_t ld, int kb, int jx, int i0, int nr, int skip, T *A, T *B) {
+  const int ni = floyd64_pair_rows(SYM, jx, i0, nr);
+  if (ni == 0) return;
   const int j = jx + (jx >= kb ? skip : 0);
   const int ia = i0 + (i0 >= kb ? skip : 0), ib = ni > 1 ? i0 + 1 + (i0 + 1 >= kb ? skip : 0) : ia;
   const T *R = mat + (int64_t)kb * kB * ld + (int64_t)j * kB;
@@ -202,7 +204,7 @@ __device__ __forceinline__ void rest_tiles(T *mat, int64_t ld, int kb, int jx, i
       store_row((i < 4 ? Ca + (ty + 16 * i) * ld : Cb + (ty + 16 * (i - 4)) * ld) + 4 * tx, acc[i]);
   if (SYM) {
     if (ia != j) store_transposed<T, 8>(acc, 0, A, mat + (int64_t)j * kB * ld + (int64_t)ia * kB, ld);
-    if (ni > 1 && i0 + 1 < jx) store_transposed<T, 8>(acc, 4, A, mat + (int64_t)j * kB * ld + (int64_t)ib * kB, ld);
+    if (ni > 1 && ib != j) store_transposed<T, 8>(acc, 4, A, mat + (int64_t)j * kB * ld + (int64_t)ib * kB, ld);
   }
 }
 
@@ -229,8 +231,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) floyd64_rest_kernel(T *mat, in
     for (int i = 0; i < 4; i++) store_row(D + (ty + 16 * i) * ld + 4 * tx, acc[i]);
     return;
   }
-  const int i0 = 2 * blockIdx.y;
-  rest_tiles<T, SYM>(mat, ld, kb, blockIdx.x, i0, min(2, nb - 1 - i0), 1, A, B);
+  rest_tiles<T, SYM>(mat, ld, kb, blockIdx.x, 2 * blockIdx.y, nb - 1, 1, A, B);
 }
 
 // Panel tile of pivot block nx (tile t of its row, or of its column) while the
@@ -330,8 +331,7 @@ __global__ void __launch_bounds__(kThreads, CTAS) floyd64_step_kernel(T *mat, in
     }
     return;
   }
-  const int jx = id % nr, i0 = 2 * (id / nr);
-  rest_tiles<T, SYM>(mat, ld, kb, jx, i0, min(2, nr - i0), skip, A, B);
+  rest_tiles<T, SYM>(mat, ld, kb, id % nr, 2 * (id / nr), nr, skip, A, B);
 }
 
 template <typename T, bool SYM>
