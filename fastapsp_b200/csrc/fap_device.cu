@@ -180,6 +180,7 @@ cudaError_t launch_gather(const PartDesc *parts, int nparts, int max_ldf, const 
                           const int32_t *st2ed, const int32_t *ed2st, const T *D, int64_t ldD,
                           T *F, cudaStream_t stream, int64_t *launches) {
   if (nparts <= 0) return cudaSuccess;
+  if (max_ldf > kFloydPartMax) return cudaErrorInvalidValue;
   size_t smem = (size_t)max_ldf * sizeof(int32_t);
   auto kern = gather_kernel<T>;
   if (smem > 48 * 1024) {
@@ -1254,7 +1255,8 @@ template <typename T>
 struct ThinShared {
   __align__(16) T As[kMinplusBM][kThinK];
   T Own[kThinOwn];
-  uint16_t own_col[kThinCols];  // (parts of more than 65,535 vertices have no Floyd matrix)
+  uint16_t own_col[kThinCols];  // part-local
+  static_assert(kFloydPartMax <= 65536, "part-local columns fit in 16 bits");
   int nown;
 };
 

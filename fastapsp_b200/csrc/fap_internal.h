@@ -178,6 +178,9 @@ cudaError_t launch_msbf(const MsbfItem *items, int nitems, const int32_t *tro, c
 // num_sources sources on this device.
 int sssp_scratch_rows(int n, int num_sources);
 
+// Side of the largest Floyd matrix of a part: launch_gather keeps a row's
+// winning arcs in a CTA's shared memory (227 KB) and refuses larger ones.
+constexpr int kFloydPartMax = 227 * 1024 / 4;
 template <typename T>
 cudaError_t launch_gather(const PartDesc *parts, int nparts, int max_ldf, const int32_t *row_offset,
                           const int32_t *col, const T *w, const int32_t *graph_id,
