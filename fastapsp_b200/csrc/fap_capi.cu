@@ -108,6 +108,15 @@ struct DevBuf {
     bytes = want;
     return FAP_OK;
   }
+  // Exactly `want` bytes, for buffers that are made once.
+  cudaError_t make(size_t want) {
+    if (want <= bytes) return cudaSuccess;
+    release();
+    const cudaError_t e = cudaMalloc(&p, want);
+    if (e == cudaSuccess) bytes = want;
+    else p = nullptr;
+    return e;
+  }
   // Stream-ordered growth for buffers used on one stream only: the old
   // buffer is freed after the stream's earlier work, and nothing waits for
   // the rest of the device (cudaFree would).  release() works on either kind.
@@ -278,65 +287,53 @@ bool queue_order_ok(const std::vector<PartDesc> &parts, bool sym, const std::vec
 // Bellman-Ford over the boundary graph (Floyd's cube grows too fast).
 constexpr int64_t kBgraphFloydMax = 8192;
 
-// Device copy of an elimination plan (fap_elim.h), one buffer made with the
-// partition.
+// An elimination plan (fap_elim.h) and its device arrays, which lie in one buffer
+// made with the partition (fap_dgraph::d_elim).
 struct ElimBuf {
   ElimPlan plan;
-  DevBuf buf;
   ElimDev dev{};
-  void release() {
-    buf.release();
-    plan = ElimPlan{};
-  }
-  int upload(bool directed) {
-    const struct { const void *p; size_t bytes; } src[] = {
-        {plan.parts.data(), plan.parts.size() * sizeof(ElimPart)},
-        {plan.loc.data(), plan.loc.size() * 4},   {plan.inv.data(), plan.inv.size() * 4},
-        {plan.eptr.data(), plan.eptr.size() * 4}, {plan.ecol.data(), plan.ecol.size() * 4},
-        {plan.eend.data(), plan.eend.size() * 4}, {plan.w0.data(), plan.w0.size() * 4},
-        {plan.w0b.data(), directed ? plan.w0b.size() * 4 : 0}, {plan.lev.data(), plan.lev.size() * 4},
-        {plan.units.data(), plan.units.size() * sizeof(ElimUnit)},
-        {plan.glev.data(), plan.glev.size() * 4}, {plan.rows8.data(), plan.rows8.size() * 4},
-        {plan.sloc.data(), plan.sloc.size() * 4}, {plan.list.data(), plan.list.size() * 2},
-        {plan.chunks.data(), plan.chunks.size() * sizeof(ElimChunk)},
-        {nullptr, plan.ecol.size() * sizeof(int2)}, {nullptr, directed ? plan.ecol.size() * 4 : 0}};
-    constexpr int N = sizeof(src) / sizeof(src[0]);
-    size_t off[N], bytes = 0;
-    for (int i = 0; i < N; i++) {
-      off[i] = bytes;
-      bytes += (src[i].bytes + 255) / 256 * 256;
-    }
-    FAP_TRY(buf.ensure(std::max<size_t>(bytes, 256)));
-    char *d = buf.as<char>();
-    for (int i = 0; i + 2 < N; i++)
-      if (src[i].bytes > 0) FAP_CK(cudaMemcpy(d + off[i], src[i].p, src[i].bytes, cudaMemcpyHostToDevice));
-    auto at = [&](int i) { return reinterpret_cast<const int32_t *>(d + off[i]); };
+  int4 *coef32 = nullptr, *coef16 = nullptr;  // the group merge's streams (ElimMerge)
+  int32_t *far = nullptr;
+  void clear() { *this = ElimBuf{}; }
+  // Lays the arrays out from byte `at` on and returns the end; with a buffer
+  // (base) also fills them and sets the pointers.
+  size_t place(char *base, size_t at, bool directed, cudaError_t *err) {
+    auto put = [&](const void *src, size_t bytes) -> char * {
+      char *d = base ? base + at : nullptr;
+      at += (bytes + 255) / 256 * 256;
+      if (base && src && bytes > 0 && *err == cudaSuccess) *err = cudaMemcpy(d, src, bytes, cudaMemcpyHostToDevice);
+      return d;
+    };
+    auto ints = [&](const std::vector<int32_t> &v) { return reinterpret_cast<const int32_t *>(put(v.data(), v.size() * 4)); };
     dev = ElimDev{};
-    dev.parts = reinterpret_cast<const ElimPart *>(d);
-    dev.loc = at(1);
-    dev.inv = at(2);
-    dev.eptr = at(3);
-    dev.ecol = at(4);
-    dev.eend = at(5);
-    dev.w0 = at(6);
-    dev.w0b = directed ? at(7) : nullptr;
-    dev.lev = at(8);
-    dev.units = reinterpret_cast<const ElimUnit *>(d + off[9]);
-    dev.glev = at(10);
-    dev.rows8 = at(11);
-    dev.sloc = at(12);
-    dev.list = reinterpret_cast<const uint16_t *>(d + off[13]);
-    dev.chunks = reinterpret_cast<const ElimChunk *>(d + off[14]);
-    dev.ent = reinterpret_cast<int2 *>(d + off[15]);
-    dev.entb = directed ? reinterpret_cast<int32_t *>(d + off[16]) : nullptr;
+    dev.parts = reinterpret_cast<const ElimPart *>(put(plan.parts.data(), plan.parts.size() * sizeof(ElimPart)));
+    dev.loc = ints(plan.loc);
+    dev.inv = ints(plan.inv);
+    dev.eptr = ints(plan.eptr);
+    dev.ecol = ints(plan.ecol);
+    dev.eend = ints(plan.eend);
+    dev.w0 = ints(plan.w0);
+    dev.w0b = directed ? ints(plan.w0b) : nullptr;
+    dev.lev = ints(plan.lev);
+    dev.units = reinterpret_cast<const ElimUnit *>(put(plan.units.data(), plan.units.size() * sizeof(ElimUnit)));
+    dev.glev = ints(plan.glev);
+    dev.rows8 = ints(plan.rows8);
+    dev.sloc = ints(plan.sloc);
+    dev.list = reinterpret_cast<const uint16_t *>(put(plan.list.data(), plan.list.size() * 2));
+    dev.chunks = reinterpret_cast<const ElimChunk *>(put(plan.chunks.data(), plan.chunks.size() * sizeof(ElimChunk)));
+    dev.ent = reinterpret_cast<int2 *>(put(nullptr, plan.ecol.size() * sizeof(int2)));
+    dev.entb = directed ? reinterpret_cast<int32_t *>(put(nullptr, plan.ecol.size() * 4)) : nullptr;
     dev.nparts = (int32_t)plan.parts.size();
     dev.max_s = plan.max_s;
-    dev.max_b = plan.max_b;
     dev.max_nent = plan.max_nent;
     dev.max_nlev = plan.max_nlev;
     dev.max_chunk16 = plan.max_chunk16;
     dev.max_chunks = plan.max_chunks;
-    return FAP_OK;
+    const size_t stream = plan.stream16 > 0 ? (size_t)plan.stream16 * 16 : 0;
+    coef32 = reinterpret_cast<int4 *>(put(nullptr, stream));
+    coef16 = reinterpret_cast<int4 *>(put(nullptr, stream));
+    far = reinterpret_cast<int32_t *>(put(nullptr, stream > 0 ? plan.parts.size() * 4 : 0));
+    return at;
   }
 };
 
@@ -457,13 +454,15 @@ struct fap_dgraph {
   bool last_elim = false;  // the prepared batch uses it
   ElimBuf el, el2;
   std::vector<int32_t> barcs;
-  DevBuf d_barcs, d_elist, d_eoff;
+  const int32_t *dev_barcs = nullptr;
+  DevBuf d_elim;  // both plans, the merge's streams and barcs
+  DevBuf d_elist, d_eoff;
   // Parts of the prepared batch whose inner rows the group merge makes
-  // (plan part, batch index), and its coefficients (ElimMerge).
+  // (plan part, batch index).
   std::vector<int2> merge;
   bool last_merge = false, last_given = false;
   int32_t merge_units = 0, merge_slots = 0;
-  DevBuf d_merge, d_coef32, d_coef16, d_far;
+  DevBuf d_merge;
   std::vector<int32_t> boff;
   std::vector<int32_t> bpcol;  // boundary columns of dB padded per part to multiples of 4 (prefix sums)
   bool last_bmethod = false;   // the prepared batch uses it
@@ -725,18 +724,14 @@ constexpr int64_t kElimGraphEntries = 24576;
 // (el_sym: every arc has its reverse with the same weight, no duplicate arcs
 // inside a part) of the boundary graph.  Host work of some milliseconds on up
 // to 16 threads.
-int build_elim(fap_dgraph *G) {
-  G->el.release();
-  G->el2.release();
-  G->barcs.clear();
-  G->el_sym = false;
-  if (G->total_b <= 0) return FAP_OK;
+void plan_elim(fap_dgraph *G) {
+  if (G->total_b <= 0) return;
   const bool i32 = G->dtype == FAP_DTYPE_I32;
   // A float32 arc heavier than the sentinel keeps its weight in a closure
   // where no path is shorter; the sweeps start from the sentinel and would lose it.
   if (!i32)
     for (const uint32_t bits : G->h_w)
-      if (bits > kInfBitsF32) return FAP_OK;  // (weights are finite and at least 0; -0.0 is left to the general path too)
+      if (bits > kInfBitsF32) return;  // (weights are finite and at least 0; -0.0 is left to the general path too)
   const int32_t inf = i32 ? kInfI32 : (int32_t)kInfBitsF32;
   const int threads = std::min(16, (int)std::thread::hardware_concurrency());
   const int32_t K = (int32_t)G->vnum.size() - 1;
@@ -765,16 +760,10 @@ int build_elim(fap_dgraph *G) {
     }
   };
   elim_build(K, part_graph, threads, inf, i32, &G->el.plan);
-  if (!G->el.plan.ok) return FAP_OK;
+  if (!G->el.plan.ok) return;
   // (float32 parts keep min-plus over the boundary, which distance rows from
-  // the resident cache match bit for bit; their symmetry is sym_local's)
-  FAP_TRY(G->el.upload(!G->sym_local));
-  if (G->el.plan.stream16 > 0) {  // (with the plan, so that a server counts them as held)
-    FAP_TRY(G->d_coef32.ensure((size_t)G->el.plan.stream16 * 16));
-    FAP_TRY(G->d_coef16.ensure((size_t)G->el.plan.stream16 * 16));
-    FAP_TRY(G->d_far.ensure(G->el.plan.parts.size() * 4));
-  }
-  if (!i32 || !G->sym_local) return FAP_OK;
+  // the resident cache match bit for bit)
+  if (!i32 || !G->sym_local) return;
   std::vector<std::array<int32_t, 3>> cross;
   for (int32_t p = 1; p <= K; p++)
     for (int32_t i = 0; i < G->bnum[p]; i++) {
@@ -794,15 +783,12 @@ int build_elim(fap_dgraph *G) {
               cross.end());
   for (const auto &a : cross) {
     const auto it = std::lower_bound(cross.begin(), cross.end(), std::array<int32_t, 3>{a[1], a[0], 0});
-    if (it == cross.end() || (*it)[0] != a[1] || (*it)[1] != a[0] || (*it)[2] != a[2]) return FAP_OK;
+    if (it == cross.end() || (*it)[0] != a[1] || (*it)[1] != a[0] || (*it)[2] != a[2]) return;
   }
   for (const auto &a : cross) G->barcs.insert(G->barcs.end(), a.begin(), a.end());
-  if (G->barcs.size() > (size_t)INT32_MAX) return FAP_OK;
+  if (G->barcs.size() > (size_t)INT32_MAX) return;
   G->el_sym = true;
-  FAP_TRY(G->d_barcs.ensure(std::max<size_t>(G->barcs.size(), 4) * 4));
-  if (!G->barcs.empty())
-    FAP_CK(cudaMemcpy(G->d_barcs.p, G->barcs.data(), G->barcs.size() * 4, cudaMemcpyHostToDevice));
-  if (G->total_b > kElimGraphMax) return FAP_OK;
+  if (G->total_b > kElimGraphMax) return;
   auto boundary_graph = [&](int, ElimGraph *g) {
     g->s = (int32_t)G->total_b;
     g->ptr.push_back(0);
@@ -817,9 +803,42 @@ int build_elim(fap_dgraph *G) {
   };
   elim_build(1, boundary_graph, 1, inf, false, &G->el2.plan);
   if (G->el2.plan.nent > kElimGraphEntries) G->el2.plan = ElimPlan{};
-  if (!G->el2.plan.ok) return FAP_OK;
-  elim_offsets(round_up(G->total_b, kFloydTile), &G->el2.plan);
-  return G->el2.upload(false);
+  if (G->el2.plan.ok) elim_offsets(round_up(G->total_b, kFloydTile), &G->el2.plan);
+}
+
+// The plans and their device arrays, made with the partition (a server then
+// counts them as held).  Without memory for them the graph has no plans and
+// takes the general path.
+int build_elim(fap_dgraph *G) {
+  G->el.clear();
+  G->el2.clear();
+  G->barcs.clear();
+  G->dev_barcs = nullptr;
+  G->el_sym = false;
+  plan_elim(G);
+  if (!G->el.plan.ok) return FAP_OK;
+  const bool directed = !G->sym_local;  // (el2 is symmetric)
+  cudaError_t e = cudaSuccess;
+  const size_t at2 = G->el.place(nullptr, 0, directed, &e), at3 = G->el2.place(nullptr, at2, false, &e);
+  FAP_CK(cudaStreamSynchronize(G->ctx->stream));  // (solves of an earlier partition may still read its plans)
+  e = G->d_elim.make(at3 + G->barcs.size() * 4);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    G->el.clear();
+    G->el2.clear();
+    G->barcs.clear();
+    G->el_sym = false;
+    return FAP_OK;
+  }
+  FAP_CK(e);
+  char *base = G->d_elim.as<char>();
+  G->el.place(base, 0, directed, &e);
+  G->el2.place(base, at2, false, &e);
+  if (e == cudaSuccess && !G->barcs.empty())
+    e = cudaMemcpy(base + at3, G->barcs.data(), G->barcs.size() * 4, cudaMemcpyHostToDevice);
+  FAP_CK(e);
+  G->dev_barcs = reinterpret_cast<const int32_t *>(base + at3);
+  return FAP_OK;
 }
 
 // Whether solves close the boundary graph and the parts by elimination:
@@ -861,9 +880,7 @@ extern "C" int fap_graph_destroy(fap_dgraph *G) try {
     DeviceGuard g(c->device);
     cudaStreamSynchronize(c->stream);
     if (G->gexec) cudaGraphExecDestroy(G->gexec);
-    G->el.release();
-    G->el2.release();
-    for (DevBuf *b : {&G->d_barcs, &G->d_elist, &G->d_eoff, &G->d_merge, &G->d_coef32, &G->d_coef16, &G->d_far, &G->ro, &G->col, &G->w, &G->ro_s, &G->col_s, &G->w_s, &G->sssp_scratch, &G->d_thin,
+    for (DevBuf *b : {&G->d_elim, &G->d_elist, &G->d_eoff, &G->d_merge, &G->ro, &G->col, &G->w, &G->ro_s, &G->col_s, &G->w_s, &G->sssp_scratch, &G->d_thin,
                       &G->d_gid, &G->d_st2ed, &G->d_ed2st, &G->D, &G->F, &G->d_parts, &G->d_work,
                       &G->d_src, &G->d_srcrows, &G->d_status, &G->d_checks, &G->staging, &G->P,
                       &G->d_tro, &G->d_tcol, &G->d_tw, &G->d_dB, &G->d_bpart, &G->d_brows, &G->d_FB,
@@ -999,7 +1016,6 @@ extern "C" int fap_graph_set_parts(fap_dgraph *G, int32_t K, const int32_t *grap
       G->sym_local = sym;
     }
   }
-  FAP_TRY(build_elim(G));
   {
     // edges of the boundary graph
     int64_t cross = 0;
@@ -1013,6 +1029,7 @@ extern "C" int fap_graph_set_parts(fap_dgraph *G, int32_t K, const int32_t *grap
   G->row_base.assign(K + 1, -1);
   G->last_ids.clear();
   cache_drop(G);
+  FAP_TRY(build_elim(G));
   FAP_TRY(G->d_gid.ensure((size_t)n * 4));
   FAP_TRY(G->d_st2ed.ensure((size_t)n * 4));
   FAP_TRY(G->d_ed2st.ensure((size_t)n * 4));
@@ -1388,7 +1405,7 @@ int run_elim(fap_dgraph *G, const PartDesc *dp, int count, int max_s, int32_t *F
   int nrows = 0;
   if (!all)
     for (const PartDesc &d : G->parts) nrows += d.b;
-  FAP_CK(launch_elim_seed(dB, G->ldB, nb, G->el2.plan.ok ? nb : (int)G->ldB, G->d_barcs.as<const int32_t>(),
+  FAP_CK(launch_elim_seed(dB, G->ldB, nb, G->el2.plan.ok ? nb : (int)G->ldB, G->dev_barcs,
                           (int)(G->barcs.size() / 3), st, L));
   FAP_CK(launch_elim_up<int32_t>(G->el.dev, nullptr, 0, nullptr, dB, G->ldB, st, L));
   FAP_CK(record_event(ev1, st));
@@ -1425,8 +1442,7 @@ bool merge_ok(const fap_dgraph *G, int32_t p) {
 int run_merge(fap_dgraph *G, const PartDesc *dp, const int32_t *F, int64_t *L) {
   if (G->merge.empty()) return FAP_OK;
   cudaStream_t st = G->ctx->stream;
-  const ElimMerge m{G->d_merge.as<const int2>(), (int32_t)G->merge.size(), G->d_coef32.as<int4>(),
-                    G->d_coef16.as<int4>(), G->d_far.as<int32_t>(),
+  const ElimMerge m{G->d_merge.as<const int2>(), (int32_t)G->merge.size(), G->el.coef32, G->el.coef16, G->el.far,
                     G->pack16 ? G->d_pk_tiles.as<unsigned long long>() : nullptr};
   FAP_CK(launch_elim_coef(G->el.dev, m, dp, F, G->merge_units, st, L));
   FAP_CK(launch_elim_merge(G->el.dev, m, dp, F, G->n, G->D.as<int32_t>(), G->ldD, G->d_gid.as<const int32_t>(),
@@ -2804,10 +2820,8 @@ extern "C" int fap_graph_device_bytes(const fap_dgraph *G, int64_t *bytes) try {
                           &G->d_bDt, &G->d_bact, &G->d_bpact, &G->d_bgpart, &G->d_bpcolmap, &G->d_grow,
                           &G->d_bTc, &G->d_pk_off, &G->d_pk_range, &G->d_pk_maxa, &G->d_pk_tiles, &G->d_pk_s16,
                           &G->d_pk_at, &G->d_pk_krow, &G->d_xk_off, &G->d_xk_range, &G->d_xk_maxb, &G->d_xk_tiles,
-                          &G->d_xk_ap, &G->d_xk_bd, &G->d_barcs, &G->d_elist, &G->d_eoff, &G->d_merge, &G->d_coef32, &G->d_coef16,
-                          &G->d_far})
+                          &G->d_xk_ap, &G->d_xk_bd, &G->d_elim, &G->d_elist, &G->d_eoff, &G->d_merge})
     t += (int64_t)b->bytes;
-  t += (int64_t)(G->el.buf.bytes + G->el2.buf.bytes);
   *bytes = t;
   return FAP_OK;
 } catch (...) {

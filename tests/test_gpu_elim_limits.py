@@ -67,3 +67,53 @@ def test_some_of_more_parts_than_a_grid_has_rows(cuda_ok):
             if v < 8:
                 want[:8] = 3 * np.abs(path - v)
             assert np.array_equal(b[r], want), (p, r)
+
+
+def test_no_memory_for_the_plans(cuda_ok):
+    """A partition is accepted when the device has no room for the elimination's
+    plans (tens of MB for this graph): the graph then takes the general path."""
+    import torch
+    el = G.grid_graph(224, 224, extra_frac=0.01, wmin=1, wmax=100, seed=42)
+    ro, col, w = G.edges_to_csr(el)
+    K = 48
+    fg = fapGraph.from_csr(el.n, int(ro[-1]), ro, col, w, K, directed=el.directed)
+    fg.preCondition()
+    vn, vo, bn = fg.partInfo()
+    parts = (K, fg.getGraphId(), fg.getMapping(), vn, vo, bn)
+    dg = DeviceGraph(Context(0), ro, col, w)
+    before = dg.device_bytes()
+    dg.set_parts(*parts)
+    plans = dg.device_bytes() - before
+    assert plans > 30 << 20                  # (more than what is left below)
+    del dg
+    dg = DeviceGraph(Context(0), ro, col, w)
+    torch.cuda.empty_cache()
+    held = []
+
+    def free():
+        return torch.cuda.mem_get_info()[0]
+
+    try:
+        size = free() - (20 << 20)
+        while free() > 24 << 20 and size > 10 << 20:    # all but 20 MB of the device
+            try:
+                held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                size //= 2
+            size = min(size, free() - (20 << 20))
+        if not 8 << 20 < free() <= 24 << 20:
+            pytest.skip(f"{free()} bytes of the device left")
+        dg.set_parts(*parts)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    dg.reserve(int(vn[1:4].sum()))
+    some = [1, 2, 3]
+    dg.solve(some, FAP_MODE_BATCHED)
+    assert "elimination" not in dg.stage1_name()
+    got = [dg.copy_block(p) for p in some]
+    dg.set_parts(*parts)                     # now there is room
+    dg.reserve(int(vn[1:4].sum()))
+    dg.solve(some, FAP_MODE_BATCHED)
+    for a, p in zip(got, some):
+        assert np.array_equal(a, dg.copy_block(p)), p
