@@ -103,6 +103,8 @@ _SIGS = {
     "fap_graph_cache_timing": (INT, [P, P]),
     "fap_graph_cache_release": (INT, [P]),
     "fap_graph_cache_bytes": (INT, [P, ctypes.POINTER(I64), ctypes.POINTER(INT)]),
+    "fap_graph_batch_bytes": (INT, [P, P, I32, I64, I64, ctypes.POINTER(I64)]),
+    "fap_graph_rows_bytes": (INT, [P, I32, ctypes.POINTER(I64)]),
     "fap_server_create": (INT, [INT, DBL, I64, PP]),
     "fap_server_destroy": (INT, [P]),
     "fap_server_add_graph": (INT, [P, I32, I64, P, P, P, INT, I32, P, P, P, P, P, ctypes.POINTER(I32)]),

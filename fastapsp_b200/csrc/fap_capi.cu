@@ -108,14 +108,18 @@ struct DevBuf {
     bytes = want;
     return FAP_OK;
   }
-  // Exactly `want` bytes, for buffers that are made once.
-  cudaError_t make(size_t want) {
-    if (want <= bytes) return cudaSuccess;
+  // Exactly `want` bytes, for large buffers of one use (blocks, plans).
+  int ensure_exact(size_t want) {
+    if (want <= bytes) return FAP_OK;
     release();
     const cudaError_t e = cudaMalloc(&p, want);
-    if (e == cudaSuccess) bytes = want;
-    else p = nullptr;
-    return e;
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+      return fail(FAP_ERR_NOMEM, "cudaMalloc(%zu bytes): %s", want, cudaGetErrorString(e));
+    }
+    bytes = want;
+    return FAP_OK;
   }
   // Stream-ordered growth for buffers used on one stream only: the old
   // buffer is freed after the stream's earlier work, and nothing waits for
@@ -821,16 +825,13 @@ int build_elim(fap_dgraph *G) {
   cudaError_t e = cudaSuccess;
   const size_t at2 = G->el.place(nullptr, 0, directed, &e), at3 = G->el2.place(nullptr, at2, false, &e);
   FAP_CK(cudaStreamSynchronize(G->ctx->stream));  // (solves of an earlier partition may still read its plans)
-  e = G->d_elim.make(at3 + G->barcs.size() * 4);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
+  if (G->d_elim.ensure_exact(at3 + G->barcs.size() * 4) != FAP_OK) {
     G->el.clear();
     G->el2.clear();
     G->barcs.clear();
     G->el_sym = false;
     return FAP_OK;
   }
-  FAP_CK(e);
   char *base = G->d_elim.as<char>();
   G->el.place(base, 0, directed, &e);
   G->el2.place(base, at2, false, &e);
@@ -1081,11 +1082,11 @@ extern "C" int fap_graph_reserve(fap_dgraph *G, int64_t max_rows) try {
   G->epoch++;
   if (G->D.bytes < bytes) {
     G->D.release();
-    FAP_TRY(G->D.ensure(bytes));
+    FAP_TRY(G->D.ensure_exact(bytes));
   }
   if (G->paths && G->P.bytes < bytes) {
     G->P.release();
-    FAP_TRY(G->P.ensure(bytes));
+    FAP_TRY(G->P.ensure_exact(bytes));
   }
   G->max_rows = max_rows;
   return FAP_OK;
@@ -1349,13 +1350,24 @@ int expand_bgraph(fap_dgraph *G, const PartDesc *dp, int np, int max_s, const T 
 }
 
 // Device state of the elimination form for the listed parts (row_base and
-// f_off final): the plans, dB, the parts to close and, for a batch of some of
-// the parts, the boundary rows to write.  given: for run_elim_given only.
-int prepare_elim(fap_dgraph *G, const std::vector<PartDesc> &parts, bool given = false) {
-  if (!given) {
-    G->ldB = round_up(std::max<int64_t>(G->total_b, 1), kFloydTile);
-    FAP_TRY(G->d_dB.ensure((size_t)bgraph_words(G->ldB) * 4));
-  }
+// f_off final): the parts to close and, for a batch of some of the parts
+// (some), dB and the boundary rows to write, which prepare_bgraph makes for
+// all of them.  grow_elim makes room in stream order (a cudaFree would wait for
+// every stream of a server); the stream has to be waited for before fill_elim
+// copies.
+int grow_elim(fap_dgraph *G, const std::vector<PartDesc> &parts, bool some) {
+  cudaStream_t st = G->ctx->stream;
+  FAP_TRY(G->d_elist.ensure_async(parts.size() * 4, st));
+  FAP_TRY(G->d_eoff.ensure_async((parts.size() + 1) * 8, st));
+  if (!some) return FAP_OK;
+  int64_t nrows = 0;
+  for (const PartDesc &d : parts) nrows += d.b;
+  G->ldB = round_up(std::max<int64_t>(G->total_b, 1), kFloydTile);
+  FAP_TRY(G->d_dB.ensure_async((size_t)bgraph_words(G->ldB) * 4, st));
+  return G->d_brows.ensure_async((size_t)std::max<int64_t>(2 * nrows, 2) * 8, st);
+}
+
+int fill_elim(fap_dgraph *G, const std::vector<PartDesc> &parts, bool some) {
   std::vector<int32_t> list;
   std::vector<int64_t> off{0}, rows;  // (the first offset is the boundary graph's own)
   for (const PartDesc &d : parts) {
@@ -1366,17 +1378,10 @@ int prepare_elim(fap_dgraph *G, const std::vector<PartDesc> &parts, bool given =
       rows.push_back(d.row_base + k);
     }
   }
-  FAP_TRY(G->d_elist.ensure(list.size() * 4));
-  FAP_TRY(G->d_eoff.ensure(off.size() * 8));
-  if (given) {
-    FAP_CK(cudaMemcpy(G->d_elist.p, list.data(), list.size() * 4, cudaMemcpyHostToDevice));
-    FAP_CK(cudaMemcpy(G->d_eoff.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice));
-    return FAP_OK;
-  }
-  FAP_TRY(G->d_brows.ensure(std::max<size_t>(rows.size(), 2) * 8));
   FAP_CK(cudaMemcpy(G->d_elist.p, list.data(), list.size() * 4, cudaMemcpyHostToDevice));
   FAP_CK(cudaMemcpy(G->d_eoff.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice));
-  if (!rows.empty()) FAP_CK(cudaMemcpy(G->d_brows.p, rows.data(), rows.size() * 8, cudaMemcpyHostToDevice));
+  if (some && !rows.empty())
+    FAP_CK(cudaMemcpy(G->d_brows.p, rows.data(), rows.size() * 8, cudaMemcpyHostToDevice));
   return FAP_OK;
 }
 
@@ -1621,10 +1626,12 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
     FAP_TRY(G->q.items.ensure_async(std::max<size_t>(qitems.size(), 1) * sizeof(QItem), st));
     FAP_TRY(G->q.cnt.ensure_async(((size_t)G->q.nparts * G->q.stride + 2) * 4, st));
   }
+  const bool some = elim && (int32_t)ids.size() < G->K;
+  if (elim || given) FAP_TRY(grow_elim(G, G->parts, some));
   FAP_CK(cudaStreamSynchronize(st));
   if (!qitems.empty())
     FAP_CK(cudaMemcpy(G->q.items.p, qitems.data(), qitems.size() * sizeof(QItem), cudaMemcpyHostToDevice));
-  if (elim || given) FAP_TRY(prepare_elim(G, G->parts, given));
+  if (elim || given) FAP_TRY(fill_elim(G, G->parts, some));
   if (bmethod && (int32_t)ids.size() == G->K) FAP_TRY(prepare_bgraph(G, G->parts, true));
   FAP_CK(cudaMemcpy(G->d_parts.p, G->parts.data(), G->parts.size() * sizeof(PartDesc), cudaMemcpyHostToDevice));
   if (!G->work.empty())
@@ -1941,7 +1948,7 @@ extern "C" int fap_solve(fap_dgraph *G, const int32_t *parts, int32_t count, int
   if (G->paths && G->P.bytes < (size_t)G->max_rows * G->ldD * 4) {
     FAP_CK(cudaStreamSynchronize(G->ctx->stream));
     G->P.release();
-    FAP_TRY(G->P.ensure((size_t)G->max_rows * G->ldD * 4));
+    FAP_TRY(G->P.ensure_exact((size_t)G->max_rows * G->ldD * 4));
     G->epoch++;
   }
   const bool cached = mode == FAP_MODE_BATCHED && G->cache_ready && G->use_cache;
@@ -2104,7 +2111,7 @@ extern "C" int fap_graph_copy_block(fap_dgraph *G, int32_t part, void *host, int
     FAP_CK(cudaMemcpy2DAsync(host, (size_t)n * 4, dp, (size_t)ld * 4, (size_t)n * 4, (size_t)rows,
                              cudaMemcpyDeviceToHost, st));
   } else if (G->dtype == FAP_DTYPE_I32 && out_dtype == FAP_DTYPE_F32) {
-    FAP_TRY(G->staging.ensure((size_t)rows * n * 4));
+    FAP_TRY(G->staging.ensure_exact((size_t)rows * n * 4));
     int64_t L = 0;
     FAP_CK(launch_i32_to_f32(reinterpret_cast<const int32_t *>(dp), rows, n, ld,
                              G->staging.as<float>(), st, &L));
@@ -2156,7 +2163,7 @@ extern "C" int fap_graph_copy_block_async(fap_dgraph *G, int32_t part, void *hos
   if (cs.staging.bytes < (size_t)rows * n * 4) {
     int32_t most = 0;
     for (int32_t q = 1; q <= G->K; q++) most = std::max(most, G->vnum[q]);
-    FAP_TRY(cs.staging.ensure((size_t)std::max<int64_t>(most, rows) * n * 4));
+    FAP_TRY(cs.staging.ensure_exact((size_t)std::max<int64_t>(most, rows) * n * 4));
   }
   int64_t L = 0;
   // the conversion on the context stream (after the solve that made the
@@ -2828,6 +2835,132 @@ extern "C" int fap_graph_device_bytes(const fap_dgraph *G, int64_t *bytes) try {
   return fail_exception();
 }
 
+namespace {
+// Bytes that ensure(want) or ensure_exact(want) adds to a buffer.
+int64_t grown_by(const DevBuf &b, int64_t want) {
+  return want <= (int64_t)b.bytes ? 0 : (int64_t)alloc_size((size_t)want) - (int64_t)b.bytes;
+}
+int64_t growth_exact(const DevBuf &b, int64_t want) { return std::max<int64_t>(0, want - (int64_t)b.bytes); }
+
+// What prepare_bgraph and expand_bgraph allocate for all parts, whose Floyd
+// matrices have sides of ldf (fresh: as if nothing were held yet).
+int64_t bgraph_growth(const fap_dgraph *G, int64_t ldf, bool col_table, bool fresh) {
+  auto growth = [fresh](const DevBuf &b, int64_t want) {
+    return fresh ? (int64_t)alloc_size((size_t)want) : grown_by(b, want);
+  };
+  const int64_t tb = std::max<int64_t>(G->total_b, 1), K = G->K;
+  const bool bf = bgraph_bf(G);
+  const int64_t ldB = round_up(std::max<int64_t>(bf ? G->bpcol[K + 1] : G->total_b, 1), kFloydTile);
+  int64_t t = growth(G->d_dB, bgraph_words(ldB) * 4) + growth(G->d_FB, tb * ldf * 4) +
+              growth(G->d_bpart, (K + 1) * (int64_t)sizeof(BPart)) + growth(G->d_brows, std::max<int64_t>(2 * G->total_b, 2) * 8);
+  int32_t max_b = 0;
+  for (int32_t p = 1; p <= K; p++) max_b = std::max(max_b, G->bnum[p]);
+  if (bgraph_tiled_expand(G)) t += growth(G->d_grow, G->total_b * 8);
+  else if (col_table && !bf && (size_t)max_b * G->ldD * 4 <= kColTableBytes) t += growth(G->d_bTc, max_b * G->ldD * 4);
+  if (!bf) return t;
+  // cross-arc CSRs, work lists, tiles, stamps, part table
+  const int64_t xe = std::max<int64_t>(G->bgraph_cross, 1), z = bgraph_ztiles(G);
+  t += growth(G->d_bitro, (tb + 1) * 4) + growth(G->d_botro, (tb + 1) * 4) + growth(G->d_bgpart, tb * 4) +
+       growth(G->d_bpcolmap, tb * 4) + growth(G->d_bitcol, xe * 4) + growth(G->d_bitw, xe * 4) +
+       growth(G->d_botcol, xe * 4) + growth(G->d_bDt, z * tb * kMsbfS * 4) + growth(G->d_bact, 3 * z * tb * 4) +
+       growth(G->d_bpact, z * (K + 1) * 4) + growth(G->d_bitems, 2 * z * tb * 4 + 4 * (int64_t)sizeof(int)) +
+       growth(G->d_msbf_changed, 4 * (int64_t)sizeof(int));
+  if (G->pack16 && G->dtype == FAP_DTYPE_I32) {
+    t += growth(G->d_xk_off, K * tb * 4) + growth(G->d_xk_range, K * ceil_div(tb, 128) * 4) + growth(G->d_xk_maxb, K * 4) +
+         growth(G->d_xk_tiles, 16);
+    const int64_t ap = tb * round_up(ceil_div(tb, 2), 4) * 4, bd = tb * ldf * 4;
+    if (G->prepack && ap + bd <= (int64_t)kPrepackBytes) t += growth(G->d_xk_ap, ap) + growth(G->d_xk_bd, bd);
+  }
+  return t;
+}
+
+// What run_stage1_sssp allocates for `count` sources (the frontier's scratch
+// whatever the form when `frontier`).
+int64_t sssp_growth(const fap_dgraph *G, int64_t count, bool frontier) {
+  const int cnt = (int)std::min<int64_t>(count, INT32_MAX);
+  int64_t scratch = 0, t = 0;
+  if (frontier || !use_msbf(G)) scratch = (int64_t)std::max(sssp_scratch_rows(G->n, cnt), 1) * G->n * 4;
+  if (use_msbf(G)) {
+    const int64_t z = msbf_ztiles(G, cnt);
+    scratch = std::max(scratch, z * G->n * kMsbfS * 4);
+    t += grown_by(G->d_msbf_act, 2 * z * ceil_div(G->n, 32) * 4) + grown_by(G->d_msbf_changed, 16) +
+         grown_by(G->d_msbf_items, (G->m / 32 + G->n + 1) * (int64_t)sizeof(MsbfItem)) +
+         grown_by(G->d_tro, (G->n + 1) * (int64_t)4) + grown_by(G->d_tcol, std::max<int64_t>(G->m, 1) * 4) +
+         grown_by(G->d_tw, std::max<int64_t>(G->m, 1) * 4);
+  }
+  return t + grown_by(G->sssp_scratch, scratch);
+}
+}  // namespace
+
+extern "C" int fap_graph_batch_bytes(const fap_dgraph *G, const int32_t *parts, int32_t count, int64_t rows,
+                                     int64_t copied_rows, int64_t *bytes) try {
+  if (!G || !bytes) return fail(FAP_ERR_INVALID, "NULL argument");
+  if (G->K == 0) return fail(FAP_ERR_STATE, "no partition");
+  const int64_t np = parts ? count : G->K, n = G->n;
+  int64_t need = 0, sources = 0, ldf = kFloydTile, work = 0;
+  for (int64_t i = 0; i < np; i++) {
+    const int32_t p = parts ? parts[i] : (int32_t)i + 1;
+    if (p < 1 || p > G->K) return fail(FAP_ERR_INVALID, "part id %d outside 1..%d", p, G->K);
+    need += G->vnum[p];
+    sources += G->bnum[p];
+    ldf = std::max<int64_t>(ldf, round_up(std::max(G->vnum[p], 1), kFloydTile));
+    work += ceil_div(G->vnum[p], kMinplusBM);
+  }
+  DeviceGuard g(G->ctx->device);
+  rows = std::min<int64_t>(std::max(rows, need), n);
+  const bool all = np == G->K, cached = G->cache_ready && G->use_cache, i32 = G->dtype == FAP_DTYPE_I32;
+  if (cached) ldf = G->cache_ldf;
+  int64_t t = growth_exact(G->D, rows * G->ldD * 4) + grown_by(G->d_parts, np * (int64_t)sizeof(PartDesc)) +
+              grown_by(G->d_work, std::max<int64_t>(work, 1) * (int64_t)sizeof(MPWork)) +
+              grown_by(G->d_thin, std::max<int64_t>(np, 1) * 4) + grown_by(G->d_src, std::max<int64_t>(sources, 1) * 4) +
+              grown_by(G->d_srcrows, std::max<int64_t>(sources, 1) * 8) + grown_by(G->d_merge, np * (int64_t)sizeof(int2));
+  if (i32) t += growth_exact(G->staging, copied_rows * n * 4);  // (int32 blocks are copied out as float32)
+  if (G->paths)
+    t += growth_exact(G->P, rows * G->ldD * 4) + grown_by(G->d_tro, (n + 1) * 4) + grown_by(G->d_tcol, std::max<int64_t>(G->m, 1) * 4) +
+         grown_by(G->d_tw, std::max<int64_t>(G->m, 1) * 4);
+  if (i32 && G->pack16) {
+    t += grown_by(G->d_pk_off, np * G->ldD * 4) + grown_by(G->d_pk_range, np * (G->ldD / kMinplusBN) * 4) +
+         grown_by(G->d_pk_maxa, np * 4) + grown_by(G->d_pk_tiles, 16);
+    const int64_t s16 = sources * G->ldD * 2, at = sources * ldf * 4;
+    if (G->prepack && s16 + at <= (int64_t)kPrepackBytes)
+      t += grown_by(G->d_pk_s16, s16) + grown_by(G->d_pk_at, at) + grown_by(G->d_pk_krow, np * 4);
+  }
+  if (!cached) {
+    t += grown_by(G->F, std::max<int64_t>(np * ldf * ldf, 1) * 4) + grown_by(G->d_elist, np * 4) + grown_by(G->d_eoff, (np + 1) * 8);
+    if (elim_ok(G, all ? -1 : sources)) {
+      if (all) {
+        t += bgraph_growth(G, ldf, true, false);
+      } else {
+        const int64_t ldB = round_up(std::max<int64_t>(G->total_b, 1), kFloydTile);
+        t += grown_by(G->d_dB, bgraph_words(ldB) * 4) + grown_by(G->d_brows, std::max<int64_t>(2 * sources, 2) * 8);
+      }
+    } else if (all && bmethod_ok(G)) {
+      t += bgraph_growth(G, ldf, true, false);
+    } else {
+      t += sssp_growth(G, sources, true);
+    }
+  }
+  *bytes = t;
+  return FAP_OK;
+} catch (...) {
+  return fail_exception();
+}
+
+extern "C" int fap_graph_rows_bytes(const fap_dgraph *G, int32_t count, int64_t *bytes) try {
+  if (!G || !bytes || count < 0) return fail(FAP_ERR_INVALID, "bad argument");
+  DeviceGuard g(G->ctx->device);
+  const int64_t r = std::max(count, 1);
+  if (G->cache_ready && G->use_cache)
+    *bytes = grown_by(G->d_rowgroups, r * (int64_t)sizeof(RowGroup)) + grown_by(G->d_rowloc, r * 4) + grown_by(G->d_rowout, r * 8) +
+             grown_by(G->d_rowidx, 2 * r * 8);
+  else
+    *bytes = grown_by(G->d_src, r * 4) +
+             (G->K > 0 ? grown_by(G->sssp_scratch, (int64_t)std::max(sssp_scratch_rows(G->n, (int)r), 1) * G->n * 4) : 0);
+  return FAP_OK;
+} catch (...) {
+  return fail_exception();
+}
+
 extern "C" int fap_graph_resident(fap_dgraph *G, int32_t part) try {
   if (!G || part < 1 || part > G->K) return 0;
   return G->row_base[part] >= 0 ? 1 : 0;
@@ -2844,11 +2977,11 @@ struct CacheShape {
   int32_t ldf = kFloydTile, max_b = 0, max_s = 0;
   int64_t total_b = 0;
   int64_t bytes(const fap_dgraph *G) const {
-    // boundary rows + Floyd squares + descriptors + the sources' lists
+    // boundary rows + Floyd squares + descriptors + the sources' and the elimination's lists
     auto a = [](int64_t b) { return (int64_t)alloc_size((size_t)b); };
     return a(std::max<int64_t>(total_b, 1) * G->ldD * 4) + a((int64_t)G->K * ldf * ldf * 4) +
            a((int64_t)G->K * (int64_t)sizeof(PartDesc)) + a(std::max<int64_t>(total_b, 1) * 4) +
-           a(std::max<int64_t>(total_b, 1) * 8);
+           a(std::max<int64_t>(total_b, 1) * 8) + (G->el.plan.ok ? a((int64_t)G->K * 4) + a((int64_t)(G->K + 1) * 8) : 0);
   }
 };
 
@@ -2905,7 +3038,11 @@ int cache_build_impl(fap_dgraph *G) {
     FAP_TRY(G->sssp_scratch.ensure(
         (size_t)std::max(sssp_scratch_rows(G->n, (int)src.size()), 1) * (size_t)G->n * 4));
   const bool given = !bm && elim_given_ok(G);
-  if (!elim && !given) {
+  if (elim || given) {
+    FAP_TRY(grow_elim(G, G->cparts, false));
+    FAP_CK(cudaStreamSynchronize(st));
+    FAP_TRY(fill_elim(G, G->cparts, false));
+  } else {
     int32_t mnb = 0;
     G->cq.sym = bm && G->sym_local && G->floyd_sym;
     const std::vector<QItem> qitems = floyd_queue_items(G->cparts, G->cq.sym, &G->cq.nfloyd, &mnb);
@@ -2940,7 +3077,6 @@ int cache_build_impl(fap_dgraph *G) {
     // Elimination: phases [numeric elimination, boundary graph, closures,
     // boundary rows].
     if constexpr (std::is_same<T, int32_t>::value) {
-      FAP_TRY(prepare_elim(G, G->cparts));
       FAP_TRY(prepare_bgraph(G, G->cparts));
       FAP_CK(cudaEventRecord(G->cev[0], st));
       FAP_TRY(run_elim(G, dp, K, cs.max_s, F, cs.ldf, Bd, G->cev[1], G->cev[2], G->cev[3], status, &L));
@@ -2979,7 +3115,6 @@ int cache_build_impl(fap_dgraph *G) {
   FAP_CK(cudaEventRecord(G->cev[2], st));
   G->cache_bmethod = false;
   if (given) {
-    FAP_TRY(prepare_elim(G, G->cparts, true));
     FAP_TRY(run_elim_given<T>(G, dp, K, cs.max_s, F, cs.ldf, Bd, &L));
   } else if (G->floyd_per_cta) {
     FAP_CK(launch_floyd_parts<T>(dp, K, F, cs.ldf, Bd, G->ldD, st2ed, status, st, &L));
@@ -3352,21 +3487,7 @@ extern "C" int fap_graph_cache_bytes(const fap_dgraph *G, int64_t *bytes, int *b
     // boundary-graph matrix and tables
     const CacheShape cs = cache_shape(G);
     if (bmethod_ok(G)) {
-      const int64_t ldB =
-          round_up(std::max<int64_t>(bgraph_bf(G) ? G->bpcol[G->K + 1] : G->total_b, 1), kFloydTile);
-      *bytes = cs.bytes(G) + (int64_t)alloc_size((size_t)bgraph_words(ldB) * 4) +
-               (int64_t)alloc_size((size_t)std::max<int64_t>(G->total_b, 1) * cs.ldf * 4) +
-               (int64_t)alloc_size((size_t)(G->K + 1) * sizeof(BPart)) +
-               (int64_t)alloc_size((size_t)std::max<int64_t>(2 * G->total_b, 2) * 8);
-      if (bgraph_tiled_expand(G)) *bytes += (int64_t)alloc_size((size_t)G->total_b * 8);
-      if (bgraph_bf(G)) {  // cross-arc CSR, work lists, tiles, stamps, part table
-        const int64_t xe = std::max<int64_t>(G->bgraph_cross, 1);
-        *bytes += 3 * (int64_t)alloc_size((size_t)(G->total_b + 1) * 4) + 3 * (int64_t)alloc_size((size_t)xe * 4) +
-                  (int64_t)alloc_size((size_t)2 * bgraph_ztiles(G) * G->total_b * 4 + 4 * sizeof(int)) +
-                  (int64_t)alloc_size((size_t)bgraph_ztiles(G) * G->total_b * kMsbfS * 4) +
-                  (int64_t)alloc_size((size_t)3 * bgraph_ztiles(G) * G->total_b * 4) +
-                  (int64_t)alloc_size((size_t)bgraph_ztiles(G) * (G->K + 1) * 4);
-      }
+      *bytes = cs.bytes(G) + bgraph_growth(G, cs.ldf, false, true);
     } else {
       const int cnt = (int)std::min<int64_t>(cs.total_b, INT32_MAX);
       if (use_msbf(G))  // tiles, bitmaps, work items

@@ -15,6 +15,7 @@
 #include <cstring>
 #include <deque>
 #include <exception>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -72,7 +73,6 @@ struct GSlot {
   int64_t base_bytes = 0;  // CSR + partition, always resident
   std::vector<int32_t> vnum, voff, bnum;
   int64_t max_part = 0;        // largest part (rows)
-  int64_t bgraph_bytes = 0;    // the boundary graph's matrix
   int64_t reserved_rows = 0;   // output rows the graph's D holds (0: released)
   // the batch in flight: distance rows, checksums on the device and their
   // pinned host copy, status word (buffers grow with the largest batch)
@@ -157,7 +157,7 @@ struct fap_server {
   bool complete(GSlot &g);
   bool launch(int gi);
   int64_t held_bytes();
-  bool make_room(int64_t need, int self, bool *hopeless);
+  bool make_room(const std::function<int64_t()> &bytes, int self, bool *hopeless);
   void finish(Req *r, int state, int status);
 };
 
@@ -254,14 +254,16 @@ bool grow_dev(T **p, int64_t *cap, int64_t want) {
 }
 }  // namespace
 
-// Frees memory until `need` more bytes fit in the budget: first the output
+// Frees memory until `need()` more bytes fit in the budget (asked again when
+// graph `self`'s own buffers have gone): first the output
 // buffers of idle graphs (least recently used first), then their resident
 // caches, then graph `self`'s own output buffers.  Returns whether they fit;
 // *hopeless is set when they cannot fit even after every busy graph
 // finishes (nothing else holds memory that could be freed).
-bool fap_server::make_room(int64_t need, int self, bool *hopeless) {
+bool fap_server::make_room(const std::function<int64_t()> &bytes, int self, bool *hopeless) {
   HostTimer timer(this, kStepRoom);
   *hopeless = false;
+  const int64_t need = bytes();
   if (held_bytes() + need <= budget) return true;
   std::vector<int> idle;
   bool others_busy = false;
@@ -289,7 +291,7 @@ bool fap_server::make_room(int64_t need, int self, bool *hopeless) {
     }
   if (output_bytes(*graphs[self]) > 0) {
     release_outputs(*graphs[self]);
-    if (held_bytes() + need <= budget) return true;
+    if (held_bytes() + bytes() <= budget) return true;
   }
   *hopeless = !others_busy;
   return false;
@@ -385,7 +387,7 @@ bool fap_server::launch(int gi) {
     int64_t cb = 0;
     int built = 0;
     bool hopeless = false;
-    if (fap_graph_cache_bytes(g.dg, &cb, &built) == FAP_OK && make_room(cb, gi, &hopeless) &&
+    if (fap_graph_cache_bytes(g.dg, &cb, &built) == FAP_OK && make_room([&] { return cb; }, gi, &hopeless) &&
         [&] {
           HostTimer t(this, kStepCache);
           return fap_graph_cache_build(g.dg);
@@ -407,43 +409,38 @@ bool fap_server::launch(int gi) {
   int64_t limit_rows = std::max<int64_t>(1, cap / row_bytes);
   if (max_batch_rows > 0) limit_rows = std::min<int64_t>(limit_rows, max_batch_rows);
   if (kind == FAP_REQ_SUBGRAPH) limit_rows = std::min<int64_t>(std::max<int64_t>(limit_rows, g.max_part), g.n);
-  // Device bytes the batch still needs beyond what the graph holds (upper
-  // bounds of what fap_solve / fap_graph_copy_block / fap_graph_rows_async
-  // allocate): the output matrix or rows buffer and the checksums up to
-  // their target sizes; without the resident cache also one padded Floyd
-  // square per part (all of the batch's largest side) and SSSP scratch rows
-  // (at most one per source); the int32->float staging of the largest block
-  // copied to the host.
-  // When the buffers at their target size do not fit the budget, the batch
-  // is sized exactly (its own rows only).
-  int64_t rows = 0, nparts = 0, ldf = 0, srcs = 0, stage_rows = 0;
+  // Device bytes the batch still needs beyond what the graph holds: what
+  // fap_solve and fap_graph_copy_block or fap_graph_rows_async allocate
+  // (fap_graph_batch_bytes, fap_graph_rows_bytes), the rows buffer and the
+  // checksums up to their target sizes.  When the buffers at their target size
+  // do not fit the budget, the batch is sized exactly (its own rows only).
+  int64_t rows = 0, stage_rows = 0;
   bool exact = false;
-  auto footprint = [&](int64_t r, int64_t np, int64_t lf, int64_t sc, int64_t sg) -> int64_t {
+  // (evaluated anew whenever make_room has released something of the graph's)
+  auto footprint = [&](const std::vector<int32_t> &with, int64_t r, int64_t sg) -> int64_t {
     const int64_t target = exact ? r : std::max(r, limit_rows);
-    int64_t need = std::max<int64_t>(0, target - g.cs_cap) * 8 + sg * (int64_t)g.n * 4;
+    int64_t need = std::max<int64_t>(0, target - g.cs_cap) * 8, own = 0;
     if (kind == FAP_REQ_ROWS) {
       const int64_t b = r * (int64_t)g.n * 4;
       // (the small buffer grows to kSmallRowsBytes at once unless the batch is sized exactly)
       need += b > kSmallRowsBytes ? b : std::max<int64_t>(0, (exact ? b : kSmallRowsBytes) - g.rows_small_cap * 4);
-      if (!cached) need += r * (int64_t)g.n * 4;
-    } else {
-      need += std::max<int64_t>(0, target - g.reserved_rows) * g.ldD * 4;
-      // (or the boundary graph's matrix, up to 4 MB more)
-      if (!cached) need += np * lf * lf * 4 + std::max(sc * (int64_t)g.n * 4, std::min(g.bgraph_bytes, int64_t(4) << 20));
+      if (fap_graph_rows_bytes(g.dg, (int32_t)std::min<int64_t>(r, INT32_MAX), &own) != FAP_OK) own = INT64_MAX / 4;
+    } else if (fap_graph_batch_bytes(g.dg, with.data(), (int32_t)with.size(), target, sg, &own) != FAP_OK) {
+      own = INT64_MAX / 4;
     }
-    return need;
+    return need + own;
   };
+  std::vector<int32_t> with;
   for (auto it = g.pending.begin(); it != g.pending.end();) {
     Req *r = *it;
     if (r->kind != kind) break;  // one kind per batch, in arrival order
-    int64_t add_rows = 0, n_parts = nparts, n_ldf = ldf, n_srcs = srcs, n_stage = stage_rows;
+    int64_t add_rows = 0, n_stage = stage_rows;
+    with = parts;
     if (kind == FAP_REQ_SUBGRAPH) {
       const int32_t p = r->ids[0];
       if (part_row[p] < 0) {
         add_rows = g.vnum[p];
-        n_parts++;
-        n_ldf = std::max<int64_t>(n_ldf, ((int64_t)std::max(g.vnum[p], 1) + 127) / 128 * 128);
-        n_srcs += g.bnum[p];
+        with.push_back(p);
       }
       if (r->host_out && g.dtype == FAP_DTYPE_I32) n_stage = std::max<int64_t>(n_stage, g.vnum[p]);
     } else {
@@ -451,10 +448,11 @@ bool fap_server::launch(int gi) {
     }
     if (!batch.empty() && rows + add_rows > limit_rows) break;
     bool hopeless = false;
-    bool fits = make_room(footprint(rows + add_rows, n_parts, n_ldf, n_srcs, n_stage), gi, &hopeless);
+    const auto need = [&] { return footprint(with, rows + add_rows, n_stage); };
+    bool fits = make_room(need, gi, &hopeless);
     if (!fits && batch.empty() && !exact) {
       exact = true;
-      fits = make_room(footprint(rows + add_rows, n_parts, n_ldf, n_srcs, n_stage), gi, &hopeless);
+      fits = make_room(need, gi, &hopeless);
     }
     if (!fits) {
       if (!batch.empty()) break;  // run what fits
@@ -464,9 +462,6 @@ bool fap_server::launch(int gi) {
       progressed = true;
       continue;
     }
-    nparts = n_parts;
-    ldf = n_ldf;
-    srcs = n_srcs;
     stage_rows = n_stage;
     batch.push_back(r);
     if (kind == FAP_REQ_SUBGRAPH) {
@@ -716,9 +711,6 @@ int fap_server_add_graph(fap_server *s, int32_t n, int64_t m, const int32_t *row
   g->vnum.assign(ver_num, ver_num + K + 1);
   g->voff.assign(ver_offset, ver_offset + K + 1);
   g->bnum.assign(bdy_num, bdy_num + K + 1);
-  int64_t bsum = 0;
-  for (int32_t p = 1; p <= K; p++) bsum += bdy_num[p];
-  g->bgraph_bytes = ((bsum + 127) / 128 * 128) * ((bsum + 127) / 128 * 128) * 4;
   for (int32_t p = 1; p <= K; p++) g->max_part = std::max<int64_t>(g->max_part, ver_num[p]);
   // Batches change from one launch to the next: launch the stages directly
   // instead of capturing a CUDA graph per batch.

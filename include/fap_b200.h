@@ -332,6 +332,14 @@ FAP_API int fap_graph_cache_release(fap_dgraph *g);
 /* Device bytes the cache holds (*built = 1) or would need to be built,
  * including its SSSP scratch (*built = 0). */
 FAP_API int fap_graph_cache_bytes(const fap_dgraph *g, int64_t *bytes, int *built);
+/* Upper bounds of the device bytes that come on top of what g holds
+ * (fap_graph_device_bytes), allocation sizes as they are rounded: for a batched
+ * solve of the parts (NULL: all) with `rows` output rows reserved (at least the
+ * parts' own) and a block of copied_rows rows copied to the host; and for
+ * fap_graph_rows_async of `count` sources. */
+FAP_API int fap_graph_batch_bytes(const fap_dgraph *g, const int32_t *parts, int32_t count, int64_t rows,
+                                  int64_t copied_rows, int64_t *bytes);
+FAP_API int fap_graph_rows_bytes(const fap_dgraph *g, int32_t count, int64_t *bytes);
 
 /* Device time (ms) of the stages of the last fap_solve, measured with events
  * on the context stream: [sssp, gather, floyd, minplus, total]. */
