@@ -164,13 +164,17 @@ struct DeviceGuard {
 
 }  // namespace
 
+// Largest scratch that fap_op_minplus allocates for packed operands.
+constexpr int64_t kPackedScratchMax = int64_t(1) << 30;
+
 struct fap_ctx {
   int device = 0;
   int sm_count = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t own = nullptr;
   cudaEvent_t ev[6] = {};
-  DevBuf scratch;     // fap_op_floyd padding copy
+  DevBuf scratch;     // fap_op_floyd padding copy, fap_op_minplus packed operands
+  int64_t packed_want = 0;  // scratch bytes the largest fap_op_minplus so far would have used
   DevBuf status;      // int device status for device-pointer ops
   DevBuf sink;        // microbenchmark sink
   int64_t launches = 0;
@@ -2358,10 +2362,20 @@ extern "C" int fap_op_minplus(fap_ctx *c, int dtype, int32_t M, int32_t N, int32
   // 900 x 20,011 x 150: int32 253 / 228, float32 290 / 260; 2,000 x 40,001 x 700:
   // 3,813 / 3,357 and 4,506 / 4,128); float32 with 16-byte rows stays generic
   // (1,024 x 20,480 x 160: 287 / 294), and so do products below 10^9 (312 x 21,881
-  // x 67: 72 / 80), where the copies and the waves' ends cost more.
+  // x 67: 72 / 80), where the copies and the waves' ends cost more.  Allocating
+  // the copies' memory takes 350 us, more than one product gains (the first one
+  // on a new context 310 us without, 660 with): it is made when a product needs
+  // that much for the second time, up to 1 GB, which the context keeps.
   const bool rows16 = ldb % 4 == 0 && N % 4 == 0 && (uintptr_t)B % 16 == 0;
-  if ((dtype == FAP_DTYPE_I32 || (dtype == FAP_DTYPE_F32 && !rows16)) && (double)M * N * K >= 1e9 &&
-      c->scratch.ensure((size_t)minplus_packed_elems(M, N, K) * 4) == FAP_OK) {
+  bool packed = (dtype == FAP_DTYPE_I32 || (dtype == FAP_DTYPE_F32 && !rows16)) && (double)M * N * K >= 1e9;
+  if (packed) {
+    const int64_t want = minplus_packed_elems(M, N, K) * 4;
+    if (want > (int64_t)c->scratch.bytes) {
+      packed = want <= c->packed_want && c->scratch.ensure((size_t)c->packed_want) == FAP_OK;
+      if (want <= kPackedScratchMax) c->packed_want = std::max(c->packed_want, want);
+    }
+  }
+  if (packed) {
     FAP_CK(cudaMemsetAsync(c->status.p, 0, sizeof(int), c->stream));
     if (dtype == FAP_DTYPE_I32)
       FAP_CK(launch_minplus_packed<int32_t>(M, N, K, (const int32_t *)A, lda, (const int32_t *)B, ldb, (int32_t *)C, ldc,

@@ -25,11 +25,12 @@ def test_tall_and_deep_minplus(cuda_ok, dtype, M, N, K):
     step = max(1, 100000000 // (M * N))
     for k in range(0, K, step):
         torch.minimum(want, (a[:, k:k + step, None] + b[None, k:k + step]).amin(1), out=want)
-    c = torch.full((M, N), 7, dtype=t, device="cuda")
     ctx = Context(0)
-    torch.cuda.synchronize()
-    ctx.minplus(a, b, c, FAP_DTYPE_I32 if dtype == "i32" else FAP_DTYPE_F32)
-    assert torch.equal(c, want)
+    for _ in range(2):                        # (the second call has packed operands)
+        c = torch.full((M, N), 7, dtype=t, device="cuda")
+        torch.cuda.synchronize()
+        ctx.minplus(a, b, c, FAP_DTYPE_I32 if dtype == "i32" else FAP_DTYPE_F32)
+        assert torch.equal(c, want)
 
 
 def test_floyd_of_more_rows_than_a_grid_has(cuda_ok):
