@@ -740,7 +740,9 @@ def run_extra(args, job, ctx, relax_peak, hbm_peak, peak_kind):
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
     torch.cuda.synchronize()
     ms, mp_ms, fl_ms = [], [], []
+    work = np.zeros(3)                     # of one step: closures, inner rows, parts from groups
     for _ in range(args.extra_steps):
+        work[:] = 0
         flush.zero_()
         e0 = torch.cuda.Event(enable_timing=True)
         e1 = torch.cuda.Event(enable_timing=True)
@@ -752,12 +754,14 @@ def run_extra(args, job, ctx, relax_peak, hbm_peak, peak_kind):
             dg.solve(grp, FAP_MODE_BATCHED, check_errors=False)
             mp += float(dg.last_timing()[3])
             fl += float(dg.last_timing()[2])
+            work += dg.last_work()
         e1.record(stream)
         e1.synchronize()
         ms.append(e0.elapsed_time(e1))
         mp_ms.append(mp)
         fl_ms.append(fl)
     dg.check()
+    batched_stage1 = dg.stage1_name()
     # the plain form of the same job: one launch sequence per part (stage 1
     # by SSSP from that part's boundary vertices), the groups as above
     plain_ms = []
@@ -775,22 +779,25 @@ def run_extra(args, job, ctx, relax_peak, hbm_peak, peak_kind):
     del flush
     ms_step = float(np.mean(ms))
     mp_step = float(np.mean(mp_ms))
-    mp_relax = float(sum(float(vn[p] - bn[p]) * float(bn[p]) * n for p in mine))
+    mp_relax = float(work[1])              # as run: separator groups relax a fraction of inner x boundary
     mp_bytes = float(sum(4.0 * ((vn[p] - bn[p]) * n + (vn[p] - bn[p]) * bn[p] + bn[p] * n) for p in mine))
-    # With stage 1 by SSSP and int32-only min-plus tiles (float32, or packing
-    # off), the min-plus tiles run inside the Floyd work queue: the stage
-    # timings then hold Floyd and min-plus together.
+    # With stage 1 by SSSP, closures by Floyd and int32-only min-plus tiles
+    # (float32, or packing off), the min-plus tiles run inside the Floyd work
+    # queue: the stage timings then hold Floyd and min-plus together.
     form = solve_tuned["params"] if solve_tuned else {"minplus_pack16": int(not args.no_pack16),
                                                       "floyd_queue": int(not args.no_queue)}
-    stage1_now = dg.stage1_name()
-    mp_in_queue = (bool(form["floyd_queue"]) and stage1_now.startswith("SSSP")
+    stage1_now = batched_stage1
+    mp_in_queue = (bool(form["floyd_queue"]) and stage1_now.startswith("SSSP") and "elimination" not in stage1_now
                    and (dtype != 0 or not form["minplus_pack16"]))
     mp_note = None
     if mp_in_queue:
         mp_step += float(np.mean(fl_ms))
-        mp_relax += float(sum(float(vn[p]) ** 3 for p in mine))
+        mp_relax += float(work[0])
         mp_note = ("the min-plus tiles ran inside the Floyd work queue: time and relaxations of "
                    "Floyd-Warshall and min-plus together")
+    elif work[2] > 0:
+        mp_note = (f"the inner rows of {int(work[2])} parts came from separator groups: the relaxations are "
+                   "those run, padding included")
     a = mp_relax / (mp_step * 1e-3) / 1e9
     gpu = gpu_parity_blocks(dg, groups, job["parts"], dtype, staged, FAP_MODE_BATCHED) if job["parts"] else {}
     stage1 = dg.stage1_name()
@@ -997,6 +1004,7 @@ def main_fap(args):
     clocks.start()
     t_timed = time.time()
     step_ms, stages = [], []
+    work = np.zeros(3)                     # of one step: closures, inner rows, parts from groups
     cache_phases = []
     launches = 0
     for _ in range(args.steps):
@@ -1005,6 +1013,7 @@ def main_fap(args):
         e1 = torch.cuda.Event(enable_timing=True)
         e0.record(stream)
         st_step = np.zeros(5)
+        work[:] = 0
         if staged:
             ec = torch.cuda.Event(enable_timing=True)
             dg.cache_build(rebuild=True)
@@ -1019,6 +1028,7 @@ def main_fap(args):
             launches += dg.last_launches()
         for grp in groups:
             dg.solve(grp, FAP_MODE_BATCHED, check_errors=False)
+            work += dg.last_work()
             if len(groups) > 1:
                 st_step += dg.last_timing()
                 launches += dg.last_launches()
@@ -1111,8 +1121,11 @@ def main_fap(args):
     m_arcs = int(ro[-1])
     srcs = int(sum(int(bn[p]) for p in mine))
     sssp_bytes = srcs * (4 * (n + 1) + 8 * m_arcs + 4 * n)
-    floyd_relax = float(sum(float(vn[p]) ** 3 for p in mine))
-    mp_relax = float(sum(float(vn[p] - bn[p]) * float(bn[p]) * n for p in mine))
+    # (relaxations as run; closures of the resident cache: Floyd-Warshall's,
+    # unless elimination closed them, which keeps no count there)
+    by_elim = "elimination" in stage1_used
+    floyd_relax = float(work[0]) or (0.0 if by_elim else float(sum(float(vn[p]) ** 3 for p in mine)))
+    mp_relax = float(work[1])
     mp_bytes = float(sum(4.0 * ((vn[p] - bn[p]) * n + (vn[p] - bn[p]) * bn[p] + bn[p] * n)
                          for p in mine))
     stage_roof = {
@@ -1129,15 +1142,17 @@ def main_fap(args):
     dom = max(("sssp", "floyd", "minplus"), key=lambda k: stage_roof[k]["ms"])
     if dom == "floyd":
         a = stage_roof["floyd"]["achieved_grelax_s"]
-        roof = {"kernel": "floyd_part_kernel", "bound": "dpx", "achieved": a,
+        kern = "elim_close_kernel" if by_elim else "floyd_part_kernel"
+        roof = {"kernel": kern, "bound": "dpx", "achieved": a,
                 "peak": peak_grelax, "unit": "Grelax/s", "frac": a / peak_grelax,
                 "peak_source": "measured relaxation microbenchmark (fap_measure_relax_peak)",
-                "traffic": read_traffic(wl.name, "floyd_part_kernel")}
+                "traffic": read_traffic(wl.name, kern)}
     else:
         thin_only = all(int(bn[p]) <= 16 for p in mine)
         kern = (("msbf_iter_kernel" if "Bellman-Ford" in stage1_used else "sssp_frontier_kernel")
                 if dom == "sssp" else
-                "minplus_thin_kernel" if thin_only else "minplus_part_kernel")
+                "minplus_thin_kernel" if thin_only else
+                "elim_merge_kernel" if work[2] > 0 else "minplus_part_kernel")
         a = stage_roof[dom]["achieved_gbs"]
         roof = {"kernel": kern, "bound": "hbm", "achieved": a, "peak": hbm_peak, "unit": "GB/s",
                 "frac": a / hbm_peak, "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
@@ -1148,7 +1163,12 @@ def main_fap(args):
     stage_roof["minplus"]["frac_of_hbm"] = stage_roof["minplus"]["achieved_gbs"] / hbm_peak
     form_now = (solve_tuned["params"] if solve_tuned else
                 {"minplus_pack16": int(not args.no_pack16), "floyd_queue": int(not args.no_queue)})
-    if (form_now["floyd_queue"] and stage1_used.startswith("SSSP")
+    if by_elim:
+        stage_roof["floyd"]["note"] = "parts closed by vertex elimination; relaxations as run"
+    if work[2] > 0:
+        stage_roof["minplus"]["note"] = (f"the inner rows of {int(work[2])} parts came from separator groups; "
+                                         "relaxations as run, padding included")
+    if (form_now["floyd_queue"] and stage1_used.startswith("SSSP") and not by_elim
             and (dtype != 0 or not form_now["minplus_pack16"])):
         stage_roof["minplus"]["note"] = ("the min-plus tiles of parts with more than 16 boundary vertices "
                                          "ran inside the Floyd work queue: their time is in the floyd stage")

@@ -471,6 +471,7 @@ struct fap_dgraph {
   bool last_merge = false, last_given = false;
   int32_t merge_units = 0, merge_slots = 0;
   DevBuf d_merge;
+  double relax[2] = {0, 0};  // fap_graph_last_work of the prepared batch
   std::vector<int32_t> boff;
   std::vector<int32_t> bpcol;  // boundary columns of dB padded per part to multiples of 4 (prefix sums)
   bool last_bmethod = false;   // the prepared batch uses it
@@ -1114,7 +1115,6 @@ constexpr int64_t kBgraphAutoMaxB = 65536;
 bool bgraph_bf(const fap_dgraph *G) {
   return G->bgraph_form == 2 || (G->bgraph_form == 0 && G->total_b > kBgraphFloydMax);
 }
-const char *stage1_form_name(const fap_dgraph *G, bool bmethod);
 
 bool bgraph_tiled_expand(const fap_dgraph *G) { return G->bgraph_form == 2 || G->total_b > kBgraphStagedMax; }
 
@@ -1496,6 +1496,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
   G->thin_pos.clear();
   G->merge.clear();
   G->merge_units = G->merge_slots = 0;
+  G->relax[0] = G->relax[1] = 0;
   // Floyd arena: equal padded squares (one tensor map describes all parts);
   // with the resident cache, the parts' closed matrices in the cache.
   int32_t ldf = kFloydTile;
@@ -1528,6 +1529,10 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
     }
     G->part_src_off.push_back((int32_t)G->src.size());
     G->part_work_begin.push_back((int32_t)G->work.size());
+    const double s = d.s, b = d.b;
+    if (elim || given) G->relax[0] += s * (G->el.plan.parts[p - 1].nent + (elim ? b * b : 0));
+    else if (!cached) G->relax[0] += s * s * s;
+    double inner = (s - b) * b;
     if (d.b <= G->thin_max_b) {
       G->thin_pos.push_back((int32_t)G->thin.size());
       G->thin.push_back((int32_t)i);
@@ -1535,6 +1540,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
       G->thin_pos.push_back(-1);
       if (merge && merge_ok(G, p)) {
         G->merge.push_back(make_int2(p - 1, (int)i));
+        inner = (double)G->el.plan.group_work[p - 1];
         const ElimPart &q = G->el.plan.parts[p - 1];
         G->merge_units = std::max(G->merge_units, G->el.plan.glev[q.glev_off + q.gnlev] - G->el.plan.glev[q.glev_off]);
         G->merge_slots = std::max(G->merge_slots, q.nslots);
@@ -1542,6 +1548,7 @@ int prepare_batch(fap_dgraph *G, const std::vector<int32_t> &ids, bool cached, b
         for (int32_t m0 = 0; m0 < d.s - d.b; m0 += kMinplusBM) G->work.push_back(MPWork{(int32_t)i, m0});
       }
     }
+    G->relax[1] += inner * (double)n;
     G->part_work_end.push_back((int32_t)G->work.size());
   }
   G->f_elems = foff;
@@ -1712,11 +1719,14 @@ bool use_msbf(const fap_dgraph *G) {
   return G->n > 0 && G->m >= 6 * (int64_t)G->n;
 }
 
-constexpr const char *kElimName = "boundary graph, Floyd class closed by elimination";
-
-const char *stage1_form_name(const fap_dgraph *G, bool bmethod) {
+// How stage 1 (and with elimination the parts' closures) runs.
+std::string stage1_form_name(const fap_dgraph *G, bool bmethod, bool elim, bool given) {
+  if (elim)
+    return G->el2.plan.ok ? "boundary graph, Floyd class closed by elimination"
+                          : "boundary graph, Floyd closure, parts closed by elimination";
   if (bmethod) return bgraph_bf(G) ? "boundary graph, Bellman-Ford closure" : "boundary graph, Floyd closure";
-  return use_msbf(G) ? "SSSP, tiled Bellman-Ford" : "SSSP, frontier";
+  return std::string(use_msbf(G) ? "SSSP, tiled Bellman-Ford" : "SSSP, frontier") +
+         (given ? ", parts closed by elimination" : "");
 }
 
 // Tiles of the tiled SSSP form run side by side: as many as fit in
@@ -1805,7 +1815,7 @@ int run_solve(fap_dgraph *G, int mode) {
       FAP_CK(record_event(c->ev[3], st));
       FAP_CK(launch_minplus_thin<T>(dp, G->d_thin.as<int32_t>(), (int)G->thin.size(), G->max_s, G->n, F, D,
                                     G->ldD, gid, ed2st, st, &L));
-    if constexpr (std::is_same<T, int32_t>::value) FAP_TRY(run_merge(G, dp, F, &L));
+      FAP_TRY(run_merge(G, dp, F, &L));
       FAP_CK(launch_minplus_parts<T>(dp, np, dw, (int)G->work.size(), G->n, F, G->max_ldf, D, G->ldD,
                                      G->max_rows, gid, ed2st, status, st, &L, pack16_of(G)));
       if (G->paths) FAP_TRY(launch_paths<T>(G, dp, np, G->max_s, F, &L));
@@ -1974,7 +1984,7 @@ extern "C" int fap_solve(fap_dgraph *G, const int32_t *parts, int32_t count, int
   // (the tiled SSSP form tests convergence on the host: not capturable)
   const bool host_loop = !cached && (bmethod ? bgraph_bf(G) : use_msbf(G));
   G->stage1_name = cached ? "resident cache (" + G->cache_stage1_name + ")"
-                          : elim ? kElimName : stage1_form_name(G, bmethod);
+                          : stage1_form_name(G, bmethod, elim, given);
   // A batch is captured the second time it is solved unchanged: a batch
   // solved once (a server's batches of changing composition) runs its
   // launches directly instead of paying for a capture and an instantiation.
@@ -2079,6 +2089,16 @@ extern "C" const char *fap_graph_stage1_name(const fap_dgraph *G) {
     return "";
   }
   return G->stage1_name.c_str();
+}
+
+extern "C" int fap_graph_last_work(const fap_dgraph *G, double *relax2, int32_t *merged_parts) try {
+  if (!G || !relax2) return fail(FAP_ERR_INVALID, "NULL argument");
+  relax2[0] = G->relax[0];
+  relax2[1] = G->relax[1];
+  if (merged_parts) *merged_parts = (int32_t)G->merge.size();
+  return FAP_OK;
+} catch (...) {
+  return fail_exception();
 }
 
 extern "C" int fap_graph_last_launches(fap_dgraph *G, int64_t *count) try {
@@ -3097,7 +3117,7 @@ int cache_build_impl(fap_dgraph *G) {
       FAP_CK(cudaEventRecord(G->cev[4], st));
     }
     G->cache_bmethod = true;
-    G->cache_stage1_name = kElimName;
+    G->cache_stage1_name = stage1_form_name(G, true, true, false);
   } else if (bm) {
     // Boundary-graph form: local closures, boundary-graph APSP, expansion.
     FAP_TRY(prepare_bgraph(G, G->cparts));
@@ -3116,9 +3136,9 @@ int cache_build_impl(fap_dgraph *G) {
     FAP_CK(launch_local_fixup<T>(dp, K, cs.max_s, F, G->d_FB.as<const T>(), cs.ldf, st, &L));
     FAP_CK(cudaEventRecord(G->cev[4], st));
     G->cache_bmethod = true;
-    G->cache_stage1_name = stage1_form_name(G, true);
+    G->cache_stage1_name = stage1_form_name(G, true, false, false);
   } else {
-  G->cache_stage1_name = stage1_form_name(G, false);
+  G->cache_stage1_name = stage1_form_name(G, false, false, given);
   FAP_CK(cudaEventRecord(G->cev[0], st));
   FAP_TRY(run_stage1_sssp<T>(G, G->d_src.as<const int32_t>(), G->d_srcrows.as<const int64_t>(),
                              (int)src.size(), Bd, status, rounds, &L));
@@ -3403,7 +3423,7 @@ int shard_finish_impl(fap_dgraph *G, const void *recv, int32_t world, const int3
   c->launches += L;
   FAP_TRY(read_status(G));
   G->cache_bmethod = true;
-  G->cache_stage1_name = std::string("sharded ") + stage1_form_name(G, true);
+  G->cache_stage1_name = "sharded " + stage1_form_name(G, true, false, false);
   G->cache_ready = true;
   G->cache_valid = mine;
   G->last_ids.clear();

@@ -573,6 +573,13 @@ class DeviceGraph:
         """How stage 1 of the last solve ran, in words (fap_graph_stage1_name)."""
         return (lib().fap_graph_stage1_name(self._h) or b"").decode()
 
+    def last_work(self):
+        """(closure relaxations, inner-row relaxations, parts from separator
+        groups) of the last batch (see fap_graph_last_work)."""
+        r, m = np.zeros(2), ctypes.c_int32()
+        check(lib().fap_graph_last_work(self._h, ptr(r), ctypes.byref(m)), "last_work")
+        return float(r[0]), float(r[1]), int(m.value)
+
     def last_launches(self) -> int:
         x = ctypes.c_int64()
         check(lib().fap_graph_last_launches(self._h, ctypes.byref(x)))

@@ -205,13 +205,21 @@ FAP_API int fap_graph_sssp_rows(fap_dgraph *g, const int32_t *sources, int32_t c
  * queue; 0: three launches per pivot block); "floyd_symmetric" (default 1:
  * on parts whose arcs all have reverses of equal weight, the queue computes
  * the local closures' tiles on and above the diagonal and stores their
- * transposes); "eliminate" (default 1: on undirected int32 graphs without
- * duplicate arcs inside a part, whose parts eliminate with short lists, the
- * batched solves and the resident cache close the parts and small boundary
- * graphs by vertex elimination instead of Floyd-Warshall and SSSP, also for
- * batches of some of the parts; needs "floyd_queue" and "floyd_symmetric" on
- * and "stage1" and "bgraph_form" not forced to another form; the same values
- * either way); "thin_max_b" (0..16, default 16: parts with at most this many
+ * transposes); "eliminate" (default 1: vertex elimination instead of
+ * Floyd-Warshall, in batched solves and the resident cache, of graphs whose
+ * parts have at most 6144 vertices each and eliminate with short lists.
+ * Undirected int32 graphs without duplicate arcs inside a part and with at most
+ * 8192 boundary vertices: parts and small boundary graphs are closed by it
+ * instead of Floyd-Warshall and SSSP, also for batches of some of the parts,
+ * unless "floyd_queue" or "floyd_symmetric" is 0 or "stage1" or "bgraph_form"
+ * forces another form.  Where stage 1 is an SSSP (float32, directed graphs,
+ * "stage1" 1): the parts are closed by it from their boundary rows, whatever
+ * "floyd_queue" and "floyd_symmetric" say; float32 graphs with an arc of
+ * more than 1e8 keep Floyd-Warshall.  int32 parts with more than 16 boundary
+ * vertices: their inner rows come from separator groups where that takes at
+ * most half of the relaxations.  int32 values are the same either way; float32
+ * sums associate differently (a few ulps; the same pairs are reachable).  0:
+ * the general path everywhere); "thin_max_b" (0..16, default 16: parts with at most this many
  * boundary vertices take the store-shaped thin min-plus kernel, the others
  * the register-tiled one); "max_resident_rows" (>= 1: at most this many
  * output rows are reserved on the device, as when HBM cannot hold all n
@@ -342,13 +350,16 @@ FAP_API int fap_graph_batch_bytes(const fap_dgraph *g, const int32_t *parts, int
 FAP_API int fap_graph_rows_bytes(const fap_dgraph *g, int32_t count, int64_t *bytes);
 
 /* Device time (ms) of the stages of the last fap_solve, measured with events
- * on the context stream: [sssp, gather, floyd, minplus, total]. */
+ * on the context stream: [sssp, gather, floyd, minplus, total].  With the
+ * boundary graph the first three are [its closure and the boundary rows,
+ * gather, local closures]; with elimination [boundary rows, numeric
+ * elimination and boundary graph, the parts' closures]. */
 FAP_API int fap_graph_last_timing(fap_dgraph *g, float *ms5);
 
 /* How the last fap_solve obtained the boundary rows (stage 1): 1 SSSP from
  * every boundary vertex; 2 the boundary graph (every part's local closure,
  * APSP over the boundary vertices, expansion; chosen for batches of all
- * parts of int32 graphs without two arcs joining the same ordered pair
+ * parts (with "eliminate" also of some) of int32 graphs without two arcs joining the same ordered pair
  * inside a part, when they have at most 8192 boundary vertices (closed by
  * Floyd) or when the boundary graph has at most 8 edges per graph edge and
  * at most 65536 vertices (closed by the tiled Bellman-Ford); with "stage1" =
@@ -356,12 +367,24 @@ FAP_API int fap_graph_last_timing(fap_dgraph *g, float *ms5);
  * rounding order, a few ulps); 3 the resident cache; 0 no solve yet. */
 FAP_API int fap_graph_last_stage1(const fap_dgraph *g);
 
-/* How stage 1 of the last solve ran, in words: "SSSP, frontier", "SSSP,
- * tiled Bellman-Ford", "boundary graph, Floyd closure", "boundary graph,
- * Bellman-Ford closure", "boundary graph, Floyd class closed by elimination"
- * (at most 8192 boundary vertices, "eliminate"), or "resident cache (<how it was built>)"; "" before
- * the first solve.  The string lives until the next solve or cache build. */
+/* How stage 1 of the last solve ran, in words: "SSSP, frontier" or "SSSP,
+ * tiled Bellman-Ford", followed by ", parts closed by elimination" where the
+ * parts' closures are ("eliminate"); "boundary graph, Floyd closure" or
+ * "boundary graph, Bellman-Ford closure"; with "eliminate" and at most 8192
+ * boundary vertices "boundary graph, Floyd class closed by elimination" (parts
+ * and boundary graph; no Floyd-Warshall runs) or "boundary graph, Floyd
+ * closure, parts closed by elimination"; or "resident cache (<how it was
+ * built>)"; "" before the first solve.  The string lives until the next solve
+ * or cache build. */
 FAP_API const char *fap_graph_stage1_name(const fap_dgraph *g);
+
+/* Relaxations that stages 2 and 3 of the last batch run, relax2[2]: closures
+ * (Floyd-Warshall s^3 a part; by elimination its list entries, and the
+ * boundary's pairs where it is closed too, per column; 0 from the resident
+ * cache) and inner rows (inner x boundary a column; from separator groups their
+ * padded list entries).  *merged_parts (may be NULL): parts whose inner rows
+ * came from separator groups. */
+FAP_API int fap_graph_last_work(const fap_dgraph *g, double *relax2, int32_t *merged_parts);
 
 /* Number of kernels the last fap_solve launched. */
 FAP_API int fap_graph_last_launches(fap_dgraph *g, int64_t *count);

@@ -191,3 +191,37 @@ def test_predecessor_rows_at_every_width(cuda_ok, n):
     for r in list(inner)[::37] + list(inner)[-9:]:
         want = _predecessors(D[r], int(st2ed[vo[p] + r]), ro, col, w)
         assert np.array_equal(P[r], want), r
+
+
+def test_forms_name_themselves(cuda_ok):
+    """The form names say what closes the parts and the boundary graph, and the
+    relaxations reported are those run."""
+    def names(dg, **params):
+        for k, v in params.items():
+            dg.set_param(k, v)
+        dg.solve(None, FAP_MODE_BATCHED)
+        return dg.stage1_name()
+
+    wl, dg = _workload("road20k")
+    vn, bn = wl.ver_num[1:].astype(float), wl.bdy_num[1:].astype(float)
+    assert names(dg) == "boundary graph, Floyd closure"
+    assert dg.last_work() == ((vn ** 3).sum(), ((vn - bn) * bn).sum() * wl.n, 0)
+    assert names(dg, eliminate=1) == "boundary graph, Floyd class closed by elimination"
+    assert 0 < dg.last_work()[0] < (vn ** 3).sum() / 100 and dg.last_work()[2] == 0
+    assert names(dg, stage1=1) == "SSSP, frontier, parts closed by elimination"
+    assert names(dg, eliminate=0) == "SSSP, frontier"
+
+    dg, *_ = _device(G.grid_graph(112, 111, extra_frac=0.01, wmin=1, wmax=100, seed=3), 30)
+    assert names(dg) == "boundary graph, Floyd closure, parts closed by elimination"
+    closures, inner, merged = dg.last_work()
+    assert merged > 0
+    assert names(dg, eliminate=0) == "boundary graph, Floyd closure"
+    assert closures < dg.last_work()[0] and inner < dg.last_work()[1] / 2 and dg.last_work()[2] == 0
+    dg.set_param("eliminate", 1)
+    dg.cache_build()
+    assert names(dg) == "resident cache (boundary graph, Floyd closure, parts closed by elimination)"
+    assert dg.last_work()[0] == 0 and dg.last_work()[1] == inner
+
+    dg, *_ = _device(G.rmat_graph(11, 30000, seed=62), 4)
+    assert names(dg) == "SSSP, tiled Bellman-Ford, parts closed by elimination"
+    assert names(dg, eliminate=0) == "SSSP, tiled Bellman-Ford"
