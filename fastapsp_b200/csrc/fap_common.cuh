@@ -18,8 +18,6 @@ namespace fapb {
 constexpr int kInfI32 = 100000000;  // 1e8, the reference's MAXVALUE
 constexpr float kInfF32 = 1e8f;
 constexpr uint32_t kInfBitsF32 = 0x4cbebc20u;  // of kInfF32
-// Largest value of the packed 16-bit min-plus (see tma_minplus_tile16).
-constexpr int32_t kPackCap = 16383;
 
 template <typename T>
 struct Dist;

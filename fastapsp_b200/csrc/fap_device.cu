@@ -1699,7 +1699,8 @@ __global__ void __launch_bounds__(kPredThreads)
   }
 }
 
-// The same rule for whole rows of graphs whose rows fit in shared memory: a CTA
+// The same rule for the inner rows of parts with wide boundaries, where the
+// graph's rows fit in shared memory: a CTA
 // holds R rows of D there, so the gathers of the in-neighbours'
 // distances are shared-memory loads instead of L2 ones (16,001-vertex geometric
 // graph, the rows of its parts with wide boundaries: 1.26 -> 0.56 ms), and walks
@@ -1708,17 +1709,15 @@ template <typename T, int R>
 __global__ void __launch_bounds__(1024, 1)
     pred_row_kernel(const PartDesc *__restrict__ parts, const T *__restrict__ D, int32_t *__restrict__ P,
                     int64_t ldD, int n, const int32_t *__restrict__ tro, const int32_t *__restrict__ tcol,
-                    const T *__restrict__ tw, const int32_t *__restrict__ st2ed, int mode) {
+                    const T *__restrict__ tw, const int32_t *__restrict__ st2ed) {
   extern __shared__ __align__(16) unsigned char pr_smem_raw[];
   using V = typename Vec4<T>::type;
   T *rows_s = reinterpret_cast<T *>(pr_smem_raw);  // R x ldD
   const PartDesc pd = parts[blockIdx.y];
-  const bool thin = pd.b <= kPredThinB;
-  if (mode == kPredThickInner && thin) return;
-  const int rlo = mode == kPredThickInner ? pd.b : 0, rhi = mode == kPredBoundaryRows ? pd.b : pd.s;
+  if (pd.b <= kPredThinB) return;
   const T inf = Dist<T>::inf();
-  for (int r0 = rlo + blockIdx.x * R; r0 < rhi; r0 += gridDim.x * R) {
-    const int rows = min(R, rhi - r0);
+  for (int r0 = pd.b + blockIdx.x * R; r0 < pd.s; r0 += gridDim.x * R) {
+    const int rows = min(R, pd.s - r0);
     const T *Dr = D + (pd.row_base + r0) * ldD;
     int32_t *Pr = P + (pd.row_base + r0) * ldD;
     __syncthreads();
@@ -1780,7 +1779,7 @@ __global__ void __launch_bounds__(1024, 1)
 // about 28,000 columns); returns false otherwise.
 template <typename T>
 bool launch_pred_rows(const PartDesc *parts, int nparts, const T *D, int32_t *P, int64_t ldD, int n,
-                      const int32_t *tro, const int32_t *tcol, const T *tw, const int32_t *st2ed, int mode,
+                      const int32_t *tro, const int32_t *tcol, const T *tw, const int32_t *st2ed,
                       cudaStream_t stream, cudaError_t *err) {
   const size_t row = (size_t)ldD * sizeof(T);
   const int fit = (int)((size_t)226 * 1024 / row);
@@ -1791,7 +1790,7 @@ bool launch_pred_rows(const PartDesc *parts, int nparts, const T *D, int32_t *P,
     *err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(R * row));
     if (*err != cudaSuccess) return;
     const int gx = std::max(1, 4 * device_sm_count() / nparts);
-    kern<<<dim3(gx, nparts), 1024, R * row, stream>>>(parts, D, P, ldD, n, tro, tcol, tw, st2ed, mode);
+    kern<<<dim3(gx, nparts), 1024, R * row, stream>>>(parts, D, P, ldD, n, tro, tcol, tw, st2ed);
     *err = cudaGetLastError();
   };
   if (fit >= 8) run(std::integral_constant<int, 8>());
@@ -1821,7 +1820,7 @@ cudaError_t launch_pred(const PartDesc *parts, int nparts, int max_s, const T *D
   pred_kernel<T><<<dim3((unsigned)ceil_div(max_s, kPredThreads), nparts, gz), kPredThreads, 0, stream>>>(
       parts, D, P, ldD, n, tro, tcol, tw, st2ed, kPredOwnColumns);
   // 4. inner rows of the other parts (the gather rule)
-  if (launch_pred_rows<T>(parts, nparts, D, P, ldD, n, tro, tcol, tw, st2ed, kPredThickInner, stream, &e)) {
+  if (launch_pred_rows<T>(parts, nparts, D, P, ldD, n, tro, tcol, tw, st2ed, stream, &e)) {
     if (e != cudaSuccess) return e;
   } else {
     pred_kernel<T><<<dim3((unsigned)ceil_div(n, kPredThreads), nparts, gz), kPredThreads, 0, stream>>>(

@@ -286,7 +286,6 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
     d.nslots = (int32_t)q.sloc.size();
     d.sloc_off = (int32_t)out->sloc.size();
     out->sloc.insert(out->sloc.end(), q.sloc.begin(), q.sloc.end());
-    out->max_slots = std::max(out->max_slots, d.nslots);
     const int32_t rows0 = (int32_t)out->rows8.size() / 2, list0 = (int32_t)out->list.size(),
                   unit0 = (int32_t)out->units.size();
     for (ElimUnit u : q.units) {
@@ -299,7 +298,6 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
     out->list.insert(out->list.end(), q.list.begin(), q.list.end());
     out->stream16 += q.stream16;
     out->group_work.push_back(q.group_work);
-    out->max_units = std::max(out->max_units, (int32_t)q.units.size());
     out->parts.push_back(d);
     out->loc.insert(out->loc.end(), q.loc.begin(), q.loc.end());
     out->inv.insert(out->inv.end(), q.inv.begin(), q.inv.end());
@@ -311,7 +309,6 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
     for (int32_t e = 0; e < d.s; e++)
       out->eend.insert(out->eend.end(), q.eptr[e + 1] - q.eptr[e], q.eptr[e + 1]);
     out->max_s = std::max(out->max_s, d.s);
-    out->max_b = std::max(out->max_b, d.b);
     out->max_nent = std::max(out->max_nent, d.nent);
     out->max_nlev = std::max(out->max_nlev, d.nlev);
   }

@@ -101,7 +101,7 @@ struct ElimPlan {
   int64_t stream16 = 0;
   int32_t max_chunk16 = 0, max_chunks = 0;
   std::vector<int64_t> group_work;  // per part: list entries times padded rows
-  int32_t max_s = 0, max_b = 0, max_nent = 0, max_nlev = 0, max_units = 0, max_slots = 0;
+  int32_t max_s = 0, max_nent = 0, max_nlev = 0;
   int64_t nent = 0;
 };
 
@@ -115,7 +115,7 @@ struct ElimGraph {
 // Symbolic elimination of the parts on up to `threads` host threads; graph(p)
 // fills in part p's adjacency and is called on any of them.  ok
 // stays false when a part has more than kElimMaxS vertices (a strip of eight
-// columns fills the shared memory) or more than s^2 / kElimDense entries.
+// columns fills the shared memory) or more than s * max(s, 256) / kElimDense entries.
 constexpr int32_t kElimMaxS = 6144;
 constexpr int64_t kElimDense = 16;
 // inf: bits of the sentinel; groups: also build the separator groups.
@@ -135,7 +135,7 @@ struct ElimDev {
   const ElimChunk *chunks;
   int2 *ent;      // {plan number of u, W(v, u)}, written by launch_elim_up
   int32_t *entb;  // W(u, v); null: symmetric
-  int32_t nparts, max_s, max_b, max_nent, max_nlev, max_chunk16, max_chunks;
+  int32_t nparts, max_s, max_nent, max_nlev, max_chunk16, max_chunks;
 };
 
 // M (ld): the sentinel on nfill x nfill, 0 on the first nb diagonal entries,

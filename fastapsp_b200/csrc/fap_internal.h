@@ -203,15 +203,20 @@ template <typename T>
 cudaError_t launch_floyd_parts_multi(const PartDesc *parts, int nparts, int max_nb, T *F, int64_t ld,
                                      int *status, cudaStream_t stream, int64_t *launches);
 
-// Plain: one padded matrix (ld a multiple of kFloydTile, nb tiles per side
-// in use), one launch per phase per pivot block.  status may be null.  s:
-// the real rows and columns (the rest is padding holding the sentinel,
-// whose pivots and tile halves are skipped); -1 = all of the nb tiles.  sym: the
-// matrix is symmetric (a hint: half of the tiles may be left out).
 // dst (side ld_dst, a multiple of 4): the s x s matrix src, the sentinel around it.
 template <typename T>
 cudaError_t launch_pad_copy(T *dst, int64_t ld_dst, const T *src, int64_t ld_src, int s, cudaStream_t stream,
                             int64_t *launches);
+
+// Plain: one padded matrix (ld a multiple of kFloydTile, nb tiles per side
+// in use), one launch per phase per pivot block.  status may be null.  s:
+// the real rows and columns (the rest is padding holding the sentinel,
+// whose pivots and tile halves are skipped); -1 = all of the nb tiles.  sym: the
+// matrix is symmetric (a hint: half of the tiles may be left out).  work: see
+// launch_floyd64, which takes the sizes where it is faster.
+template <typename T>
+cudaError_t launch_floyd_matrix(T *mat, int64_t ld, int nb, int *status, cudaStream_t stream,
+                                int64_t *launches, int s = -1, bool sym = false, T *work = nullptr);
 
 // launch_floyd_matrix in pivot blocks of 64; sym: the matrix is symmetric.
 // work: kFloyd64Work words of the call's own, 16-byte aligned (panels then run
@@ -219,9 +224,6 @@ cudaError_t launch_pad_copy(T *dst, int64_t ld_dst, const T *src, int64_t ld_src
 constexpr int64_t kFloyd64Work = 6 * 64 * 64;
 template <typename T>
 cudaError_t launch_floyd64(T *mat, int64_t ld, int s, bool sym, T *work, cudaStream_t stream, int64_t *launches);
-template <typename T>
-cudaError_t launch_floyd_matrix(T *mat, int64_t ld, int nb, int *status, cudaStream_t stream,
-                                int64_t *launches, int s = -1, bool sym = false, T *work = nullptr);
 
 // Boundary rows of the listed parts: F[i][j] -> D[row_base+i][st2ed[start+j]].
 template <typename T>
@@ -376,16 +378,17 @@ cudaError_t launch_minplus_rows(const PartDesc *parts, const RowGroup *groups, i
                                 int64_t *launches);
 
 // Generic C = min(INF, A (x) B).
+template <typename T>
+cudaError_t launch_minplus_generic(int M, int N, int K, const T *A, int64_t lda, const T *B,
+                                   int64_t ldb, T *C, int64_t ldc, cudaStream_t stream,
+                                   int64_t *launches);
+
 // ... with the operands first copied into padded scratch
 // (minplus_packed_elems(M, N, K) elements).
 int64_t minplus_packed_elems(int M, int N, int K);
 template <typename T>
 cudaError_t launch_minplus_packed(int M, int N, int K, const T *A, int64_t lda, const T *B, int64_t ldb, T *C,
                                   int64_t ldc, T *scratch, int *status, cudaStream_t stream, int64_t *launches);
-template <typename T>
-cudaError_t launch_minplus_generic(int M, int N, int K, const T *A, int64_t lda, const T *B,
-                                   int64_t ldb, T *C, int64_t ldc, cudaStream_t stream,
-                                   int64_t *launches);
 
 // Fill rows x cols of a row-major matrix with v.
 template <typename T>

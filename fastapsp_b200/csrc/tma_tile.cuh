@@ -187,6 +187,7 @@ __device__ __forceinline__ bool tma_minplus_tile(const CUtensorMap *mapA, int ax
 // exceeds 2 * kPackCap < 2^15, and a packed result r < kPackCap is exactly
 // min_k A[i][k] + B[k][c] - off[c] (r >= kPackCap: no finite path).
 // ---------------------------------------------------------------------------
+constexpr int32_t kPackCap = 16383;
 constexpr uint32_t kPackInit = 0x7FFE7FFEu;   // 32766 in both halves
 
 template <class C>
