@@ -454,11 +454,12 @@ struct fap_dgraph {
   bool sym_local = false;
   int64_t total_b = 0;
   // Elimination form of the boundary graph (elim_ok): el the parts' plan, el2
-  // the boundary graph's own (one part without a boundary, up to
-  // kElimGraphMax vertices; larger ones are closed by Floyd), barcs the arcs
+  // the boundary graph's own (one part without a boundary; without a plan it is
+  // closed by Floyd), el2_small: it is small enough for one, barcs the arcs
   // between boundary vertices as (boundary index, boundary index, weight).
   bool eliminate = true;   // parameter "eliminate"
   bool el_sym = false;     // the plans of the boundary-graph form exist
+  bool el2_small = false;
   bool last_elim = false;  // the prepared batch uses it
   ElimBuf el, el2;
   std::vector<int32_t> barcs;
@@ -720,13 +721,20 @@ void cache_drop(fap_dgraph *G) {
 }  // namespace
 
 namespace {
-// Boundary graphs are closed by elimination up to this size and number of
-// entries, larger ones by Floyd on dB: one CTA runs the numeric part, with
-// the entries in its shared memory (road114k, 650 vertices and 4,100
-// entries: 0.10 ms against 0.56 ms for Floyd; a 1,726-vertex boundary graph of
-// a geometric graph, 67,000 entries in L2: 5.5 ms against 1.9).
+// Boundary graphs are planned for elimination up to this size and number of
+// entries (batches of some of the parts close the whole boundary graph only
+// then), and closed by it where their lists hold at most kElimGraphList
+// entries on average and Floyd would take more than one block of 64: one CTA
+// runs the numeric part, level after level.  Vertices, entries, us by Floyd in
+// blocks of 64 / by elimination, with the parts' numeric elimination: road
+// 48, 160: 31 / 39; 122, 644: 65 / 57; 360, 2,720: 158 / 95; 642, 3,969:
+// 276 / 105; geometric 118, 955: 63 / 74; 341, 4,506: 161 / 157; 560, 5,803:
+// 234 / 149; 595, 9,160: 262 / 236; 389, 6,069: 184 / 191; 579, 14,150:
+// 266 / 469; 717, 22,566: 348 / 784; 1,421, 42,121: 523 / 2,370 (39 graphs: the
+// rule is at most 26 us off the better one).
 constexpr int64_t kElimGraphMax = 2048;
 constexpr int64_t kElimGraphEntries = 24576;
+constexpr int64_t kElimGraphList = 11;
 
 // The elimination plans: of the parts, for every graph with boundary vertices
 // whose parts eliminate with short lists, and on undirected int32 graphs
@@ -812,6 +820,8 @@ void plan_elim(fap_dgraph *G) {
   };
   elim_build(1, boundary_graph, 1, inf, false, &G->el2.plan);
   if (G->el2.plan.nent > kElimGraphEntries) G->el2.plan = ElimPlan{};
+  G->el2_small = G->el2.plan.ok;
+  if (G->total_b <= 64 || G->el2.plan.nent > kElimGraphList * G->total_b) G->el2.plan = ElimPlan{};
   if (G->el2.plan.ok) elim_offsets(round_up(G->total_b, kFloydTile), &G->el2.plan);
 }
 
@@ -823,7 +833,7 @@ int build_elim(fap_dgraph *G) {
   G->el2.clear();
   G->barcs.clear();
   G->dev_barcs = nullptr;
-  G->el_sym = false;
+  G->el_sym = G->el2_small = false;
   plan_elim(G);
   if (!G->el.plan.ok) return FAP_OK;
   const bool directed = !G->sym_local;  // (el2 is symmetric)
@@ -834,7 +844,7 @@ int build_elim(fap_dgraph *G) {
     G->el.clear();
     G->el2.clear();
     G->barcs.clear();
-    G->el_sym = false;
+    G->el_sym = G->el2_small = false;
     return FAP_OK;
   }
   char *base = G->d_elim.as<char>();
@@ -850,7 +860,7 @@ int build_elim(fap_dgraph *G) {
 // Whether solves close the boundary graph and the parts by elimination:
 // where a plan exists and no parameter asks for one of the other forms.
 // A batch of some of the parts (`sources` boundary vertices; all parts: -1)
-// takes it where elimination closes the whole boundary graph too, and dB
+// takes it where the whole boundary graph is small (el2_small), and dB
 // needs no more memory than the SSSP scratch rows it replaces, or 4 MB (the
 // server admits such batches by that size).  One part of a 50,001-vertex road
 // graph: 0.17 ms instead of 4.6.  (Its rows are written by one grid row per
@@ -861,7 +871,7 @@ bool elim_ok(const fap_dgraph *G, int64_t sources) {
       !G->floyd_queue || !G->floyd_sym || G->floyd_per_cta || G->total_b > kBgraphFloydMax)
     return false;
   const int64_t ldB = round_up(G->total_b, kFloydTile);
-  return sources < 0 || (G->el2.plan.ok && G->K <= kMaxGridY && ldB * ldB <= std::max<int64_t>(sources * G->n, kElimBatchElems));
+  return sources < 0 || (G->el2_small && G->K <= kMaxGridY && ldB * ldB <= std::max<int64_t>(sources * G->n, kElimBatchElems));
 }
 
 // Words of dB, with the work space of its Floyd closure after it from 1,024
@@ -2378,16 +2388,27 @@ extern "C" int fap_op_minplus(fap_ctx *c, int dtype, int32_t M, int32_t N, int32
   if (ldc < N || (K > 0 && (lda < K || ldb < N))) return fail(FAP_ERR_INVALID, "bad leading dimension");
   DeviceGuard g(c->device);
   int64_t L = 0;
-  // Large products with the operands packed first (generic / packed, us, at
-  // 900 x 20,011 x 150: int32 253 / 228, float32 290 / 260; 2,000 x 40,001 x 700:
-  // 3,813 / 3,357 and 4,506 / 4,128); float32 with 16-byte rows stays generic
-  // (1,024 x 20,480 x 160: 287 / 294), and so do products below 10^9 (312 x 21,881
-  // x 67: 72 / 80), where the copies and the waves' ends cost more.  Allocating
+  // Large products with the operands packed first: rows by TMA whatever their
+  // alignment, and a last row tile that is at most half full at half the work.
+  // Two CTAs run on an SM, and few tiles lose more in their last wave than that
+  // gains: with a half-empty row tile from one wave on (packed / generic over
+  // products drawn from 60..2,000 x 1,000..40,000 x 8..700: int32 0.89 of the time
+  // on average, at most 1.04, float32 with unaligned rows 0.91, 1.04; 148 x 31,085
+  // x 292 0.79; below one wave up to 1.10), otherwise int32 from 2.5 waves on (0.92,
+  // at most 1.00; 1.06 below), float32 from four (0.96, 1.02; 1.11 below), and all
+  // from 1.2 or 1.5 x 10^9 relaxations on (312 x 21,881 x 67: 77 us / 89).  900 x
+  // 20,011 x 150: int32 253 / 228 us, float32 290 / 260.  float32 with 16-byte rows
+  // gains little at best (1,024 x 20,480 x 160 288 / 305, 2,000 x 40,000 x 500
+  // 3,033 / 2,981) and stays generic.  Allocating
   // the copies' memory takes 350 us, more than one product gains (the first one
   // on a new context 310 us without, 660 with): it is made when a product needs
   // that much for the second time, up to 1 GB, which the context keeps.
+  const bool i32 = dtype == FAP_DTYPE_I32;
   const bool rows16 = ldb % 4 == 0 && N % 4 == 0 && (uintptr_t)B % 16 == 0;
-  bool packed = (dtype == FAP_DTYPE_I32 || (dtype == FAP_DTYPE_F32 && !rows16)) && (double)M * N * K >= 1e9;
+  const bool half = M % kMinplusBM > 0 && M % kMinplusBM <= kMinplusBM / 2;
+  const int64_t tiles = ceil_div(M, kMinplusBM) * ceil_div(N, kMinplusBN);
+  bool packed = (i32 || (dtype == FAP_DTYPE_F32 && !rows16)) && tiles >= (half ? 2 : i32 ? 5 : 8) * (int64_t)c->sm_count &&
+                (double)M * N * K >= (half ? 1.2e9 : 1.5e9);
   if (packed) {
     const int64_t want = minplus_packed_elems(M, N, K) * 4;
     if (want > (int64_t)c->scratch.bytes) {
