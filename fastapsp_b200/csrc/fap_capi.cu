@@ -312,7 +312,7 @@ struct ElimBuf {
       if (base && src && bytes > 0 && *err == cudaSuccess) *err = cudaMemcpy(d, src, bytes, cudaMemcpyHostToDevice);
       return d;
     };
-    auto ints = [&](const std::vector<int32_t> &v) { return reinterpret_cast<const int32_t *>(put(v.data(), v.size() * 4)); };
+    auto ints = [&](const PlanArray<int32_t> &v) { return reinterpret_cast<const int32_t *>(put(v.data(), v.size() * 4)); };
     dev = ElimDev{};
     dev.parts = reinterpret_cast<const ElimPart *>(put(plan.parts.data(), plan.parts.size() * sizeof(ElimPart)));
     dev.loc = ints(plan.loc);
@@ -776,7 +776,7 @@ void plan_elim(fap_dgraph *G) {
       g->ptr.push_back((int32_t)g->adj.size());
     }
   };
-  elim_build(K, part_graph, threads, inf, i32, &G->el.plan);
+  elim_build(K, part_graph, threads, inf, !G->sym_local, i32, &G->el.plan);
   if (!G->el.plan.ok) return;
   // (float32 parts keep min-plus over the boundary, which distance rows from
   // the resident cache match bit for bit)
@@ -793,8 +793,12 @@ void plan_elim(fap_dgraph *G) {
           G->barcs.insert(G->barcs.end(), {bidx(u), bidx(v), weight(e)});
       }
     }
-  // the least weight of every crossing pair has to be the same both ways
-  std::sort(cross.begin(), cross.end());
+  // the least weight of every crossing pair has to be the same both ways (the
+  // arcs come by their tails already)
+  for (size_t i = 0, k; i < cross.size(); i = k) {
+    for (k = i; k < cross.size() && cross[k][0] == cross[i][0]; k++) {}
+    std::sort(cross.begin() + i, cross.begin() + k);
+  }
   cross.erase(std::unique(cross.begin(), cross.end(),
                           [](const auto &a, const auto &b) { return a[0] == b[0] && a[1] == b[1]; }),
               cross.end());
@@ -818,7 +822,7 @@ void plan_elim(fap_dgraph *G) {
         g->ptr.push_back((int32_t)g->adj.size());
       }
   };
-  elim_build(1, boundary_graph, 1, inf, false, &G->el2.plan);
+  elim_build(1, boundary_graph, 1, inf, false, false, &G->el2.plan);
   if (G->el2.plan.nent > kElimGraphEntries) G->el2.plan = ElimPlan{};
   G->el2_small = G->el2.plan.ok;
   if (G->total_b <= 64 || G->el2.plan.nent > kElimGraphList * G->total_b) G->el2.plan = ElimPlan{};

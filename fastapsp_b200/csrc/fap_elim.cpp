@@ -28,7 +28,7 @@ struct PartPlan {
 // their levels, and pendant paths and chains are then taken every other
 // vertex instead of end to end (road114k: 17 levels instead of 53 with 1.46
 // entries per vertex instead of 1.36; a 256 x 256 grid 101 instead of 113).
-void eliminate(const ElimGraph &g, int32_t inf, PartPlan *out) {
+void eliminate(const ElimGraph &g, int32_t inf, bool directed, PartPlan *out) {
   const int32_t s = g.s, b = g.b;
   const int W = (s + 63) / 64;
   std::vector<uint64_t> A((size_t)s * W, 0);
@@ -112,22 +112,31 @@ void eliminate(const ElimGraph &g, int32_t inf, PartPlan *out) {
     out->eptr[e + 1] = out->eptr[e] + (e < b ? 0 : ncnt[out->loc[e]]);
   out->ecol.resize(nnz);
   out->w0.assign(nnz, inf);
-  out->w0b.assign(nnz, inf);
-  for (int32_t e = b; e < s; e++) {
-    const int32_t v = out->loc[e];
-    int32_t *c = &out->ecol[out->eptr[e]];
-    int32_t k = 0;
-    for (int32_t i = 0; i < ncnt[v]; i++) c[k++] = out->inv[nbr[nptr[v] + i]];
-    std::sort(c, c + k, std::greater<int32_t>());
+  if (directed) out->w0b.assign(nnz, inf);
+  // N+ in descending plan numbers: every u appends itself to the lists that
+  // hold it, the last u first (sorting list by list took three times as long)
+  std::vector<int32_t> rptr(s + 1, 0), rev(nnz), at(s);
+  for (int32_t u : nbr) rptr[u + 1]++;
+  for (int32_t u = 0; u < s; u++) {
+    rptr[u + 1] += rptr[u];
+    at[u] = rptr[u];
+  }
+  for (int32_t v : order)
+    for (int32_t i = nptr[v]; i < nptr[v] + ncnt[v]; i++) rev[at[nbr[i]]++] = out->inv[v];
+  std::copy(out->eptr.begin(), out->eptr.end() - 1, at.begin());  // (by plan number from here on)
+  for (int32_t e = s - 1; e >= 0; e--) {
+    const int32_t u = out->loc[e];
+    for (int32_t i = rptr[u]; i < rptr[u + 1]; i++) out->ecol[at[rev[i]]++] = e;
   }
   if (!g.w.empty())
     for (int32_t i = 0; i < s; i++)
       for (int32_t a = g.ptr[i]; a < g.ptr[i + 1]; a++) {
         const int32_t x = out->inv[i], y = out->inv[g.adj[a]], v = std::max(x, y), u = std::min(x, y);
         if (v < b) continue;
-        const int32_t *c = &out->ecol[out->eptr[v]], *end = &out->ecol[0] + out->eptr[v + 1];
-        const auto at = std::lower_bound(c, end, u, std::greater<int32_t>()) - &out->ecol[0];
-        (x > y ? out->w0 : out->w0b)[at] = g.w[a];
+        const int32_t *c = out->ecol.data() + out->eptr[v], *end = out->ecol.data() + out->eptr[v + 1];
+        const auto at = std::lower_bound(c, end, u, std::greater<int32_t>()) - out->ecol.data();
+        if (x > y) out->w0[at] = g.w[a];
+        else if (directed) out->w0b[at] = g.w[a];
       }
   out->ok = true;
 }
@@ -221,22 +230,42 @@ void group_rows(PartPlan *q) {
 
 }  // namespace
 
+namespace {
+// work() on up to `threads` threads, this one among them.
+template <typename F>
+void run_threads(int threads, F work) {
+  std::vector<std::thread> pool;
+  try {
+    for (int t = 1; t < threads; t++) pool.emplace_back(work);
+  } catch (...) {  // fewer threads than asked for
+  }
+  work();
+  for (std::thread &t : pool) t.join();
+}
+
+template <typename T>
+void put(PlanArray<T> *to, size_t at, const std::vector<T> &from) {
+  std::copy(from.begin(), from.end(), to->data() + at);
+}
+}  // namespace
+
 void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, int threads, int32_t inf,
-                bool groups, ElimPlan *out) {
+                bool directed, bool groups, ElimPlan *out) {
   *out = ElimPlan{};
   const int K = nparts;
   std::vector<PartPlan> pp(K);
   std::atomic<int> next{0};
   std::atomic<bool> dense{false};
   std::atomic<bool> failed{false};  // an allocation failed: no plan
-  auto work = [&] {
+  threads = std::max(1, std::min(threads, K));
+  run_threads(threads, [&] {
     try {
       for (int p = next++; p < K && !dense; p = next++) {
         ElimGraph g;
         graph(p, &g);
         pp[p].boff = g.boff;
         pp[p].b = g.b;
-        if (g.s <= kElimMaxS) eliminate(g, inf, &pp[p]);
+        if (g.s <= kElimMaxS) eliminate(g, inf, directed, &pp[p]);
         if (!pp[p].ok) dense = true;
         else if (groups && g.b > kThinBoundary) group_rows(&pp[p]);  // (the others take the thin merge)
       }
@@ -244,76 +273,97 @@ void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, 
       failed = true;
       dense = true;
     }
-  };
-  const int nt = std::max(1, std::min(threads, K));
-  std::vector<std::thread> pool;
-  try {
-    for (int t = 1; t < nt; t++) pool.emplace_back(work);
-  } catch (...) {  // fewer threads than asked for
-  }
-  work();
-  for (std::thread &t : pool) t.join();
+  });
   if (dense || failed) return;
-  size_t nv = 0, ne = 0;
-  for (const PartPlan &q : pp) {
-    nv += q.loc.size();
-    ne += q.ecol.size();
-  }
-  out->loc.reserve(nv);
-  out->inv.reserve(nv);
-  out->eptr.reserve(nv + K);
-  for (auto *a : {&out->ecol, &out->eend, &out->w0, &out->w0b}) a->reserve(ne);
+  // The parts' places in the plan's arrays, then the copies.
+  size_t nv = 0, ne = 0, np = 0, nl = 0, ng = 0, nu = 0, nr = 0, ns = 0, ni = 0, nc = 0;
+  std::vector<int32_t> unit0(K), rows0(K), list0(K);
   for (int p = 0; p < K; p++) {
     const PartPlan &q = pp[p];
     ElimPart d{};
     d.s = (int32_t)q.loc.size();
     d.b = q.b;
     d.boff = q.boff;
-    d.voff = (int32_t)out->loc.size();
-    d.eptr_off = (int32_t)out->eptr.size();
-    d.ent_off = (int32_t)out->ecol.size();
+    d.voff = (int32_t)nv;
+    d.eptr_off = (int32_t)np;
+    d.ent_off = (int32_t)ne;
     d.nent = (int32_t)q.ecol.size();
-    d.lev_off = (int32_t)out->lev.size();
+    d.lev_off = (int32_t)nl;
     d.nlev = (int32_t)q.lev.size() - 1;
-    d.glev_off = (int32_t)out->glev.size();
+    d.glev_off = (int32_t)ng;
     d.gnlev = std::max(0, (int32_t)q.glev.size() - 1);
     d.stream_off = (int32_t)out->stream16;
-    d.chunk_off = (int32_t)out->chunks.size();
+    d.chunk_off = (int32_t)nc;
     d.nchunks = (int32_t)q.chunks.size();
+    d.nslots = (int32_t)q.sloc.size();
+    d.sloc_off = (int32_t)ns;
+    unit0[p] = (int32_t)nu;
+    rows0[p] = (int32_t)(nr / 2);
+    list0[p] = (int32_t)ni;
+    nv += q.loc.size();
+    np += q.eptr.size();
+    ne += q.ecol.size();
+    nl += q.lev.size();
+    ng += q.glev.size();
+    nu += q.units.size();
+    nr += q.rows8.size();
+    ns += q.sloc.size();
+    ni += q.list.size();
+    nc += q.chunks.size();
     for (const ElimChunk &c : q.chunks) out->max_chunk16 = std::max(out->max_chunk16, c.n16);
     out->max_chunks = std::max(out->max_chunks, d.nchunks);
-    out->chunks.insert(out->chunks.end(), q.chunks.begin(), q.chunks.end());
-    d.nslots = (int32_t)q.sloc.size();
-    d.sloc_off = (int32_t)out->sloc.size();
-    out->sloc.insert(out->sloc.end(), q.sloc.begin(), q.sloc.end());
-    const int32_t rows0 = (int32_t)out->rows8.size() / 2, list0 = (int32_t)out->list.size(),
-                  unit0 = (int32_t)out->units.size();
-    for (ElimUnit u : q.units) {
-      u.rows += rows0;
-      u.list += list0;
-      out->units.push_back(u);
-    }
-    for (int32_t l : q.glev) out->glev.push_back(unit0 + l);
-    out->rows8.insert(out->rows8.end(), q.rows8.begin(), q.rows8.end());
-    out->list.insert(out->list.end(), q.list.begin(), q.list.end());
     out->stream16 += q.stream16;
     out->group_work.push_back(q.group_work);
-    out->parts.push_back(d);
-    out->loc.insert(out->loc.end(), q.loc.begin(), q.loc.end());
-    out->inv.insert(out->inv.end(), q.inv.begin(), q.inv.end());
-    out->eptr.insert(out->eptr.end(), q.eptr.begin(), q.eptr.end());
-    out->ecol.insert(out->ecol.end(), q.ecol.begin(), q.ecol.end());
-    out->w0.insert(out->w0.end(), q.w0.begin(), q.w0.end());
-    out->w0b.insert(out->w0b.end(), q.w0b.begin(), q.w0b.end());
-    out->lev.insert(out->lev.end(), q.lev.begin(), q.lev.end());
-    for (int32_t e = 0; e < d.s; e++)
-      out->eend.insert(out->eend.end(), q.eptr[e + 1] - q.eptr[e], q.eptr[e + 1]);
     out->max_s = std::max(out->max_s, d.s);
     out->max_nent = std::max(out->max_nent, d.nent);
     out->max_nlev = std::max(out->max_nlev, d.nlev);
+    out->parts.push_back(d);
   }
-  out->nent = (int64_t)out->ecol.size();
-  out->ok = out->nent < INT32_MAX / 2 && out->stream16 < INT32_MAX / 2;
+  out->nent = (int64_t)ne;
+  if (out->nent >= INT32_MAX / 2 || out->stream16 >= INT32_MAX / 2) return;
+  out->loc.make(nv);
+  out->inv.make(nv);
+  out->eptr.make(np);
+  out->ecol.make(ne);
+  out->eend.make(ne);
+  out->w0.make(ne);
+  out->w0b.make(directed ? ne : 0);
+  out->lev.make(nl);
+  out->units.make(nu);
+  out->glev.make(ng);
+  out->rows8.make(nr);
+  out->list.make(ni);
+  out->sloc.make(ns);
+  out->chunks.make(nc);
+  next = 0;
+  // (small plans: a thread costs more than its share of the copies)
+  run_threads((int)std::min<size_t>(threads, 1 + ne / 16384), [&] {
+    for (int p = next++; p < K; p = next++) {
+      const PartPlan &q = pp[p];
+      const ElimPart &d = out->parts[p];
+      put(&out->loc, d.voff, q.loc);
+      put(&out->inv, d.voff, q.inv);
+      put(&out->eptr, d.eptr_off, q.eptr);
+      put(&out->ecol, d.ent_off, q.ecol);
+      put(&out->w0, d.ent_off, q.w0);
+      if (directed) put(&out->w0b, d.ent_off, q.w0b);
+      for (int32_t e = 0; e < d.s; e++)
+        std::fill(out->eend.data() + d.ent_off + q.eptr[e], out->eend.data() + d.ent_off + q.eptr[e + 1], q.eptr[e + 1]);
+      put(&out->lev, d.lev_off, q.lev);
+      for (size_t i = 0; i < q.units.size(); i++) {
+        ElimUnit u = q.units[i];
+        u.rows += rows0[p];
+        u.list += list0[p];
+        out->units[unit0[p] + i] = u;
+      }
+      for (size_t i = 0; i < q.glev.size(); i++) out->glev[d.glev_off + i] = unit0[p] + q.glev[i];
+      put(&out->rows8, 2 * (size_t)rows0[p], q.rows8);
+      put(&out->list, list0[p], q.list);
+      put(&out->sloc, d.sloc_off, q.sloc);
+      put(&out->chunks, d.chunk_off, q.chunks);
+    }
+  });
+  out->ok = true;
 }
 
 void elim_offsets(int64_t ld, ElimPlan *plan) {

@@ -20,6 +20,7 @@
 #include <stdint.h>
 
 #include <functional>
+#include <memory>
 #include <vector>
 
 #include "fap_internal.h"
@@ -84,20 +85,37 @@ __host__ __device__ inline int32_t elim_body16(int32_t nu) {
   return kElimUnitRows / 2 + k / 4 + k * (nu & kElimWide ? 2 : 1);
 }
 
+// Array of a plan, not cleared when it is made: the parts' pieces are copied in
+// by several threads, which then also take the page faults.
+template <typename T>
+struct PlanArray {
+  std::unique_ptr<T[]> p;
+  size_t n = 0;
+  void make(size_t count) {
+    p.reset(new T[count]);
+    n = count;
+  }
+  T *data() { return p.get(); }
+  const T *data() const { return p.get(); }
+  size_t size() const { return n; }
+  T &operator[](size_t i) { return p[i]; }
+  const T &operator[](size_t i) const { return p[i]; }
+};
+
 struct ElimPlan {
   bool ok = false;
   std::vector<ElimPart> parts;
-  std::vector<int32_t> loc, inv;   // plan number <-> local index
-  std::vector<int32_t> eptr;       // entries of a vertex, relative to ent_off
-  std::vector<int32_t> ecol;       // N+(v), plan numbers, descending
-  std::vector<int32_t> eend;       // end of the entry's vertex, relative to ent_off
-  std::vector<int32_t> w0, w0b;    // weight (bits) of the arc v -> u, of u -> v, or the sentinel
-  std::vector<int32_t> lev;
-  std::vector<ElimUnit> units;
-  std::vector<int32_t> glev, rows8;  // rows8: pairs (slot, local index)
-  std::vector<uint16_t> list;
-  std::vector<int32_t> sloc;  // local index of every slot, parts one after the other (sloc_off)
-  std::vector<ElimChunk> chunks;
+  PlanArray<int32_t> loc, inv;   // plan number <-> local index
+  PlanArray<int32_t> eptr;       // entries of a vertex, relative to ent_off
+  PlanArray<int32_t> ecol;       // N+(v), plan numbers, descending
+  PlanArray<int32_t> eend;       // end of the entry's vertex, relative to ent_off
+  PlanArray<int32_t> w0, w0b;    // weight (bits) of the arc v -> u, of u -> v (directed plans), or the sentinel
+  PlanArray<int32_t> lev;
+  PlanArray<ElimUnit> units;
+  PlanArray<int32_t> glev, rows8;  // rows8: pairs (slot, local index)
+  PlanArray<uint16_t> list;
+  PlanArray<int32_t> sloc;  // local index of every slot, parts one after the other (sloc_off)
+  PlanArray<ElimChunk> chunks;
   int64_t stream16 = 0;
   int32_t max_chunk16 = 0, max_chunks = 0;
   std::vector<int64_t> group_work;  // per part: list entries times padded rows
@@ -118,9 +136,10 @@ struct ElimGraph {
 // columns fills the shared memory) or more than s * max(s, 256) / kElimDense entries.
 constexpr int32_t kElimMaxS = 6144;
 constexpr int64_t kElimDense = 16;
-// inf: bits of the sentinel; groups: also build the separator groups.
+// inf: bits of the sentinel; directed: keep both weights of an entry; groups:
+// also build the separator groups.
 void elim_build(int nparts, const std::function<void(int, ElimGraph *)> &graph, int threads, int32_t inf,
-                bool groups, ElimPlan *out);
+                bool directed, bool groups, ElimPlan *out);
 // w0 of a one-part plan := offsets of the entries in a matrix whose rows and
 // columns are the part's local indices.
 void elim_offsets(int64_t ld, ElimPlan *plan);
