@@ -737,10 +737,10 @@ constexpr int64_t kElimGraphEntries = 24576;
 constexpr int64_t kElimGraphList = 11;
 
 // The elimination plans: of the parts, for every graph with boundary vertices
-// whose parts eliminate with short lists, and on undirected int32 graphs
-// (el_sym: every arc has its reverse with the same weight, no duplicate arcs
-// inside a part) of the boundary graph.  Host work of some milliseconds on up
-// to 16 threads.
+// whose parts eliminate with short lists, and of the boundary graph, on
+// undirected int32 graphs (el_sym: every arc has its reverse with the same
+// weight, no duplicate arcs inside a part) with at most kBgraphFloydMax boundary
+// vertices.  Host work of some milliseconds on up to 16 threads.
 void plan_elim(fap_dgraph *G) {
   if (G->total_b <= 0) return;
   const bool i32 = G->dtype == FAP_DTYPE_I32;
@@ -780,7 +780,7 @@ void plan_elim(fap_dgraph *G) {
   if (!G->el.plan.ok) return;
   // (float32 parts keep min-plus over the boundary, which distance rows from
   // the resident cache match bit for bit)
-  if (!i32 || !G->sym_local) return;
+  if (!i32 || !G->sym_local || G->total_b > kBgraphFloydMax) return;
   std::vector<std::array<int32_t, 3>> cross;
   for (int32_t p = 1; p <= K; p++)
     for (int32_t i = 0; i < G->bnum[p]; i++) {
