@@ -367,14 +367,29 @@ def reference_partition(wf, workdir):
     return m
 
 
+def port_partition(wf):
+    """The same from the restatement's driver, in a process of its own, where
+    the reference binary is absent: (n, arcs, part sizes, boundary sizes)."""
+    r = subprocess.run([sys.executable, os.path.join(ROOT, "oracle", "port_cli.py"), "--dir", wf.root, "-f", wf.name,
+                        "-k", str(wf.K), "-direct", str(int(wf.edges.directed)), "-weight",
+                        str(int(wf.edges.weighted)), "--parts", "none"], capture_output=True, text=True, timeout=900)
+    if r.returncode != 0:
+        raise RuntimeError(f"CPU baseline process failed: {r.stderr[-500:]}")
+    m = next(json.loads(x) for x in r.stdout.splitlines() if x.startswith('{"event": "meta"'))
+    return m["n"], m["arcs"], np.array(m["ver_num"]), np.array(m["bdy_num"])
+
+
+def describe_counts(name, K, directed, n, arcs, vn, bn):
+    return {"workload": name, "n": int(n), "arcs": int(arcs), "K": int(K),
+            "directed": bool(directed), "avg_degree": round(float(arcs) / n, 3),
+            "part_size": [int(vn.min()), int(np.median(vn)), int(vn.max())],
+            "boundary": [int(bn.min()), int(np.median(bn)), int(bn.max()), int(bn.sum())]}
+
+
 def describe_meta(name, K, directed, m):
     """The workload description of `Workload.describe`, from the reference's
     own preprocessing."""
-    vn, bn = m.ver_num[1:], m.bdy_num[1:]
-    return {"workload": name, "n": int(m.n), "arcs": int(m.row_offset[-1]), "K": int(K),
-            "directed": bool(directed), "avg_degree": round(float(m.row_offset[-1]) / m.n, 3),
-            "part_size": [int(vn.min()), int(np.median(vn)), int(vn.max())],
-            "boundary": [int(bn.min()), int(np.median(bn)), int(bn.max()), int(bn.sum())]}
+    return describe_counts(name, K, directed, m.n, m.row_offset[-1], m.ver_num[1:], m.bdy_num[1:])
 
 
 def common_config(desc, n_gpus):
@@ -410,8 +425,7 @@ def main_reference(args):
     if meta is not None:
         config = common_config(describe_meta(wf.name, wf.K, wf.edges.directed, meta), args.gpus)
     else:
-        config = common_config({"workload": wf.name, "n": wf.n, "K": wf.K,
-                                "directed": wf.edges.directed}, args.gpus)
+        config = common_config(describe_counts(wf.name, wf.K, wf.edges.directed, *port_partition(wf)), args.gpus)
     P = cpu_procs(args.cpu_procs)
     steps = args.warmup + args.steps
     need = P * steps
@@ -435,7 +449,9 @@ def main_reference(args):
         "impl": "reference", "scaling": "strong", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic", "config": config,
         "solve": {"mode": "reference CPU path (oracle/_ref/fap_ref: the reference's fap.cpp, "
-                          "fapGraph::run per part)"},
+                          "fapGraph::run per part)" if kind == "reference" else
+                  "restatement of fapGraph::run per part on the CPU (the reference binary is absent: not the "
+                  "reference's own code, no ratio to it follows)"},
         "cpu_baseline": {"value": value, "unit": UNIT, "cores": P, "kind": kind,
                          "sample": sample},
         "e2e": {"value": value, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},

@@ -30,7 +30,7 @@ def main():
     ap.add_argument("-k", type=int, required=True)
     ap.add_argument("-direct", type=int, default=0)
     ap.add_argument("-weight", type=int, default=0)
-    ap.add_argument("--parts", default="all")
+    ap.add_argument("--parts", default="all")  # or a list, or "none": the partition only
     a = ap.parse_args()
     from fastapsp_b200.graph import fapGraph
     g = fapGraph(a.f, bool(a.direct), bool(a.weight), a.k, root=a.dir)
@@ -41,7 +41,10 @@ def main():
     ed2st = np.argsort(st2ed).astype(np.int32)
     vn, vo, bn = g.partInfo()
     n = g.num_vertexs
-    parts = range(1, a.k + 1) if a.parts == "all" else [int(x) for x in a.parts.split(",")]
+    print(json.dumps({"event": "meta", "n": int(n), "arcs": int(ro[n]), "ver_num": vn[1:].tolist(),
+                      "bdy_num": bn[1:].tolist()}), flush=True)
+    parts = (range(1, a.k + 1) if a.parts == "all" else [] if a.parts == "none"
+             else [int(x) for x in a.parts.split(",")])
     for p in parts:
         t0 = time.perf_counter()
         O.port_run_part(ro, col, w, gid, st2ed, ed2st, int(vo[p]), int(vn[p]), int(bn[p]))
