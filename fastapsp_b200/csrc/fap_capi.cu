@@ -458,6 +458,7 @@ struct fap_dgraph {
   // closed by Floyd), el2_small: it is small enough for one, barcs the arcs
   // between boundary vertices as (boundary index, boundary index, weight).
   bool eliminate = true;   // parameter "eliminate"
+  bool el_closes = false;  // closures by elimination (the plan may serve the group merge alone)
   bool el_sym = false;     // the plans of the boundary-graph form exist
   bool el2_small = false;
   bool last_elim = false;  // the prepared batch uses it
@@ -741,8 +742,20 @@ constexpr int64_t kElimGraphList = 11;
 // undirected int32 graphs (el_sym: every arc has its reverse with the same
 // weight, no duplicate arcs inside a part) with at most kBgraphFloydMax boundary
 // vertices.  Host work of some milliseconds on up to 16 threads.
+//
+// Closures are taken from the plan where one CTA's shared memory holds the
+// entries of every part's numeric elimination (28,000, 19,000 on directed
+// parts: grid parts of up to 1,500 vertices, road and geometric ones of any
+// planned size).  From L2 it takes several times as long, and graphs of few
+// large parts were slower than by Floyd (ms by Floyd / from L2: 70 x 70 grid in
+// two parts of 2,522 vertices, 52,000 entries, 3.9 / 6.0; 90 x 90 in two of
+// 4,109 10.6 / 20.6; one of a 140 x 140 grid's parts of 2,074 3.4 / 4.4; float32
+// and directed 0.55 to 1.2 of Floyd's time over whole solves, up to 1.4 for one
+// part).  int32 parts keep the plan for the group merge.
 void plan_elim(fap_dgraph *G) {
   if (G->total_b <= 0) return;
+  for (size_t p = 1; p < G->vnum.size(); p++)
+    if (G->vnum[p] > kElimMaxS) return;  // (one such part and there is no plan: nothing is eliminated in vain)
   const bool i32 = G->dtype == FAP_DTYPE_I32;
   // A float32 arc heavier than the sentinel keeps its weight in a closure
   // where no path is shorter; the sweeps start from the sentinel and would lose it.
@@ -778,6 +791,9 @@ void plan_elim(fap_dgraph *G) {
   };
   elim_build(K, part_graph, threads, inf, !G->sym_local, i32, &G->el.plan);
   if (!G->el.plan.ok) return;
+  G->el_closes = elim_up_fits(G->el.plan, !G->sym_local);
+  if (!G->el_closes && !i32) G->el.plan = ElimPlan{};
+  if (!G->el_closes) return;
   // (float32 parts keep min-plus over the boundary, which distance rows from
   // the resident cache match bit for bit)
   if (!i32 || !G->sym_local || G->total_b > kBgraphFloydMax) return;
@@ -837,7 +853,7 @@ int build_elim(fap_dgraph *G) {
   G->el2.clear();
   G->barcs.clear();
   G->dev_barcs = nullptr;
-  G->el_sym = G->el2_small = false;
+  G->el_closes = G->el_sym = G->el2_small = false;
   plan_elim(G);
   if (!G->el.plan.ok) return FAP_OK;
   const bool directed = !G->sym_local;  // (el2 is symmetric)
@@ -848,7 +864,7 @@ int build_elim(fap_dgraph *G) {
     G->el.clear();
     G->el2.clear();
     G->barcs.clear();
-    G->el_sym = G->el2_small = false;
+    G->el_closes = G->el_sym = G->el2_small = false;
     return FAP_OK;
   }
   char *base = G->d_elim.as<char>();
@@ -890,7 +906,7 @@ T *bgraph_work(T *dB, int64_t ldB) {
 
 // Whether the SSSP form closes the parts by elimination from its boundary rows
 // (any dtype, directed or not) instead of Floyd-Warshall.
-bool elim_given_ok(const fap_dgraph *G) { return G->eliminate && G->el.plan.ok && !G->floyd_per_cta; }
+bool elim_given_ok(const fap_dgraph *G) { return G->eliminate && G->el_closes && !G->floyd_per_cta; }
 }  // namespace
 
 extern "C" int fap_graph_destroy(fap_dgraph *G) try {

@@ -49,13 +49,15 @@ __global__ void elim_seed_arcs_kernel(int32_t *M, int64_t ld, const int32_t *__r
 // u_j: the entry (u_i, u_j), found in u_i's list, is lowered to
 // W(v, u_i) + W(v, u_j).  Two vertices of a level may lower the same entry
 // (atomicMin); none of them reads it before the level's barrier.
-// Bound by the latency of the levels, so SM keeps all that a level reads in
-// shared memory: entries as {u | entries after this one << 16, W}, the lists'
+// Bound by the latency of the levels, so shared memory holds all that a level
+// reads (ALL): entries as {u | entries after this one << 16, W}, the lists'
 // starts and the levels' entry ranges (a 670-vertex boundary graph: 140 us
-// with only W there, 58 us).  Otherwise the entries sit in L2 and are read
-// past L1.
+// with only W there, 58 us).  Parts of up to 38,000 entries (23,000 directed)
+// whose whole plan does not fit keep W and u there, which the updates and the
+// searches touch, and read starts and ends through L1.  (With the entries in L2
+// larger parts took longer than their Floyd-Warshall; they keep that.)
 // Directed parts (entb): an entry carries both weights, and a pair lowers both.
-template <typename T, bool SM>
+template <typename T, bool ALL>
 __global__ void __launch_bounds__(kElimUpThreads)
     elim_up_kernel(ElimDev e, const int32_t *__restrict__ list, const T *__restrict__ from, T *M, int64_t ldM) {
   extern __shared__ int2 up_smem[];
@@ -66,10 +68,13 @@ __global__ void __launch_bounds__(kElimUpThreads)
   const bool directed = e.entb != nullptr;
   int2 *gent = e.ent + P.ent_off;
   int32_t *gentb = directed ? e.entb + P.ent_off : nullptr;
-  int2 *ent = SM ? up_smem : gent;
-  int32_t *sptr = reinterpret_cast<int32_t *>(up_smem + (SM ? P.nent : 0));  // s + 1 list starts
-  int32_t *slev = sptr + P.s + 1;                                            // nlev + 1 entry ranges
-  int32_t *entb = SM ? slev + P.nlev + 1 : gentb;
+  // ALL: entries, s + 1 list starts, nlev + 1 entry ranges, second weights;
+  // else weights, second weights, heads
+  int2 *ent = up_smem;
+  int32_t *sptr = reinterpret_cast<int32_t *>(up_smem + P.nent), *slev = sptr + P.s + 1;
+  int32_t *sw = reinterpret_cast<int32_t *>(up_smem);
+  int32_t *entb = ALL ? slev + P.nlev + 1 : sw + P.nent;
+  uint16_t *su = reinterpret_cast<uint16_t *>(entb + (directed ? P.nent : 0));
   const int lane = threadIdx.x % kUpLanes, group = threadIdx.x / kUpLanes, ngroups = blockDim.x / kUpLanes;
   auto value = [](int32_t bits) -> T {
     if constexpr (std::is_same<T, float>::value) return __int_as_float(bits);
@@ -79,35 +84,44 @@ __global__ void __launch_bounds__(kElimUpThreads)
     if constexpr (std::is_same<T, float>::value) return __float_as_int(x);
     else return x;
   };
-  if (SM) {
+  auto entry = [&](int i) -> int2 {  // {head, W}
+    if (ALL) return make_int2(ent[i].x & 0xffff, ent[i].y);
+    return make_int2(su[i], sw[i]);
+  };
+  if (ALL) {
     for (int v = threadIdx.x; v <= P.s; v += blockDim.x) sptr[v] = eptr[v];
     for (int l = threadIdx.x; l <= P.nlev; l += blockDim.x) slev[l] = eptr[lev[l]];
   }
   for (int i = threadIdx.x; i < P.nent; i += blockDim.x) {
-    ent[i] = make_int2(SM ? ecol[i] | (eend[i] - i - 1) << 16 : ecol[i], from ? bits(from[w0[i]]) : w0[i]);
+    const int32_t w = from ? bits(from[w0[i]]) : w0[i];
+    if (ALL) {
+      ent[i] = make_int2(ecol[i] | (eend[i] - i - 1) << 16, w);
+    } else {
+      sw[i] = w;
+      su[i] = (uint16_t)ecol[i];
+    }
     if (directed) entb[i] = e.w0b[P.ent_off + i];
   }
-  if (!SM) __threadfence();
   __syncthreads();
   for (int l = P.nlev - 1; l >= 0; l--) {
-    const int i1 = SM ? slev[l + 1] : eptr[lev[l + 1]];
-    for (int i = (SM ? slev[l] : eptr[lev[l]]) + group; i < i1; i += ngroups) {
-      const int2 a = SM ? ent[i] : __ldcg(ent + i);
-      const int ui = SM ? a.x & 0xffff : a.x;
-      const int end = SM ? i + 1 + (int)((uint32_t)a.x >> 16) : eend[i];
+    const int i1 = ALL ? slev[l + 1] : __ldg(eptr + __ldg(lev + l + 1));
+    for (int i = (ALL ? slev[l] : __ldg(eptr + __ldg(lev + l))) + group; i < i1; i += ngroups) {
+      const int end = ALL ? i + 1 + (int)((uint32_t)ent[i].x >> 16) : __ldg(eend + i);
+      const int2 a = entry(i);
+      const int ui = a.x;
       if (ui < P.b && M == nullptr) continue;  // (pairs of boundary vertices are not wanted)
-      const T out = value(a.y), in = directed ? value(SM ? entb[i] : __ldcg(entb + i)) : out;
+      const T out = value(a.y), in = directed ? value(entb[i]) : out;
       if (out >= inf && in >= inf) continue;
       int lo = 0, hi = 0;
       if (ui >= P.b) {
-        lo = SM ? sptr[ui] : eptr[ui];
-        hi = SM ? sptr[ui + 1] : eptr[ui + 1];
+        lo = ALL ? sptr[ui] : __ldg(eptr + ui);
+        hi = ALL ? sptr[ui + 1] : __ldg(eptr + ui + 1);
       }
       for (int j = i + 1 + lane; j < end; j += kUpLanes) {
-        const int2 c = SM ? ent[j] : __ldcg(ent + j);
-        const int uj = SM ? c.x & 0xffff : c.x;
+        const int2 c = entry(j);
+        const int uj = c.x;
         const T fwd = in + value(c.y);  // u_i -> v -> u_j
-        const T back = directed ? value(SM ? entb[j] : __ldcg(entb + j)) + out : fwd;
+        const T back = directed ? value(entb[j]) + out : fwd;
         if (fwd >= inf && back >= inf) continue;
         if (ui < P.b) {
           Dist<T>::atomic_min(M + (int64_t)(P.boff + ui) * ldM + P.boff + uj, fwd);
@@ -117,21 +131,20 @@ __global__ void __launch_bounds__(kElimUpThreads)
         int x = lo, y = hi - 1;  // descending; u_j is in the list
         while (x < y) {
           const int m = (x + y) >> 1;
-          if ((SM ? ent[m].x & 0xffff : ecol[m]) > uj) x = m + 1;
+          if ((ALL ? ent[m].x & 0xffff : (int)su[m]) > uj) x = m + 1;
           else y = m;
         }
         // (non-negative float bits order like int32)
-        if (fwd < inf) atomicMin(&ent[x].y, bits(fwd));
+        if (fwd < inf) atomicMin(ALL ? &ent[x].y : sw + x, bits(fwd));
         if (directed && back < inf) atomicMin(entb + x, bits(back));
       }
     }
     __syncthreads();
   }
-  if (SM)
-    for (int i = threadIdx.x; i < P.nent; i += blockDim.x) {
-      gent[i] = make_int2(ent[i].x & 0xffff, ent[i].y);
-      if (directed) gentb[i] = entb[i];
-    }
+  for (int i = threadIdx.x; i < P.nent; i += blockDim.x) {
+    gent[i] = entry(i);
+    if (directed) gentb[i] = entb[i];
+  }
 }
 
 // What a sweep reads of a part's plan: the entries, the lists' starts and the
@@ -602,6 +615,13 @@ __global__ void __launch_bounds__(kMergeThreads, 2)
   }
 }
 
+// Shared memory of elim_up_kernel<ALL>.
+size_t up_smem_bytes(bool all, int32_t max_nent, int32_t max_s, int32_t max_nlev, bool directed) {
+  const size_t n = max_nent;
+  if (!all) return n * (directed ? 10 : 6);
+  return (n * (directed ? 3 : 2) + (size_t)max_s + max_nlev + 2) * sizeof(int32_t);
+}
+
 template <class K>
 cudaError_t allow_smem(K kern, size_t smem) {
   return smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
@@ -644,14 +664,14 @@ cudaError_t launch_elim_up(const ElimDev &e, const int32_t *list, int count, con
   if (list == nullptr) count = e.nparts;
   if (count <= 0) return cudaSuccess;
   if (M != nullptr && e.entb != nullptr) return cudaErrorInvalidValue;
-  const size_t smem = ((size_t)e.max_nent * (e.entb ? 3 : 2) + (size_t)e.max_s + e.max_nlev + 2) * sizeof(int32_t);
-  if (smem <= kElimSmem) {
-    cudaError_t err = allow_smem(elim_up_kernel<T, true>, smem);
-    if (err != cudaSuccess) return err;
-    elim_up_kernel<T, true><<<count, kElimUpThreads, smem, stream>>>(e, list, from, M, ldM);
-  } else {
-    elim_up_kernel<T, false><<<count, kElimUpThreads, 0, stream>>>(e, list, from, M, ldM);
-  }
+  const bool directed = e.entb != nullptr;
+  const bool all = up_smem_bytes(true, e.max_nent, e.max_s, e.max_nlev, directed) <= kElimSmem;
+  const size_t smem = up_smem_bytes(all, e.max_nent, e.max_s, e.max_nlev, directed);
+  if (smem > kElimSmem) return cudaErrorInvalidValue;  // (elim_up_fits)
+  auto kern = all ? elim_up_kernel<T, true> : elim_up_kernel<T, false>;
+  cudaError_t err = allow_smem(kern, smem);
+  if (err != cudaSuccess) return err;
+  kern<<<count, kElimUpThreads, smem, stream>>>(e, list, from, M, ldM);
   *launches += 1;
   return cudaGetLastError();
 }
@@ -698,6 +718,11 @@ cudaError_t launch_elim_expand(const ElimDev &e, const int64_t *rows, int nrows,
     *launches += 1;
     return cudaGetLastError();
   });
+}
+
+bool elim_up_fits(const ElimPlan &p, bool directed) {
+  return up_smem_bytes(false, p.max_nent, p.max_s, p.max_nlev, directed) <= kElimSmem ||
+         up_smem_bytes(true, p.max_nent, p.max_s, p.max_nlev, directed) <= kElimSmem;
 }
 
 bool elim_merge_fits(const ElimPlan &p, int slots) {

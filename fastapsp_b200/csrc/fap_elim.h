@@ -216,6 +216,9 @@ cudaError_t launch_elim_coef(const ElimDev &e, const ElimMerge &m, const PartDes
 cudaError_t launch_elim_merge(const ElimDev &e, const ElimMerge &m, const PartDesc *parts, const int32_t *F, int n,
                               int32_t *D, int64_t ldD, const int32_t *graph_id, const int32_t *ed2st, int max_slots,
                               cudaStream_t stream, int64_t *launches);
+// Whether the numeric elimination of every part keeps its entries in a CTA's
+// shared memory.
+bool elim_up_fits(const ElimPlan &p, bool directed);
 // Whether a part with that many slots fits in a CTA's shared memory.
 bool elim_merge_fits(const ElimPlan &p, int slots);
 

@@ -117,3 +117,47 @@ def test_no_memory_for_the_plans(cuda_ok):
     dg.solve(some, FAP_MODE_BATCHED)
     for a, p in zip(got, some):
         assert np.array_equal(a, dg.copy_block(p)), p
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("side,K,closes", [(36, 2, True),     # whole plan in shared memory
+                                           (64, 2, None),     # weights and heads only (directed: too large)
+                                           (70, 2, False)])   # the parts keep Floyd-Warshall
+def test_numeric_elimination_by_size(cuda_ok, side, K, closes, directed):
+    """Grid parts below and above what a CTA's shared memory holds of the numeric
+    elimination: the same blocks as the general path, for all parts, one part and
+    from the resident cache; the form's name says which closed them."""
+    el = G.grid_graph(side, side, extra_frac=0.01 if side == 70 else 0.0, wmin=1, wmax=100, seed=43)
+    if directed:
+        rng = np.random.default_rng(43)
+        el = G.EdgeList(el.n, np.concatenate([el.edges, el.edges[:, ::-1]]),
+                        rng.integers(1, 100, 2 * el.edges.shape[0]).astype(np.float32), directed=True, weighted=True,
+                        integral=True)
+        closes = closes if side == 36 else False
+    elif closes is None:
+        closes = True
+    ro, col, w = G.edges_to_csr(el)
+    fg = fapGraph.from_csr(el.n, int(ro[-1]), ro, col, w, K, directed=el.directed)
+    fg.preCondition()
+    dg = DeviceGraph(Context(0), ro, col, w)
+    vn, vo, bn = fg.partInfo()
+    dg.set_parts(K, fg.getGraphId(), fg.getMapping(), vn, vo, bn)
+    if directed:
+        dg.set_param("stage1", 1)
+    dg.set_param("eliminate", 0)
+    dg.solve(mode=FAP_MODE_BATCHED)
+    want = [dg.copy_block(p) for p in range(1, K + 1)]
+    dg.set_param("eliminate", 1)
+    for parts in (None, [2], None, None, None):          # (launched directly, then captured and replayed)
+        dg.solve(parts, FAP_MODE_BATCHED)
+        assert ("elimination" in dg.stage1_name()) == closes
+        for p in parts or range(1, K + 1):
+            assert np.array_equal(dg.copy_block(p), want[p - 1]), p
+    dg.cache_build()
+    assert np.array_equal(dg.rows([int(fg.getMapping()[vo[2] + 40])])[0], want[1][40].astype(np.float32))
+    for parts in ([1], None):
+        dg.solve(parts, FAP_MODE_BATCHED)
+        assert dg.last_stage1() == 3 and ("elimination" in dg.stage1_name()) == closes
+        for p in parts or range(1, K + 1):
+            assert np.array_equal(dg.copy_block(p), want[p - 1]), p
+
