@@ -161,3 +161,32 @@ def test_numeric_elimination_by_size(cuda_ok, side, K, closes, directed):
         for p in parts or range(1, K + 1):
             assert np.array_equal(dg.copy_block(p), want[p - 1]), p
 
+
+def test_some_parts_merged(cuda_ok):
+    """Parts whose separator rows do not fit a CTA's shared memory beside others
+    that do: the batch takes the tiles for all, a batch of the others the merge."""
+    el = G.grid_graph(110, 110, wmin=1, wmax=100, seed=4)
+    ro, col, w = G.edges_to_csr(el)
+    K = 4
+    fg = fapGraph.from_csr(el.n, int(ro[-1]), ro, col, w, K, directed=el.directed)
+    fg.preCondition()
+    dg = DeviceGraph(Context(0), ro, col, w)
+    vn, vo, bn = fg.partInfo()
+    dg.set_parts(K, fg.getGraphId(), fg.getMapping(), vn, vo, bn)
+    every = list(range(1, K + 1))
+    dg.set_param("eliminate", 0)
+    dg.solve(every, FAP_MODE_BATCHED)
+    want = [dg.copy_block(p) for p in every]
+    dg.set_param("eliminate", 1)
+    alone = []
+    for p in every:
+        dg.solve([p], FAP_MODE_BATCHED)
+        alone.append(dg.last_work()[2])
+        assert np.array_equal(dg.copy_block(p), want[p - 1]), p
+    assert 0 < sum(alone) < K
+    for _ in range(3):
+        dg.solve(every, FAP_MODE_BATCHED)
+        assert dg.last_work()[2] == 0
+        for p in every:
+            assert np.array_equal(dg.copy_block(p), want[p - 1]), p
+    assert dg.last_launches() < 60
