@@ -1251,6 +1251,11 @@ constexpr int kThinHalf = kThinCols / 2;
 constexpr int kThinRows = 32;   // a CTA's rows are a multiple of this
 constexpr int kThinOwn = 8192;  // own-part values staged at a time (rows x own columns of the strip)
 
+__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
 template <typename T>
 struct ThinShared {
   __align__(16) T As[kMinplusBM][kThinK];
@@ -1302,8 +1307,9 @@ __device__ __forceinline__ void thin_rows(ThinShared<T> &sh, const PartDesc &pd,
     }
     for (int t = threadIdx.x; t < rows * nown; t += blockDim.x) {
       const int r = t / nown, o = t - r * nown;
-      sh.Own[t] = __ldg(Fr + (int64_t)r * pd.ldf + sh.own_col[o]);
+      cp_async4(&sh.Own[t], Fr + (int64_t)r * pd.ldf + sh.own_col[o]);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     T *Cm = D + (pd.row_base + pd.b + m0) * ldD + c0;
 #pragma unroll 2
