@@ -1470,9 +1470,15 @@ int run_elim(fap_dgraph *G, const PartDesc *dp, int count, int max_s, int32_t *F
 
 // Whether part p's inner rows come from the group merge instead of the
 // min-plus tiles: its padded relaxations have to be at most half of the
-// tiles' inner x b.
+// tiles' inner x b, and where an SM holds one CTA only the boundary has to be
+// wide (geometric parts of 3,000 to 6,000 vertices with 25 to 45 boundary
+// vertices: tiles 1.97 and 2.45 ms, merge 2.05 and 2.59; grid parts of 2,450 to
+// 2,900 with 77 and more: 0.41 to 0.6 of the tiles' time).
+constexpr int32_t kMergeWide = 64;
 bool merge_ok(const fap_dgraph *G, int32_t p) {
-  return G->bnum[p] > kThinBoundary && elim_merge_fits(G->el.plan, G->el.plan.parts[p - 1].nslots) && G->vnum[p] > G->bnum[p] &&
+  if (G->bnum[p] <= kThinBoundary || G->vnum[p] <= G->bnum[p]) return false;
+  const int ctas = elim_merge_ctas(G->el.plan, G->el.plan.parts[p - 1].nslots);
+  return (ctas == 2 || (ctas == 1 && G->bnum[p] >= kMergeWide)) &&
          2 * G->el.plan.group_work[p - 1] <= (int64_t)(G->vnum[p] - G->bnum[p]) * G->bnum[p];
 }
 

@@ -725,8 +725,9 @@ bool elim_up_fits(const ElimPlan &p, bool directed) {
          up_smem_bytes(true, p.max_nent, p.max_s, p.max_nlev, directed) <= kElimSmem;
 }
 
-bool elim_merge_fits(const ElimPlan &p, int slots) {
-  return merge_smem(slots, 128, p.max_chunk16, p.max_chunks) <= kElimSmem;
+int elim_merge_ctas(const ElimPlan &p, int slots) {
+  const size_t smem = merge_smem(slots, 128, p.max_chunk16, p.max_chunks);
+  return smem <= kElimHalf ? 2 : smem <= kElimSmem ? 1 : 0;
 }
 
 cudaError_t launch_elim_coef(const ElimDev &e, const ElimMerge &m, const PartDesc *parts, const int32_t *F,

@@ -219,7 +219,7 @@ cudaError_t launch_elim_merge(const ElimDev &e, const ElimMerge &m, const PartDe
 // Whether the numeric elimination of every part keeps its entries in a CTA's
 // shared memory.
 bool elim_up_fits(const ElimPlan &p, bool directed);
-// Whether a part with that many slots fits in a CTA's shared memory.
-bool elim_merge_fits(const ElimPlan &p, int slots);
+// CTAs of the merge that an SM holds for a part with that many slots (0 to 2).
+int elim_merge_ctas(const ElimPlan &p, int slots);
 
 }  // namespace fapb

@@ -190,3 +190,25 @@ def test_some_parts_merged(cuda_ok):
         for p in every:
             assert np.array_equal(dg.copy_block(p), want[p - 1]), p
     assert dg.last_launches() < 60
+
+
+def test_large_parts_with_narrow_boundaries_keep_the_tiles(cuda_ok):
+    """Where one CTA of the merge fits on an SM and the boundary has few vertices,
+    the tiles are faster; the blocks are the same."""
+    el = G.random_geometric_graph(9600, 4.0, seed=3)
+    ro, col, w = G.edges_to_csr(el)
+    K = 2
+    fg = fapGraph.from_csr(el.n, int(ro[-1]), ro, col, w, K, directed=el.directed)
+    fg.preCondition()
+    dg = DeviceGraph(Context(0), ro, col, w)
+    vn, vo, bn = fg.partInfo()
+    assert 16 < bn[1:].min() and bn[1:].max() < 64
+    dg.set_parts(K, fg.getGraphId(), fg.getMapping(), vn, vo, bn)
+    out = []
+    for eliminate in (0, 1):
+        dg.set_param("eliminate", eliminate)
+        dg.solve(mode=FAP_MODE_BATCHED)
+        assert ("elimination" in dg.stage1_name()) == bool(eliminate) and dg.last_work()[2] == 0
+        out.append([dg.copy_block(p) for p in range(1, K + 1)])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
