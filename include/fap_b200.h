@@ -207,7 +207,9 @@ FAP_API int fap_graph_sssp_rows(fap_dgraph *g, const int32_t *sources, int32_t c
  * the local closures' tiles on and above the diagonal and stores their
  * transposes); "eliminate" (default 1: vertex elimination instead of
  * Floyd-Warshall, in batched solves and the resident cache, of graphs whose
- * parts have at most 6144 vertices each and eliminate with short lists.
+ * parts have at most 6144 vertices each and eliminate with short lists: at
+ * most about 38,000 entries a part, 23,000 on directed ones (grid parts of
+ * 2,000 and 1,300 vertices, road and geometric ones of any such size).
  * Undirected int32 graphs without duplicate arcs inside a part and with at most
  * 8192 boundary vertices: parts and small boundary graphs are closed by it
  * instead of Floyd-Warshall and SSSP, also for batches of some of the parts,
@@ -217,7 +219,7 @@ FAP_API int fap_graph_sssp_rows(fap_dgraph *g, const int32_t *sources, int32_t c
  * "floyd_queue" and "floyd_symmetric" say; float32 graphs with an arc of
  * more than 1e8 keep Floyd-Warshall.  int32 parts with more than 16 boundary
  * vertices: their inner rows come from separator groups where that takes at
- * most half of the relaxations.  int32 values are the same either way; float32
+ * most half of the relaxations (also of parts with more entries).  int32 values are the same either way; float32
  * sums associate differently (a few ulps; the same pairs are reachable).  0:
  * the general path everywhere); "thin_max_b" (0..16, default 16: parts with at most this many
  * boundary vertices take the store-shaped thin min-plus kernel, the others
