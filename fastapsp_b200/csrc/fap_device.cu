@@ -1295,7 +1295,7 @@ __device__ __forceinline__ void thin_rows(ThinShared<T> &sh, const PartDesc &pd,
   // merge of graphs of five parts).  The own values are copied asynchronously,
   // all of a block in flight: loaded a few at a time, the short blocks of graphs
   // of few large parts waited for memory (12,000 vertices in three parts from
-  // the resident cache 0.39 ms, 0.20 so; road20k 0.42 -> 0.33, road114k 8.7 -> 8.6).
+  // the resident cache 0.39 ms, 0.20 so; road20k 0.39 -> 0.31, road114k 8.74 -> 8.59).
   const bool warp_own = __any_sync(0xffffffffu, any_own);
   const int nown = sh.nown;  // same in every thread
   const int block = nown <= kThinOwn / kMinplusBM ? kMinplusBM : kThinOwn / nown;

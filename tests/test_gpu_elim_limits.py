@@ -4,7 +4,7 @@ against 0."""
 import numpy as np
 import pytest
 
-from fastapsp_b200 import FAP_DTYPE_F32, FAP_MODE_BATCHED, Context, DeviceGraph, fapGraph
+from fastapsp_b200 import FAP_DTYPE_F32, FAP_DTYPE_I32, FAP_MODE_BATCHED, Context, DeviceGraph, fapGraph
 from fastapsp_b200 import generators as G
 
 pytestmark = pytest.mark.gpu
@@ -119,30 +119,31 @@ def test_no_memory_for_the_plans(cuda_ok):
         assert np.array_equal(a, dg.copy_block(p)), p
 
 
-@pytest.mark.parametrize("directed", [False, True])
-@pytest.mark.parametrize("side,K,closes", [(36, 2, True),     # whole plan in shared memory
-                                           (64, 2, None),     # weights and heads only (directed: too large)
-                                           (70, 2, False)])   # the parts keep Floyd-Warshall
-def test_numeric_elimination_by_size(cuda_ok, side, K, closes, directed):
+@pytest.mark.parametrize("dtype", ["i32", "f32"])
+@pytest.mark.parametrize("directed,side,closes", [
+    (False, 36, True),      # whole plan in shared memory
+    (False, 64, True),      # weights and heads only
+    (False, 70, False),     # the parts keep Floyd-Warshall
+    (True, 36, True), (True, 50, True), (True, 64, False)])
+def test_numeric_elimination_by_size(cuda_ok, directed, side, closes, dtype):
     """Grid parts below and above what a CTA's shared memory holds of the numeric
-    elimination: the same blocks as the general path, for all parts, one part and
-    from the resident cache; the form's name says which closed them."""
+    elimination: the same blocks as the general path (whole weights: float32 sums
+    are exact), for all parts, one part and from the resident cache; the form's
+    name says which closed them."""
+    K = 2
     el = G.grid_graph(side, side, extra_frac=0.01 if side == 70 else 0.0, wmin=1, wmax=100, seed=43)
     if directed:
         rng = np.random.default_rng(43)
         el = G.EdgeList(el.n, np.concatenate([el.edges, el.edges[:, ::-1]]),
                         rng.integers(1, 100, 2 * el.edges.shape[0]).astype(np.float32), directed=True, weighted=True,
                         integral=True)
-        closes = closes if side == 36 else False
-    elif closes is None:
-        closes = True
     ro, col, w = G.edges_to_csr(el)
     fg = fapGraph.from_csr(el.n, int(ro[-1]), ro, col, w, K, directed=el.directed)
     fg.preCondition()
-    dg = DeviceGraph(Context(0), ro, col, w)
+    dg = DeviceGraph(Context(0), ro, col, w, FAP_DTYPE_I32 if dtype == "i32" else FAP_DTYPE_F32)
     vn, vo, bn = fg.partInfo()
     dg.set_parts(K, fg.getGraphId(), fg.getMapping(), vn, vo, bn)
-    if directed:
+    if directed or dtype == "f32":
         dg.set_param("stage1", 1)
     dg.set_param("eliminate", 0)
     dg.solve(mode=FAP_MODE_BATCHED)
