@@ -2993,6 +2993,7 @@ int64_t sssp_growth(const fap_dgraph *G, int64_t count, bool frontier) {
 extern "C" int fap_graph_batch_bytes(const fap_dgraph *G, const int32_t *parts, int32_t count, int64_t rows,
                                      int64_t copied_rows, int64_t *bytes) try {
   if (!G || !bytes) return fail(FAP_ERR_INVALID, "NULL argument");
+  if (parts && count < 0) return fail(FAP_ERR_INVALID, "negative count");
   if (G->K == 0) return fail(FAP_ERR_STATE, "no partition");
   const int64_t np = parts ? count : G->K, n = G->n;
   int64_t need = 0, sources = 0, ldf = kFloydTile, work = 0;

@@ -105,3 +105,11 @@ def test_server_keeps_within_a_tight_budget(cuda_ok, name, slack_mb):
         st = srv.stats()
         assert st.failed == 0 and st.completed == len(reqs)
         assert st.peak_bytes <= budget, st.peak_bytes - budget
+
+
+def test_a_negative_count_is_refused(cuda_ok):
+    dg, K, vn, _ = _graph("road")
+    b = ctypes.c_int64()
+    ids = np.asarray([1], np.int32)
+    with pytest.raises(Exception, match="negative count"):
+        check(lib().fap_graph_batch_bytes(dg._h, ptr(ids), -1, 1, 1, ctypes.byref(b)))
